@@ -319,7 +319,7 @@ static int check_limits(tm_machine *m) {
 // A train-kernel variant a caller may pin: modes 0-3 with 1, 2 or 4
 // clauses per warp, or mode 4 with one of its configurations.
 static bool variant_ok(int mode, int cpw) {
-  if (mode == TM_MODE_WPT) return cpw >= 1 && cpw <= wpt_configs();
+  if (mode == TM_MODE_WPT) return cpw >= 1 && cpw <= TM_WPT_PINNED;
   return mode >= -1 && mode <= TM_MODE_WARP && (cpw == 1 || cpw == 2 || cpw == 4);
 }
 
@@ -445,7 +445,7 @@ extern "C" int tm_force_variant(tm_machine *m, int32_t mode, int32_t cpw) {
   if (!m) return fail(TM_ERR_ARG, "null machine");
   if (!variant_ok(mode, cpw))
     return fail(TM_ERR_ARG, "force_variant: mode -1..3 with clauses per warp 1, 2 or 4, or mode 4 "
-                            "with a configuration 1..%d", wpt_configs());
+                            "with a configuration 1..%d", TM_WPT_PINNED);
   m->force_mode = mode;
   m->force_cpw = cpw;
   return TM_OK;
@@ -748,8 +748,8 @@ static int launch_plan(const TrainPlan &p, const TrainShape &sh, const std::vect
                          (unsigned long long *)(err + 2)));
   else if (p.mode == TM_MODE_WPT)
     CK(launch_train_wpt(p.cpw, (const TrainDev *)base, (const WorkItem *)(base + off_w),
-                        (uint32_t)work.size(), counter, e0, e1, sh.Wpmax, sh.smax, m0->row_wait,
-                        p.grid, err, st));
+                        (uint32_t)work.size(), counter, e0, e1, sh.Wpmax, sh.smax, p.grid, err,
+                        st));
   else
     CK(launch_train((const TrainDev *)base, (const WorkItem *)(base + off_w),
                     (uint32_t)work.size(), counter, e0, e1, lay, p.mode, sh.Bmin, sh.Bmax,
@@ -806,19 +806,31 @@ static int autotune_plan(std::vector<TrainJob> &jobs, const std::vector<TrainDev
     CK(cudaEventCreate(&m0->ev1));
   }
   std::vector<TrainPlan> cand;
-  for (int mode : {TM_MODE_WARP, TM_MODE_SMEM, TM_MODE_GLOBAL, TM_MODE_PAIR, TM_MODE_WPT}) {
-    if (mode == TM_MODE_WARP && m0->no_warp) continue;
-    if (mode == TM_MODE_WPT) {
-      for (int id = 1; id <= wpt_configs(); id++) {
-        TrainPlan p;
-        if (plan_mode(mode, sh, p, id)) cand.push_back(p);
-      }
-      continue;
-    }
-    for (int cpw : {1, 2, 4}) {
+  // 8-bit units of rows up to 1,024 words: the kernels of tm_train_wpt.cu beat
+  // every other variant at each width measured (28 to 1,024 words, 40 to
+  // 93,000 units), so only their choices are tried; the others serve what
+  // these cannot hold (other state widths, wider rows, overflow lists of a
+  // very low specificity that do not fit the shared memory).
+  if (sh.Bmin == 8 && sh.Bmax == 8) {
+    int ids[4];
+    const int k = wpt_choices(sh.Wpmax, sh.smax, sh.units, sh.sms, sh.optin, ids, 4);
+    for (int i = 0; i < k; i++) {
       TrainPlan p;
-      if (plan_mode(mode, sh, p, cpw)) cand.push_back(p);
+      if (plan_mode(TM_MODE_WPT, sh, p, ids[i])) cand.push_back(p);
     }
+  }
+  if (cand.empty())
+    for (int mode : {TM_MODE_WARP, TM_MODE_SMEM, TM_MODE_GLOBAL, TM_MODE_PAIR}) {
+      if (mode == TM_MODE_WARP && m0->no_warp) continue;
+      for (int cpw : {1, 2, 4}) {
+        TrainPlan p;
+        if (plan_mode(mode, sh, p, cpw)) cand.push_back(p);
+      }
+    }
+  if (cand.size() == 1 && cand[0].mode == TM_MODE_WPT) {  // nothing to time
+    out = cand[0];
+    tuned = true;
+    return TM_OK;
   }
   if (cand.size() < 2) return TM_OK;  // nothing to choose: the heuristic plan
   // Two trials, each on automata reset to the initial state (capi.c:1136-
@@ -1706,7 +1718,7 @@ static int search_round(tm_machine *const *ms, const tm_train_args *args, uint32
                                (unsigned long long *)(d_err + 2));
     if (pl.mode == TM_MODE_WPT)
       return launch_train_wpt(pl.cpw, (const TrainDev *)tbase, wk, nw, ctr, 0, 1, shp.Wpmax,
-                              shp.smax, m0->row_wait, pl.grid, d_err, s_);
+                              shp.smax, pl.grid, d_err, s_);
     return launch_train((const TrainDev *)tbase, wk, nw, ctr, 0, 1, ly, pl.mode, shp.Bmin,
                         shp.Bmax, pl.cpw, pl.grid, d_err, s_);
   };

@@ -144,16 +144,18 @@ uint64_t gemm_bucket(uint64_t k, uint64_t cap);
 // The fused train kernels report through err[0] (status bits) and
 // err[2..3], a 64-bit count of active (unit, sample) steps -- the samples
 // each unit actually trained on after negative sampling.
-// k_train_wpt (tm_train_wpt.cu): one CTA per unit, every thread owning a
-// few words of all eight clauses, the automata held in registers and shared
-// memory; `cpw` of a plan with this mode is the configuration id (1-based).
+// The kernels of tm_train_wpt.cu: one CTA per unit, the automata of 8-bit
+// units on the SM while the unit trains; `cpw` of a plan with this mode is
+// the configuration id (1-based).  Callers may pin ids up to TM_WPT_PINNED.
+constexpr int TM_WPT_PINNED = 8;
 constexpr int TM_MODE_WPT = 4;
-int wpt_configs();
+int wpt_choices(uint32_t Wpmax, uint32_t smax, uint32_t units, int sms, int optin, int *ids,
+                int max);
 int train_wpt_occupancy(int id, uint32_t Wpmax, uint32_t smax, size_t *smem_bytes);
 cudaError_t launch_train_wpt(int id, const TrainDev *machines, const WorkItem *work,
                              uint32_t nwork, uint32_t *counter, uint32_t e_begin, uint32_t e_end,
-                             uint32_t Wpmax, uint32_t smax, uint32_t wait_limit, int grid,
-                             uint32_t *err, cudaStream_t st);
+                             uint32_t Wpmax, uint32_t smax, int grid, uint32_t *err,
+                             cudaStream_t st);
 cudaError_t launch_lits(const uint32_t *act, const ClassDev *cls, uint32_t classes,
                         uint32_t clauses, int32_t *lits, cudaStream_t st);
 cudaError_t launch_predict(const uint32_t *act, const int32_t *lits, const ClassDev *cls,

@@ -1,31 +1,46 @@
-// k_train_wpt: the fused train kernel with one CTA per unit of 8 clauses in
-// which every thread owns WPT consecutive words of all eight clauses
-// (capi.c:85-243 evaluation and feedback, automata.h:88-742 updates).
+// The fused train kernels for units of 8-bit automata whose rows have at most
+// 1,024 words (capi.c:85-243 evaluation and feedback, automata.h:88-742
+// updates).  A unit's automata stay on its SM while it trains.
 //
-// The action plane and the lowest RP count planes of the thread's words
-// live in its registers; the other 7 - RP count planes in shared memory.  A
-// unit's automata therefore never leave the SM while it trains (the
-// global-plane variant of k_train reads and writes every fed-back clause's
-// count planes through L2 on every sample), and because each thread updates
-// only its own words, no barrier separates one sample's feedback from the
-// next sample's evaluation.  Per active sample:
-//   1. the row arrives in a 3-slot shared-memory ring by TMA bulk copy
-//      (issued 2 samples ahead, mbarrier completion, no multicast);
-//   2. every thread counts its words' failed (and, for clauses updated
-//      since, included) literals of the eight clauses, warps reduce them
-//      and write one partial per warp; barrier;
-//   3. warp 0 sums the partials, forms votes, the clamped chunk vote and the
-//      eight feedback decisions from the pre-drawn chance values (the
-//      draw contract of k_train), writes four decision masks; barrier;
-//   4. Type Ib clauses (at most one per clause pair): all threads draw the
-//      picks into per-clause binary level counters in shared memory; barrier;
-//   5. every thread applies Type Ia / Ib / II to its own words of every
-//      fed-back clause, register and shared planes alike.
+//   k_train_wpt   every thread owns WPT consecutive words of all eight clauses
+//   k_train_spec  few units: eight warps evaluate eight samples at once
+//
+// What bounds them: integer issue (LOP3 at half rate, POPC at an eighth) and the
+// dependent chain of one sample's step.  Hence:
+//   - saturation is decided before any plane is written: a carry chain of one
+//     LOP3 per plane finds the bits that would overflow, then one LOP3 per
+//     plane applies the update to the others (count_step and its kin);
+//   - one body of update code serves all eight clauses, the planes addressed
+//     in shared memory: eight unrolled bodies (automata in registers) were 77 KB
+//     of code and half the warps waited for instructions (search rows: 127 ms
+//     against 69 ms); only rows above 64 words keep their lowest planes in
+//     registers, for room;
+//   - a sample's row words go straight to the thread that owns them by 4- to
+//     16-byte asynchronous copies, three samples ahead: no mbarrier stands
+//     between a copy and its use;
+//   - the failed-literal counts of two clauses share one 32-bit word, so a
+//     warp reduces eight clauses in four __reduce_add_sync;
+//   - the chance draws are turned into vote thresholds (feedback fires when
+//     the signed chunk vote is below the threshold) for a group of samples at
+//     once, outside the dependent chain;
+//   - a unit of one warp needs no CTA barrier at all; larger units add their
+//     counts into a rotating shared accumulator and pass one barrier per
+//     sample (a second one when the sample has Type Ib clauses), every warp
+//     taking the same decisions from it.
+// Measured (train calls, B200, before -> after): search rows of 49 words, 28.5M
+// active steps, 44.7 -> 25.7 ms (narrow rows 34.7 -> 17.4 ms); plain classifier
+// 8,000 samples x 10 epochs, 320 units, 15.0 -> 2.8 ms; encoder rows of 256
+// words 190 -> 156 ms; sparse classifier rows of 1,024 words 127 -> 105 ms.
 // The same rules and draws as k_train, so the same automata bit for bit.
 #include "tm_device.cuh"
 
 namespace tmb {
 
+namespace {
+
+constexpr int M7 = 7;      // count planes (8 state bits)
+constexpr int RING = 4;    // sample rows in flight per thread (3 ahead)
+constexpr int SC = 2;      // positions a thread examines per scan of the epoch order
 
 template <int WPT>
 struct WVec;
@@ -33,17 +48,6 @@ template <>
 struct WVec<1> {
   __device__ static void ld(const uint32_t *p, uint32_t (&v)[1]) { v[0] = *p; }
   __device__ static void st(uint32_t *p, const uint32_t (&v)[1]) { *p = v[0]; }
-};
-template <>
-struct WVec<2> {
-  __device__ static void ld(const uint32_t *p, uint32_t (&v)[2]) {
-    const uint2 t = *(const uint2 *)p;
-    v[0] = t.x;
-    v[1] = t.y;
-  }
-  __device__ static void st(uint32_t *p, const uint32_t (&v)[2]) {
-    *(uint2 *)p = make_uint2(v[0], v[1]);
-  }
 };
 template <>
 struct WVec<4> {
@@ -58,75 +62,760 @@ struct WVec<4> {
     *(uint4 *)p = make_uint4(v[0], v[1], v[2], v[3]);
   }
 };
+template <>
+struct WVec<2> {
+  __device__ static void ld(const uint32_t *p, uint32_t (&v)[2]) {
+    const uint2 t = *(const uint2 *)p;
+    v[0] = t.x;
+    v[1] = t.y;
+  }
+  __device__ static void st(uint32_t *p, const uint32_t (&v)[2]) {
+    *(uint2 *)p = make_uint2(v[0], v[1]);
+  }
+};
 
-// Shared-memory layout of one launch (byte offsets; planes are
-// [plane - RP][clause][Wp] words)
-__host__ __device__ inline void wpt_layout(uint32_t Wp, uint32_t NT, int RP, int IBS,
-                                           uint32_t ovf_cap, uint32_t *o) {
+// asynchronous copy of a thread's own row words (4, 8 or 16 bytes)
+template <int BYTES>
+__device__ __forceinline__ void cp_async_words(void *dst, const void *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(smem_u32(dst)), "l"(src),
+               "n"(BYTES)
+               : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_wait() {
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
+
+// philox with the key taken as new at every call: its ten round keys are then
+// computed there instead of being kept in (and spilled from) registers
+// across the sample loop.
+__device__ __forceinline__ void draw4(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3,
+                                      uint64_t key, uint32_t *o) {
+  asm volatile("" : "+l"(key));
+  philox(c0, c1, c2, c3, key, o);
+}
+
+// The updates below run on a thread's WPT words plane by plane, so that the
+// words' carry chains (one dependent LOP3 per plane) overlap.
+
+// +1 on the bits of `c0` outside `dm`, -1 on those inside it, both saturating
+// (automata.h:88-318).  A decrement is an increment of the complement, so the
+// carry runs through p ^ dm; bits whose carry leaves the action plane are
+// saturated and keep every plane.
+template <int N>
+__device__ __forceinline__ void count_step(uint32_t (&p)[M7][N], uint32_t (&a)[N],
+                                           const uint32_t (&c0)[N], const uint32_t (&dm)[N],
+                                           const uint32_t (&am)[N]) {
+  uint32_t c[M7 + 1][N], keep[N];
+#pragma unroll
+  for (int q = 0; q < N; q++) c[0][q] = c0[q];
+#pragma unroll
+  for (int b = 0; b < M7; b++)
+#pragma unroll
+    for (int q = 0; q < N; q++) c[b + 1][q] = c[b][q] & (p[b][q] ^ dm[q]);
+#pragma unroll
+  for (int q = 0; q < N; q++) {
+    const uint32_t ca = c[M7][q] & am[q];
+    keep[q] = ~(ca & (a[q] ^ dm[q]));
+    a[q] ^= ca & keep[q];
+  }
+#pragma unroll
+  for (int b = 0; b < M7; b++)
+#pragma unroll
+    for (int q = 0; q < N; q++) p[b][q] ^= c[b][q] & keep[q];
+}
+
+// +1 on bits whose automaton is not included (action 0 with one include bit,
+// so the carry into the action plane never saturates)
+template <int N>
+__device__ __forceinline__ void count_inc0(uint32_t (&p)[M7][N], uint32_t (&a)[N], uint32_t (&c)[N],
+                                           const uint32_t (&am)[N]) {
+#pragma unroll
+  for (int b = 0; b < M7; b++)
+#pragma unroll
+    for (int q = 0; q < N; q++) {
+      const uint32_t t = c[q] & p[b][q];
+      p[b][q] ^= c[q];
+      c[q] = t;
+    }
+#pragma unroll
+  for (int q = 0; q < N; q++) a[q] ^= c[q] & am[q];
+}
+
+// -1 on bits with action 0: the action plane stays, a borrow that reaches it
+// means the count was zero
+template <int N>
+__device__ __forceinline__ void count_dec0(uint32_t (&p)[M7][N], const uint32_t (&d)[N],
+                                           const uint32_t (&am)[N]) {
+  uint32_t c[M7 + 1][N], keep[N];
+#pragma unroll
+  for (int q = 0; q < N; q++) c[0][q] = d[q];
+#pragma unroll
+  for (int b = 0; b < M7; b++)
+#pragma unroll
+    for (int q = 0; q < N; q++) c[b + 1][q] = c[b][q] & ~p[b][q];
+#pragma unroll
+  for (int q = 0; q < N; q++) keep[q] = ~(c[M7][q] & am[q]);
+#pragma unroll
+  for (int b = 0; b < M7; b++)
+#pragma unroll
+    for (int q = 0; q < N; q++) p[b][q] ^= c[b][q] & keep[q];
+}
+
+// Saturating subtraction of m0 + 2 m1 per bit (Type Ib picks counted in two
+// binary levels): a two-bit subtractor, then the borrow through the higher
+// planes; bits whose borrow leaves the action plane end at zero.
+template <int N>
+__device__ __forceinline__ void count_sub(uint32_t (&p)[M7][N], uint32_t (&a)[N],
+                                          const uint32_t (&m0)[N], const uint32_t (&m1)[N],
+                                          const uint32_t (&am)[N]) {
+  uint32_t r[M7 + 1][N], keep[N];
+#pragma unroll
+  for (int q = 0; q < N; q++) r[1][q] = m0[q] & ~p[0][q];
+#pragma unroll
+  for (int q = 0; q < N; q++)
+    r[2][q] = (~p[1][q] & (m1[q] | r[1][q])) | (m1[q] & r[1][q]);
+#pragma unroll
+  for (int b = 2; b < M7; b++)
+#pragma unroll
+    for (int q = 0; q < N; q++) r[b + 1][q] = r[b][q] & ~p[b][q];
+#pragma unroll
+  for (int q = 0; q < N; q++) {
+    const uint32_t ra = r[M7][q] & am[q];
+    keep[q] = ~(ra & ~a[q]);
+    a[q] &= ~ra;
+    p[0][q] = (p[0][q] ^ m0[q]) & keep[q];
+    p[1][q] = (p[1][q] ^ m1[q] ^ r[1][q]) & keep[q];
+  }
+#pragma unroll
+  for (int b = 2; b < M7; b++)
+#pragma unroll
+    for (int q = 0; q < N; q++) p[b][q] = (p[b][q] ^ r[b][q]) & keep[q];
+}
+
+// automata.h:499-512: action AND the top include_bits - 1 count planes
+template <int N>
+__device__ __forceinline__ uint32_t included(const uint32_t (&p)[M7][N], uint32_t a, int q,
+                                             uint32_t ib) {
+#pragma unroll
+  for (int b = 0; b < M7; b++)
+    if (b + (int)ib > M7) a &= p[b][q];
+  return a;
+}
+
+// Vote thresholds of sample `ent` (index | positive << 31) for the eight
+// clauses.  Clause c's draw d fires iff floor(d 2T / 2^32) < T - v for a
+// positive sample, T + v for a negative one, v clamped to [-T, T]
+// (capi.c:217-242): iff v (or -v) < T - floor(d 2T / 2^32), a value in
+// (-T, T], so the clamp never decides.
+__device__ __forceinline__ void vote_thresholds(uint32_t ent, uint32_t ee, uint32_t g, uint32_t T,
+                                                uint64_t seed, int32_t *out) {
+  const uint32_t s = ent & 0x7FFFFFFFu;
+  uint32_t d[8];
+  draw4(s, ee, g, ST_CH0, seed, d);
+  draw4(s, ee, g, ST_CH1, seed, d + 4);
+  int32_t t[8];
+#pragma unroll
+  for (int c = 0; c < 8; c++) {
+    // draw 2p decides Type I of pair p, draw 2p + 1 Type II; a positive
+    // sample gives Type I to the even clause
+    const uint32_t dd = ((ent >> 31) != 0) == ((c & 1) == 0) ? d[c & ~1] : d[c | 1];
+    int64_t v = (int64_t)T - (int64_t)bounded64(dd, 2ull * T);
+    v = v > INT32_MAX ? INT32_MAX : (v <= INT32_MIN ? INT32_MIN + 1 : v);
+    t[c] = T ? (int32_t)v : INT32_MIN;
+  }
+  *(int4 *)out = make_int4(t[0], t[1], t[2], t[3]);
+  *(int4 *)(out + 4) = make_int4(t[4], t[5], t[6], t[7]);
+}
+
+// The picks of every Type Ib clause of `ibm` (capi.c:181-190), spread over
+// the unit's threads: counted per bit in two binary levels of the clause's
+// slot, larger counts as overflow entries worth 4 each (saturating
+// subtraction is order-free).  The four level-0 exchanges of a draw are
+// issued together; only draws that carry go on.
+template <uint32_t NT, uint32_t SW>
+__device__ __forceinline__ void draw_picks(uint32_t ibm, uint32_t sp, uint32_t ee, uint32_t g,
+                                           uint64_t seed, uint32_t npk, uint32_t nq,
+                                           uint32_t input_bits, uint32_t *lev, uint16_t *ovf,
+                                           uint32_t *oc, uint32_t ovf_cap) {
+  uint32_t clist = 0, nib = 0;
+  for (uint32_t cm = ibm; cm; cm &= cm - 1, nib++)
+    clist |= (uint32_t)(__ffs(cm) - 1) << (4 * nib);
+  const uint32_t total = nib * nq;
+  for (uint32_t it = threadIdx.x; it < total; it += NT) {
+    const uint32_t slot = (it >= nq) + (it >= 2 * nq) + (it >= 3 * nq);
+    const uint32_t q = it - slot * nq, c = (clist >> (4 * slot)) & 15u;
+    uint32_t *l0 = lev + slot * (2 * SW), *l1 = l0 + SW;
+    uint32_t r[4], mk[4], old[4];
+    draw4(sp, ee, g, ST_IB | (c << 20) | q, seed, r);
+    const uint32_t nv = npk - 4 * q;  // picks left: fewer than 4 in the last draw
+#pragma unroll
+    for (uint32_t z = 0; z < 4; z++) {
+      r[z] = __umulhi(r[z], input_bits);
+      mk[z] = z < nv ? 1u << (r[z] & 31) : 0u;
+      old[z] = atomicXor(&l0[r[z] >> 5], mk[z]);
+    }
+#pragma unroll
+    for (uint32_t z = 0; z < 4; z++) mk[z] &= old[z];
+    if (mk[0] | mk[1] | mk[2] | mk[3]) {
+#pragma unroll
+      for (uint32_t z = 0; z < 4; z++) old[z] = atomicXor(&l1[r[z] >> 5], mk[z]);
+#pragma unroll
+      for (uint32_t z = 0; z < 4; z++) mk[z] &= old[z];
+      if (mk[0] | mk[1] | mk[2] | mk[3]) {
+#pragma unroll
+        for (uint32_t z = 0; z < 4; z++)
+          if (mk[z]) {
+            const uint32_t k = atomicAdd(&oc[slot], 1u);
+            if (k < ovf_cap) ovf[slot * ovf_cap + k] = (uint16_t)r[z];
+          }
+      }
+    }
+  }
+}
+
+// Samples listed before a unit starts on them: enough that the threshold
+// pass (one sample per thread) and the row copies' start-up weigh little.
+__host__ __device__ constexpr uint32_t wpt_fill(uint32_t NT) {
+  return NT == 32 ? 96 : (NT == 64 ? 128 : NT);
+}
+
+// Shared-memory layout of a unit (byte offsets): NT threads, SW words per
+// row slot, IBS Type Ib slots.
+struct WptLayout {
+  uint32_t planes, ring, list, thr, acc, lev, ovf, misc, total;
+};
+__host__ __device__ constexpr WptLayout wpt_layout(uint32_t NT, uint32_t SW, int RP, int IBS,
+                                                   uint32_t ovf_cap) {
+  WptLayout L{};
   uint32_t at = 0;
   auto take = [&](uint32_t bytes) {
     const uint32_t r = at;
-    at += (bytes + 127) / 128 * 128;
+    at += (bytes + 15) / 16 * 16;
     return r;
   };
-  o[0] = take((7 - RP) * 8 * Wp * 4);               // planes
-  o[1] = take(TM_RING * Wp * 4);                    // ring
-  o[2] = take(TM_RING * 8);                         // barriers
-  o[3] = take(NT * 4);                              // list_s
-  o[4] = take(NT * 8 * 4);                          // list_d
-  o[5] = take((NT / 32) * 16 * 4);                  // partials
-  o[6] = take(IBS * 2 * Wp * 4);                    // Type Ib levels
-  o[7] = take(IBS * ovf_cap * 4);                   // Type Ib overflow entries
-  o[8] = take(64 * 4);                              // misc
-  o[9] = at;                                        // total
+  L.planes = take((8 - RP) * 8 * SW * 4);
+  L.ring = take(RING * SW * 4);
+  L.list = take((wpt_fill(NT) + SC * NT) * 4);
+  L.thr = take(NT * 8 * 4);
+  L.acc = take(3 * 16 * 4);
+  L.lev = take(IBS * 2 * SW * 4);
+  L.misc = take(64 * 4);
+  L.ovf = take(IBS * ovf_cap * 2);
+  L.total = at;
+  return L;
 }
 
-// misc: [0] unit, [1..32] warp live counts, [40..43] decision masks,
-// [44] abort, [48..51] overflow counts
-// NT threads per unit, WPT words per thread, RP count planes in registers,
-// MINB CTAs per SM the registers are sized for, IBS Type Ib level-counter
-// slots (a sample with more Ib clauses takes further rounds)
-template <int NT, int WPT, int RP, int MINB, int IBS>
+}  // namespace
+
+// misc: [0] unit, [8..39] live counts of a scan, [48..55] overflow counts (2 parities x 4)
+// NT threads per unit (32: the one-warp form) of WPT words, SW words per
+// row slot (at most NT * WPT, at least the widest row), RP count planes in
+// registers, MINB CTAs per SM the registers are sized for.
+template <int NT, int WPT, int SW, int RP, int MINB>
 __global__ void __launch_bounds__(NT, MINB)
     k_train_wpt(const TrainDev *__restrict__ machines, const WorkItem *__restrict__ work,
                 uint32_t nwork, uint32_t *__restrict__ counter, uint32_t e_begin, uint32_t e_end,
-                uint32_t Wpmax, uint32_t ovf_cap, uint32_t wait_limit, uint32_t *__restrict__ err) {
-  constexpr int NW = NT / 32;
-  constexpr int M7 = 7;  // count planes (8 state bits)
+                uint32_t ovf_cap, uint32_t *__restrict__ err) {
+  constexpr bool ONE = NT == 32;
+  constexpr uint32_t NW = NT / 32;
+  constexpr int IBS = 4;       // a sample has at most one Type I clause per pair
+  constexpr int SP = 8 - RP;   // planes in shared memory: count planes RP..6, then the actions
+  constexpr uint32_t FULL = 0xFFFFFFFFu;
   extern __shared__ __align__(128) uint8_t smem[];
-  uint32_t o[10];
-  wpt_layout(Wpmax, NT, RP, IBS, ovf_cap, o);
-  uint32_t *splanes = (uint32_t *)(smem + o[0]);
-  uint32_t *ring = (uint32_t *)(smem + o[1]);
-  uint64_t *bars = (uint64_t *)(smem + o[2]);
-  uint32_t *list_s = (uint32_t *)(smem + o[3]);
-  uint32_t *list_d = (uint32_t *)(smem + o[4]);
-  uint32_t *partial = (uint32_t *)(smem + o[5]);
-  uint32_t *lev = (uint32_t *)(smem + o[6]);
-  uint32_t *ovf = (uint32_t *)(smem + o[7]);
-  uint32_t *misc = (uint32_t *)(smem + o[8]);
+  const WptLayout o = wpt_layout(NT, SW, RP, IBS, ovf_cap);
   const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t w0 = tid * WPT;  // this thread's first word
-  if (tid == 0) {
-    for (int r = 0; r < TM_RING; r++) mbar_init(&bars[r], 1);
-    mbar_fence_init();
-    misc[44] = 0;
+  // threads past the row slots own no words: they load word 0's (under masks
+  // that are zero) and store nothing
+  const uint32_t ws = w0 < SW ? w0 : 0;
+  uint32_t *splanes = (uint32_t *)(smem + o.planes) + ws;
+  uint32_t *ring = (uint32_t *)(smem + o.ring) + ws;
+  uint32_t *list = (uint32_t *)(smem + o.list);
+  int32_t *thr = (int32_t *)(smem + o.thr);
+  uint32_t *acc = (uint32_t *)(smem + o.acc);
+  uint32_t *lev = (uint32_t *)(smem + o.lev);
+  uint16_t *ovf = (uint16_t *)(smem + o.ovf);
+  uint32_t *misc = (uint32_t *)(smem + o.misc);
+  auto sync = [] {
+    if constexpr (ONE) __syncwarp();
+    else __syncthreads();
+  };
+  for (uint32_t i = tid; i < IBS * 2 * SW; i += NT) lev[i] = 0;
+  if (tid < 8) misc[48 + tid] = 0;
+  // lane c of every warp decides clause c (lanes above 8 repeat them)
+  const uint32_t cl = lane & 7;
+  const int32_t sign = lane < 8 ? ((lane & 1) ? -1 : 1) : 0;
+  uint32_t step = 0;  // parity of the overflow counts, ring slot
+  uint32_t ab = 0;    // accumulator of this step
+
+  while (true) {
+    uint32_t u = 0;
+    if (tid == 0) {
+      // the next unit, passing over those of machines whose gate is closed
+      u = atomicAdd(counter, 1u);
+      while (u < nwork) {
+        const uint32_t *gt = machines[work[u].m].gate;
+        if (!gt || *gt) break;
+        u = atomicAdd(counter, 1u);
+      }
+      if (!ONE) misc[0] = u;
+    }
+    if (ONE) {
+      u = __shfl_sync(FULL, u, 0);
+    } else {
+      if (tid < 48) acc[tid] = 0;
+      __syncthreads();
+      u = misc[0];
+      __syncthreads();
+    }
+    if (u >= nwork) break;
+    const WorkItem wi = work[u];
+    const TrainDev &M = machines[wi.m];
+    const ClassDev C = M.cls[wi.h];
+    const uint32_t Wp = C.Wp, W = C.W;
+    const uint32_t g = wi.h * M.clause_chunks + wi.k;
+    uint32_t *gact = M.act + C.act_off + (uint64_t)wi.k * 8 * Wp + w0;
+    uint32_t *gcnt = M.cnt + C.cnt_off + (uint64_t)wi.k * 8 * M7 * Wp + w0;
+    // ---- the unit's automata onto the SM ------------------------------------
+    uint32_t pl[8][RP > 0 ? RP : 1][WPT];
+    const bool mine = w0 < Wp;  // Wp is a multiple of 4, so of WPT
+#pragma unroll
+    for (int c = 0; c < 8; c++)
+#pragma unroll
+      for (int b = 0; b < 8; b++) {
+        uint32_t t[WPT] = {};
+        if (mine) WVec<WPT>::ld(b < M7 ? gcnt + (c * M7 + b) * Wp : gact + c * Wp, t);
+        if (b < RP) {
+#pragma unroll
+          for (int q = 0; q < WPT; q++) pl[c][b < RP ? b : 0][q] = t[q];
+        } else if (w0 < SW) {
+          WVec<WPT>::st(splanes + (c * SP + b - RP) * SW, t);
+        }
+      }
+    uint32_t vm[WPT], em[WPT], am[WPT];
+#pragma unroll
+    for (int q = 0; q < WPT; q++) {
+      vm[q] = word_mask(w0 + q, W, C.vmask);
+      em[q] = word_mask(w0 + q, W, C.emask);
+      am[q] = word_mask(w0 + q, W, C.amask);
+    }
+    // this thread's words of clause c, c known at run time (one body of update
+    // code for all eight clauses keeps the kernel in the instruction cache):
+    // the register planes through a branch to the clause's registers (the
+    // empty asm keeps it a branch: selects would read all eight), the others
+    // by address
+#define TM_CLAUSES(X) X(0) X(1) X(2) X(3) X(4) X(5) X(6) X(7)
+    auto gather = [&](uint32_t c, uint32_t (&p)[M7][WPT], uint32_t (&a)[WPT]) {
+      const uint32_t *base = splanes + c * (SP * SW);
+#pragma unroll
+      for (int b = RP; b < 8; b++) {
+        uint32_t t[WPT];
+        WVec<WPT>::ld(base + (b - RP) * SW, t);
+#pragma unroll
+        for (int q = 0; q < WPT; q++) {
+          if (b < M7) p[b < M7 ? b : 0][q] = t[q];
+          else a[q] = t[q];
+        }
+      }
+      if constexpr (RP > 0) {
+#define TM_IN(K)                                                                         \
+  case K:                                                                                \
+    asm volatile("");                                                                    \
+    _Pragma("unroll") for (int q = 0; q < WPT; q++)                                      \
+        _Pragma("unroll") for (int b = 0; b < RP; b++) p[b][q] = pl[K][b][q];            \
+    break;
+        switch (c) { TM_CLAUSES(TM_IN) }
+#undef TM_IN
+      }
+    };
+    auto scatter = [&](uint32_t c, const uint32_t (&p)[M7][WPT], const uint32_t (&a)[WPT]) {
+      uint32_t *base = splanes + c * (SP * SW);
+      if (mine) {
+#pragma unroll
+        for (int b = RP; b < 8; b++) {
+          uint32_t t[WPT];
+#pragma unroll
+          for (int q = 0; q < WPT; q++) t[q] = b < M7 ? p[b < M7 ? b : 0][q] : a[q];
+          WVec<WPT>::st(base + (b - RP) * SW, t);
+        }
+      }
+      if constexpr (RP > 0) {
+#define TM_OUT(K)                                                                        \
+  case K:                                                                                \
+    asm volatile("");                                                                    \
+    _Pragma("unroll") for (int q = 0; q < WPT; q++)                                      \
+        _Pragma("unroll") for (int b = 0; b < RP; b++) pl[K][b][q] = p[b][q];            \
+    break;
+        switch (c) { TM_CLAUSES(TM_OUT) }
+#undef TM_OUT
+      }
+    };
+    // this warp's share of clause c's literal count
+    auto lits_of = [&](const uint32_t (&a)[WPT]) {
+      uint32_t l = 0;
+#pragma unroll
+      for (int q = 0; q < WPT; q++) l += __popc(a[q] & em[q]);
+      return __reduce_add_sync(FULL, l);
+    };
+    const uint32_t tol = M.tol, maxlit = M.maxlit, ib = M.ib, n = M.n, type = M.type;
+    const uint64_t seed = M.seed;
+    const uint32_t npk = C.s_picks, nq = (npk + 3) >> 2, input_bits = C.input_bits;
+    const uint32_t ep_end = e_end < M.epochs ? e_end : M.epochs;
+    const uint32_t *xbase = M.x + C.x_off + w0;
+    // literal counts: lane c's clause; in the multi-warp form each warp's
+    // share waits in lane 4 + c for the next exchange
+    uint32_t dirty = 0xFFu, L = 0, lval = 0, incM = 0;
+    int32_t cap = 0;
+#pragma unroll
+    for (int c = 0; c < 8; c++) {
+      uint32_t a[WPT];
+      WVec<WPT>::ld(splanes + (c * SP + SP - 1) * SW, a);
+      const uint32_t l = lits_of(a);
+      if (ONE) L = cl == (uint32_t)c ? l : L;
+      else lval = lane == 4u + c ? l : lval;
+    }
+    auto settle = [&]() {  // the vote cap of lane c's clause, and the increment mask
+      cap = (int32_t)(L == 0 || L > tol ? tol : L);
+      incM = __ballot_sync(FULL, L <= maxlit);
+    };
+    if (ONE) settle();
+    uint64_t nsteps = 0;
+
+    for (uint32_t e = e_begin; e < ep_end; e++) {
+      const uint32_t ee = M.epoch_base + e;
+      const uint32_t *perm = M.perm + (uint64_t)(e - e_begin) * n;
+      uint32_t at = 0;  // next position of the epoch order
+      while (at < n) {
+        // ---- the next samples this unit trains on ---------------------------
+        // Skip decisions (capi.c:215) do not depend on the automata: scan
+        // positions until the list holds enough samples, in order.
+        uint32_t cnt = 0;
+        while (at < n && cnt < wpt_fill(NT)) {
+          uint32_t s[SC], y[SC], bal[SC];
+#pragma unroll
+          for (int j = 0; j < SC; j++) {
+            const uint32_t i = at + j * NT + tid;
+            s[j] = i < n ? perm[i] : FULL;
+          }
+#pragma unroll
+          for (int j = 0; j < SC; j++) {
+            y[j] = 0;
+            if (s[j] != FULL) {
+              if (type == 0) y[j] = (uint32_t)M.labels[s[j]] == wi.h;
+              else y[j] = (M.codes[(uint64_t)s[j] * M.code_bytes + (wi.h >> 3)] >> (wi.h & 7)) & 1u;
+            }
+          }
+#pragma unroll
+          for (int j = 0; j < SC; j++) {
+            bool live = s[j] != FULL;
+            if (live && type == 0 && !y[j]) {
+              uint32_t r[4];
+              draw4(s[j], ee, g, ST_NEG, seed, r);
+              live = (uint64_t)r[0] >= M.thr_neg;
+            }
+            bal[j] = __ballot_sync(FULL, live);
+          }
+          const uint32_t below = (1u << lane) - 1u;
+          if (ONE) {
+#pragma unroll
+            for (int j = 0; j < SC; j++) {
+              if ((bal[j] >> lane) & 1u) list[cnt + __popc(bal[j] & below)] = s[j] | (y[j] << 31);
+              cnt += __popc(bal[j]);
+            }
+          } else {
+            if (lane == 0)
+#pragma unroll
+              for (int j = 0; j < SC; j++) misc[8 + j * NW + warp] = __popc(bal[j]);
+            __syncthreads();
+            // order: scan j, then warp, then lane
+            const uint32_t own = lane < SC * NW ? misc[8 + lane] : 0;
+            uint32_t inc = own;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+              const uint32_t t = __shfl_up_sync(FULL, inc, d);
+              if (lane >= (uint32_t)d) inc += t;
+            }
+#pragma unroll
+            for (int j = 0; j < SC; j++) {
+              const uint32_t off = __shfl_sync(FULL, inc - own, j * NW + warp);
+              if ((bal[j] >> lane) & 1u)
+                list[cnt + off + __popc(bal[j] & below)] = s[j] | (y[j] << 31);
+            }
+            cnt += __shfl_sync(FULL, inc, 31);
+            __syncthreads();
+          }
+          at += SC * NT;
+        }
+        sync();
+        nsteps += cnt;
+        // rows of the first samples of the list
+        auto fetch = [&](uint32_t a) {
+          if (a < cnt && mine)
+            cp_async_words<WPT * 4>(ring + ((step + a) & (RING - 1)) * SW,
+                                    xbase + (uint64_t)(list[a] & 0x7FFFFFFFu) * Wp);
+          cp_commit();
+        };
+        if (cnt) {
+#pragma unroll
+          for (uint32_t a = 0; a < RING - 1; a++) fetch(a);
+        }
+        for (uint32_t g0 = 0; g0 < cnt; g0 += NT) {
+          // ---- vote thresholds of a group of samples --------------------------
+          if (g0) sync();
+          if (g0 + tid < cnt) vote_thresholds(list[g0 + tid], ee, g, M.T, seed, thr + tid * 8);
+          sync();
+          const uint32_t ge = cnt - g0 < NT ? cnt - g0 : NT;
+          // ---- sequential per-sample steps ------------------------------------
+          for (uint32_t a = 0; a < ge; a++) {
+            fetch(g0 + a + RING - 1);
+            const uint32_t ent = list[g0 + a];
+            const int32_t tc = thr[a * 8 + cl];
+            const uint32_t par = (step + g0 + a) & 1u;
+            cp_wait<RING - 1>();
+            uint32_t x[WPT];
+            WVec<WPT>::ld(ring + ((step + g0 + a) & (RING - 1)) * SW, x);
+            // failed literals of the eight clauses, two per word
+            uint32_t pk[4];
+#pragma unroll
+            for (int c = 0; c < 8; c += 2) {
+              uint32_t f0 = 0, f1 = 0, a0[WPT], a1[WPT];
+              WVec<WPT>::ld(splanes + (c * SP + SP - 1) * SW, a0);
+              WVec<WPT>::ld(splanes + ((c + 1) * SP + SP - 1) * SW, a1);
+#pragma unroll
+              for (int q = 0; q < WPT; q++) {
+                f0 += __popc(a0[q] & em[q] & ~x[q]);
+                f1 += __popc(a1[q] & em[q] & ~x[q]);
+              }
+              pk[c >> 1] = __reduce_add_sync(FULL, f0 + (f1 << 16));
+            }
+            uint32_t pr = (lane & 2) ? ((lane & 1) ? pk[3] : pk[2]) : ((lane & 1) ? pk[1] : pk[0]);
+            if (ONE) {
+              pr = (lane & 4) ? ((lane & 2) ? pk[3] : pk[2]) : ((lane & 2) ? pk[1] : pk[0]);
+            } else {
+              // accumulator ab is zero since step - 2; the one of step + 2
+              // was read before this step's barrier and is cleared after it
+              if (lane < 12) atomicAdd(&acc[ab * 16 + lane], lane < 4 ? pr : lval);
+              __syncthreads();
+              const uint32_t *A = acc + ab * 16;
+              pr = A[cl >> 1];
+              if (dirty) {
+                const uint32_t l = A[4 + cl];
+                if ((dirty >> cl) & 1u) L = l;
+                settle();
+              }
+              const uint32_t nx2 = ab == 0 ? 2 : ab - 1;
+              if (tid < 16) acc[nx2 * 16 + tid] = 0;
+              // the previous step's overflow counts, for the next step
+              if (tid < IBS) misc[48 + (par ^ 1u) * IBS + tid] = 0;
+              ab = ab == 2 ? 0 : ab + 1;
+            }
+            const uint32_t F = (lane & 1) ? pr >> 16 : pr & 0xFFFFu;
+            // votes (capi.c:110-118), signed by clause parity (:148-161)
+            int32_t vote = cap - (int32_t)F;
+            vote = vote < 0 ? 0 : vote;
+            const int32_t v = (int32_t)__reduce_add_sync(FULL, (uint32_t)(vote * sign));
+            const bool pa = ent >> 31;
+            const uint32_t fm = __ballot_sync(FULL, (pa ? v : -v) < tc) & 0xFFu;
+            const uint32_t vt = __ballot_sync(FULL, vote > 0);
+            const uint32_t t1 = pa ? 0x55u : 0xAAu;  // Type I clauses
+            const uint32_t ibm = fm & t1 & ~vt;      // Type Ib (capi.c:181-190)
+            const uint32_t fbm = fm & vt;            // Type Ia and II
+            dirty = 0;
+            if (!(ibm | fbm)) continue;
+            const uint32_t sp = ent & 0x7FFFFFFFu;
+            uint32_t *oc = misc + 48 + par * IBS;
+            if (ibm) {
+              if (ONE) __syncwarp();
+              draw_picks<NT, SW>(ibm, sp, ee, g, seed, npk, nq, input_bits, lev, ovf, oc, ovf_cap);
+              sync();
+            }
+#pragma unroll 1
+            for (uint32_t cm = ibm | fbm; cm; cm &= cm - 1) {
+              const uint32_t c = __ffs(cm) - 1;
+              uint32_t p[M7][WPT], ac[WPT];
+              gather(c, p, ac);
+              const bool is1 = (t1 >> c) & 1u;
+              bool changed = true;  // false: the action plane is as it was
+              if ((ibm >> c) & 1u) {
+                const uint32_t slot = __popc(ibm & ((1u << c) - 1u));
+                uint32_t *l0 = lev + slot * (2 * SW) + ws, *l1 = l0 + SW;
+                uint32_t m0[WPT], m1[WPT];
+                WVec<WPT>::ld(l0, m0);
+                WVec<WPT>::ld(l1, m1);
+                if (mine) {
+                  const uint32_t zero[WPT] = {};
+                  WVec<WPT>::st(l0, zero);
+                  WVec<WPT>::st(l1, zero);
+                } else {
+#pragma unroll
+                  for (int q = 0; q < WPT; q++) m0[q] = m1[q] = 0;
+                }
+                // an overflow entry is worth 4: twice a level-1 count
+                const uint32_t no = 2 * min(oc[slot], ovf_cap);
+                for (uint32_t t = 0;; t++) {
+                  count_sub(p, ac, m0, m1, am);
+                  if (t >= no) break;
+                  const uint32_t bit = ovf[slot * ovf_cap + (t >> 1)];
+#pragma unroll
+                  for (int q = 0; q < WPT; q++) {
+                    m0[q] = 0;
+                    m1[q] = (bit >> 5) == w0 + q ? 1u << (bit & 31) : 0u;
+                  }
+                }
+              } else {
+                // Type Ia (capi.c:177-180): inc where x = 1 (if L <= maximum),
+                // dec where x = 0 and not included.  Type II (capi.c:192-196):
+                // inc where x = 0 and not included.
+                const bool incx = is1 && ((incM >> c) & 1u);
+                uint32_t nx[WPT];
+                if (ib == 1 && !incx) {
+#pragma unroll
+                  for (int q = 0; q < WPT; q++) nx[q] = ~(x[q] | ac[q]) & vm[q];
+                  if (is1) count_dec0(p, nx, am);
+                  else count_inc0(p, ac, nx, am);
+                  changed = !is1;
+                } else {
+                  uint32_t c0[WPT], dm[WPT];
+#pragma unroll
+                  for (int q = 0; q < WPT; q++) {
+                    nx[q] = ~(x[q] | included(p, ac[q], q, ib)) & vm[q];
+                    c0[q] = nx[q] | (incx ? x[q] & vm[q] : 0u);
+                    dm[q] = is1 ? nx[q] : 0u;
+                  }
+                  count_step(p, ac, c0, dm, am);
+                }
+              }
+              scatter(c, p, ac);
+              if (changed) {
+                dirty |= 1u << c;
+                const uint32_t l = lits_of(ac);
+                if (ONE) L = cl == c ? l : L;
+                else lval = lane == 4u + c ? l : lval;
+              }
+            }
+            if (ONE) {
+              if (ibm) {
+                __syncwarp();
+                if (lane < IBS) oc[lane] = 0;
+              }
+              if (dirty) settle();
+            }
+          }
+        }
+        step += cnt;
+        sync();
+      }
+    }
+    // ---- the unit's automata back to global memory ----------------------------
+    // (the row stride read again, so that the 64 addresses of the load above
+    // are not kept, spilled, until here)
+    uint32_t Wo = Wp;
+    asm volatile("" : "+r"(Wo));
+    if (mine) {
+#pragma unroll
+      for (int c = 0; c < 8; c++)
+#pragma unroll
+        for (int b = 0; b < 8; b++) {
+          uint32_t t[WPT];
+          if (b < RP) {
+#pragma unroll
+            for (int q = 0; q < WPT; q++) t[q] = pl[c][b < RP ? b : 0][q];
+          } else {
+            WVec<WPT>::ld(splanes + (c * SP + b - RP) * SW, t);
+          }
+          WVec<WPT>::st(b < M7 ? gcnt + (c * M7 + b) * Wo : gact + c * Wo, t);
+        }
+    }
+    if (tid == 0 && nsteps) atomicAdd((unsigned long long *)(err + 2), (unsigned long long)nsteps);
   }
-  for (uint32_t i = tid; i < IBS * 2 * Wpmax; i += NT) lev[i] = 0;
-  if (tid < IBS) misc[48 + tid] = 0;
-  __syncthreads();
-  uint32_t gs = 0, issued = 0;
-  bool aborted = false;
+}
+
+// ---------------------------------------------------------------------------
+// k_train_spec: for launches of few units, whose time is the dependent chain
+// of one unit's samples.  A CTA of eight warps holds a unit in shared memory
+// and works in rounds: warp w evaluates sample b + w of the unit's list
+// (votes and feedback decisions of all eight clauses) against the same
+// automata, one barrier publishes the eight results, and the samples'
+// feedback is applied in order, warp j updating clause j.  Evaluation reads
+// only the action planes, so a sample's feedback leaves the later results
+// valid unless it may move an action (Type II, Type Ib, Type Ia with
+// increments or several include bits): then the round ends after that sample
+// and the others are evaluated again.  Bit for bit the sequential rule.
+// Rows arrive in a ring of R slots, at least two rounds ahead.
+// ---------------------------------------------------------------------------
+namespace {
+
+constexpr int SPW = 8;              // warps per unit: samples per round, clauses
+constexpr uint32_t SP_NT = 32 * SPW;
+constexpr uint32_t SP_SC = 4;       // positions a thread examines per scan
+constexpr uint32_t SP_FILL = 128;
+
+struct SpecLayout {
+  uint32_t planes, ring, list, thr, lev, ovf, misc, total;
+};
+__host__ __device__ constexpr SpecLayout spec_layout(uint32_t SW, uint32_t R, uint32_t ovf_cap) {
+  SpecLayout L{};
+  uint32_t at = 0;
+  auto take = [&](uint32_t bytes) {
+    const uint32_t r = at;
+    at += (bytes + 15) / 16 * 16;
+    return r;
+  };
+  L.planes = take(8 * 8 * SW * 4);
+  L.ring = take(R * SW * 4);
+  L.list = take((SP_FILL + SP_SC * SP_NT) * 4);
+  L.thr = take(SP_NT * 8 * 4);
+  L.lev = take(4 * 2 * SW * 4);
+  L.misc = take(96 * 4);
+  L.ovf = take(4 * ovf_cap * 2);
+  L.total = at;
+  return L;
+}
+
+}  // namespace
+
+// misc: [0] unit, [8..39] live counts of a scan, [48..55] overflow counts
+// (2 parities x 4), [56..63] literal counts, [64..79] results (2 x 8)
+template <int SW, int R, int MINB>
+__global__ void __launch_bounds__(SP_NT, MINB)
+    k_train_spec(const TrainDev *__restrict__ machines, const WorkItem *__restrict__ work,
+                 uint32_t nwork, uint32_t *__restrict__ counter, uint32_t e_begin, uint32_t e_end,
+                 uint32_t ovf_cap, uint32_t *__restrict__ err) {
+  constexpr int NK = SW / 64;       // word pairs per lane
+  constexpr uint32_t FULL = 0xFFFFFFFFu;
+  // rows a round may need were issued two rounds before it (R = 32) or one
+  constexpr int AHEAD = R >= 32 ? 1 : 0;
+  extern __shared__ __align__(128) uint8_t smem[];
+  const SpecLayout o = spec_layout(SW, R, ovf_cap);
+  uint32_t *planes = (uint32_t *)(smem + o.planes);  // [clause][count planes 0..6, action][SW]
+  uint32_t *ring = (uint32_t *)(smem + o.ring);
+  uint32_t *list = (uint32_t *)(smem + o.list);
+  int32_t *thr = (int32_t *)(smem + o.thr);
+  uint32_t *lev = (uint32_t *)(smem + o.lev);
+  uint16_t *ovf = (uint16_t *)(smem + o.ovf);
+  uint32_t *misc = (uint32_t *)(smem + o.misc);
+  uint32_t *lits = misc + 56, *res = misc + 64;
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t cl = lane & 7;  // lane c decides clause c
+  const int32_t sign = lane < 8 ? ((lane & 1) ? -1 : 1) : 0;
+  const uint32_t jbit = 1u << warp;
+  uint32_t *own = planes + warp * (8 * SW) + 2 * lane;  // this warp's clause, this lane's words
+  for (uint32_t i = tid; i < 8 * SW; i += SP_NT) lev[i] = 0;
+  if (tid < 8) misc[48 + tid] = 0;
+  uint32_t par = 0, opar = 0, win = SPW;
+
   while (true) {
     if (tid == 0) {
       // the next unit, passing over those of machines whose gate is closed
-      uint32_t v = atomicAdd(counter, 1u);
-      while (v < nwork) {
-        const uint32_t *gt = machines[work[v].m].gate;
+      uint32_t u = atomicAdd(counter, 1u);
+      while (u < nwork) {
+        const uint32_t *gt = machines[work[u].m].gate;
         if (!gt || *gt) break;
-        v = atomicAdd(counter, 1u);
+        u = atomicAdd(counter, 1u);
       }
-      misc[0] = v;
+      misc[0] = u;
     }
     __syncthreads();
     const uint32_t u = misc[0];
@@ -136,368 +825,318 @@ __global__ void __launch_bounds__(NT, MINB)
     const ClassDev C = M.cls[wi.h];
     const uint32_t Wp = C.Wp, W = C.W;
     const uint32_t g = wi.h * M.clause_chunks + wi.k;
-    uint32_t *gact = M.act + C.act_off + (uint64_t)wi.k * 8 * Wp;
-    uint32_t *gcnt = M.cnt + C.cnt_off + (uint64_t)wi.k * 8 * M7 * Wp;
-    // ---- the unit's automata onto the SM ------------------------------------
-    uint32_t act[8][WPT], pl[8][RP > 0 ? RP : 1][WPT];
-    const bool mine = w0 < Wp;  // Wp is a multiple of 4 and of WPT
+    uint32_t *gact = M.act + C.act_off + ((uint64_t)wi.k * 8 + warp) * Wp + 2 * lane;
+    uint32_t *gcnt = M.cnt + C.cnt_off + ((uint64_t)wi.k * 8 + warp) * M7 * Wp + 2 * lane;
+    // masks of this lane's words: only a row's last word and the words past
+    // it have masks other than all ones
+    uint32_t vm[NK][2], em[NK][2], am[NK][2];
 #pragma unroll
-    for (int c = 0; c < 8; c++) {
-      if (mine) {
-        WVec<WPT>::ld(gact + c * Wp + w0, act[c]);
+    for (int k = 0; k < NK; k++)
 #pragma unroll
-        for (int b = 0; b < RP; b++) WVec<WPT>::ld(gcnt + (c * M7 + b) * Wp + w0, pl[c][b]);
-      } else {
+      for (int q = 0; q < 2; q++) {
+        const uint32_t w = 64 * k + 2 * lane + q;
+        vm[k][q] = word_mask(w, W, C.vmask);
+        em[k][q] = word_mask(w, W, C.emask);
+        am[k][q] = word_mask(w, W, C.amask);
+      }
+    // ---- the unit's automata onto the SM: warp j loads clause j ---------------
+    auto recount = [&]() {  // literal count of this warp's clause
+      uint32_t l = 0;
 #pragma unroll
-        for (int k = 0; k < WPT; k++) {
-          act[c][k] = 0;
+      for (int k = 0; k < NK; k++) {
+        const uint2 a = *(const uint2 *)(own + M7 * SW + 64 * k);
+        l += __popc(a.x & em[k][0]) + __popc(a.y & em[k][1]);
+      }
+      l = __reduce_add_sync(FULL, l);
+      if (lane == 0) lits[warp] = l;
+    };
 #pragma unroll
-          for (int b = 0; b < RP; b++) pl[c][b][k] = 0;
-        }
+    for (int k = 0; k < NK; k++) {
+      const bool mine = 64 * k + 2 * lane < Wp;
+#pragma unroll
+      for (int b = 0; b < 8; b++) {
+        uint2 t = make_uint2(0, 0);
+        if (mine) t = *(const uint2 *)((b < M7 ? gcnt + b * Wp : gact) + 64 * k);
+        *(uint2 *)(own + b * SW + 64 * k) = t;
       }
     }
-    for (uint32_t i = tid; i < (uint32_t)(M7 - RP) * 8 * Wp; i += NT) {
-      const uint32_t bb = i / (8 * Wp), rem = i - bb * 8 * Wp, c = rem / Wp, w = rem - c * Wp;
-      splanes[i] = gcnt[(c * M7 + RP + bb) * Wp + w];
-    }
-    uint32_t vm[WPT], em[WPT], am[WPT];
-#pragma unroll
-    for (int k = 0; k < WPT; k++) {
-      vm[k] = word_mask(w0 + k, W, C.vmask);
-      em[k] = word_mask(w0 + k, W, C.emask);
-      am[k] = word_mask(w0 + k, W, C.amask);
-    }
+    recount();
     __syncthreads();
-    const uint32_t T = M.T;
-    const uint64_t T2 = 2ull * T;
+    const uint32_t tol = M.tol, maxlit = M.maxlit, ib = M.ib, n = M.n, type = M.type;
+    const uint64_t seed = M.seed;
+    const uint32_t npk = C.s_picks, nq = (npk + 3) >> 2, input_bits = C.input_bits;
     const uint32_t ep_end = e_end < M.epochs ? e_end : M.epochs;
     const uint32_t *xbase = M.x + C.x_off;
-    uint32_t dirty = 0xFFu;  // clauses whose literal counts must be recounted
-    uint32_t lcache = 0;     // warp 0, lane c < 8: literal count of clause c
-    // the count planes of this thread's words of clause c: registers for
-    // planes below RP, shared memory for the others
-    auto gather = [&](int c, uint32_t (&p)[WPT][M7]) {
-#pragma unroll
-      for (int b = 0; b < M7; b++) {
-        if (b < RP) {
-#pragma unroll
-          for (int q = 0; q < WPT; q++) p[q][b] = pl[c][b < RP ? b : 0][q];
-        } else {
-          uint32_t t[WPT];
-          WVec<WPT>::ld(splanes + ((b - RP) * 8 + c) * Wp + w0, t);
-#pragma unroll
-          for (int q = 0; q < WPT; q++) p[q][b] = t[q];
-        }
-      }
-    };
-    auto scatter = [&](int c, const uint32_t (&p)[WPT][M7]) {
-#pragma unroll
-      for (int b = 0; b < M7; b++) {
-        if (b < RP) {
-#pragma unroll
-          for (int q = 0; q < WPT; q++) pl[c][b < RP ? b : 0][q] = p[q][b];
-        } else {
-          uint32_t t[WPT];
-#pragma unroll
-          for (int q = 0; q < WPT; q++) t[q] = p[q][b];
-          WVec<WPT>::st(splanes + ((b - RP) * 8 + c) * Wp + w0, t);
-        }
-      }
-    };
+    uint64_t nsteps = 0;
 
-    for (uint32_t e = e_begin; e < ep_end && !aborted; e++) {
+    for (uint32_t e = e_begin; e < ep_end; e++) {
       const uint32_t ee = M.epoch_base + e;
-      const uint32_t *perm = M.perm + (uint64_t)(e - e_begin) * M.n;
-      for (uint32_t base = 0; base < M.n && !aborted; base += NT) {
-        // ---- batch phase: skip decisions and chance draws (as k_train) -------
-        const uint32_t i = base + tid;
-        bool live = false;
-        uint32_t s = 0, pos = 0;
-        if (i < M.n) {
-          s = perm[i];
-          if (M.type == 0) {
-            pos = (uint32_t)M.labels[s] == wi.h;
-            live = pos;
-            if (!pos) {
+      const uint32_t *perm = M.perm + (uint64_t)(e - e_begin) * n;
+      uint32_t at = 0;  // next position of the epoch order
+      while (at < n) {
+        // ---- the next samples this unit trains on, in order -------------------
+        uint32_t cnt = 0;
+        while (at < n && cnt < SP_FILL) {
+          uint32_t s[SP_SC], y[SP_SC], bal[SP_SC];
+#pragma unroll
+          for (uint32_t j = 0; j < SP_SC; j++) {
+            const uint32_t i = at + j * SP_NT + tid;
+            s[j] = i < n ? perm[i] : FULL;
+          }
+#pragma unroll
+          for (uint32_t j = 0; j < SP_SC; j++) {
+            y[j] = 0;
+            if (s[j] != FULL) {
+              if (type == 0) y[j] = (uint32_t)M.labels[s[j]] == wi.h;
+              else y[j] = (M.codes[(uint64_t)s[j] * M.code_bytes + (wi.h >> 3)] >> (wi.h & 7)) & 1u;
+            }
+          }
+#pragma unroll
+          for (uint32_t j = 0; j < SP_SC; j++) {
+            bool live = s[j] != FULL;
+            if (live && type == 0 && !y[j]) {
               uint32_t r[4];
-              philox(s, ee, g, ST_NEG, M.seed, r);
+              draw4(s[j], ee, g, ST_NEG, seed, r);
               live = (uint64_t)r[0] >= M.thr_neg;
             }
-          } else {
-            pos = (M.codes[(uint64_t)s * M.code_bytes + (wi.h >> 3)] >> (wi.h & 7)) & 1u;
-            live = true;
-          }
-        }
-        const uint32_t bal = __ballot_sync(0xFFFFFFFFu, live);
-        if (lane == 0) misc[1 + warp] = __popc(bal);
-        __syncthreads();
-        uint32_t off = 0, nact = 0;
-        for (uint32_t w = 0; w < (uint32_t)NW; w++) {
-          const uint32_t cnt = misc[1 + w];
-          off += w < warp ? cnt : 0;
-          nact += cnt;
-        }
-        if (live) {
-          const uint32_t slot = off + __popc(bal & ((1u << lane) - 1u));
-          list_s[slot] = s | (pos << 31);
-          uint32_t d[8];
-          philox(s, ee, g, ST_CH0, M.seed, d);
-          philox(s, ee, g, ST_CH1, M.seed, d + 4);
-#pragma unroll
-          for (int k = 0; k < 8; k++) list_d[slot * 8 + k] = d[k];
-        }
-        __syncthreads();
-        if (tid == 0) {
-          const uint32_t pre = nact < TM_RING - 1 ? nact : TM_RING - 1;
-          for (uint32_t a = 0; a < pre; a++) {
-            const uint32_t k = gs + a, sl = k % TM_RING;
-            tma_row(&bars[sl], ring + sl * Wpmax, xbase + (uint64_t)(list_s[a] & 0x7FFFFFFFu) * Wp,
-                    Wp * 4);
-          }
-          issued = gs + pre;
-          if (nact) atomicAdd((unsigned long long *)(err + 2), (unsigned long long)nact);
-        }
-        // ---- sequential per-sample steps ------------------------------------
-        for (uint32_t a = 0; a < nact; a++) {
-          const uint32_t k = gs + a, sl = k % TM_RING;
-          if (!mbar_wait(&bars[sl], (k / TM_RING) & 1u, wait_limit)) {
-            misc[44] = 1;
-            atomicOr(err, 1u);
-          }
-          uint32_t x[WPT];
-          if (mine) WVec<WPT>::ld(ring + sl * Wpmax + w0, x);
-          else
-#pragma unroll
-            for (int q = 0; q < WPT; q++) x[q] = 0xFFFFFFFFu;
-          // failed literal counts (and literal counts of dirty clauses)
-#pragma unroll
-          for (int c = 0; c < 8; c++) {
-            uint32_t f = 0, l = 0;
-#pragma unroll
-            for (int q = 0; q < WPT; q++) {
-              const uint32_t aw = act[c][q] & em[q];
-              f += __popc(aw & ~x[q]);
-              l += __popc(aw);
-            }
-            f = __reduce_add_sync(0xFFFFFFFFu, f);
-            if ((dirty >> c) & 1u) l = __reduce_add_sync(0xFFFFFFFFu, l);
-            if (lane == 0) {
-              partial[warp * 16 + c] = f;
-              partial[warp * 16 + 8 + c] = l;
-            }
+            bal[j] = __ballot_sync(FULL, live);
+            if (lane == 0) misc[8 + j * SPW + warp] = __popc(bal[j]);
           }
           __syncthreads();
-          if (misc[44]) {
-            aborted = true;
-            gs += a;
-            break;
-          }
-          if (tid == 0) {
-            for (int q = 0; q < IBS; q++) misc[48 + q] = 0;  // previous sample's overflow lists
-            if (a + TM_RING - 1 < nact) {
-              const uint32_t k2 = gs + a + TM_RING - 1, sl2 = k2 % TM_RING;
-              tma_row(&bars[sl2], ring + sl2 * Wpmax,
-                      xbase + (uint64_t)(list_s[a + TM_RING - 1] & 0x7FFFFFFFu) * Wp, Wp * 4);
-              issued = k2 + 1;
-            }
-          }
-          const uint32_t ent = list_s[a];
-          if (warp == 0) {
-            // votes (capi.c:110-118), chunk vote, clamp, p (capi.c:217-225),
-            // decisions (capi.c:226-242), lane c deciding clause c
-            uint32_t sum = 0;
-            if (lane < 16)
-              for (uint32_t w = 0; w < (uint32_t)NW; w++) sum += partial[w * 16 + lane];
-            const uint32_t Ls = __shfl_sync(0xFFFFFFFFu, sum, (lane & 7) + 8);
-            if (lane < 8 && ((dirty >> lane) & 1u)) lcache = Ls;
-            const uint32_t Lq = lane < 8 ? lcache : 0u;
-            int32_t vq = 0;
-            if (lane < 8) {
-              if (Lq == 0)
-                vq = (int32_t)M.tol;
-              else {
-                vq = (int32_t)(Lq < M.tol ? Lq : M.tol) - (int32_t)sum;
-                vq = vq < 0 ? 0 : vq;
-              }
-            }
-            int32_t v = __reduce_add_sync(0xFFFFFFFFu, (lane & 1) ? -vq : vq);
-            v = v > (int32_t)T ? (int32_t)T : v;
-            v = v < -(int32_t)T ? -(int32_t)T : v;
-            const uint32_t pa = ent >> 31;
-            const uint64_t av = (uint64_t)(pa ? (int64_t)T - v : (int64_t)T + v);
-            const uint32_t c = lane & 7;
-            const bool type1 = pa ? !(c & 1u) : (c & 1u);
-            const uint64_t drv = bounded64(list_d[a * 8 + 2 * (c >> 1) + (type1 ? 0 : 1)], T2);
-            const bool fire = lane < 8 && drv < av;
-            const uint32_t ibm = __ballot_sync(0xFFFFFFFFu, fire && type1 && vq == 0);
-            const uint32_t fbm = __ballot_sync(0xFFFFFFFFu, fire && vq > 0);
-            const uint32_t t1m = __ballot_sync(0xFFFFFFFFu, fire && type1 && vq > 0);
-            const uint32_t incm =
-                __ballot_sync(0xFFFFFFFFu, fire && type1 && vq > 0 && Lq <= M.maxlit);
-            if (lane == 0) {
-              misc[40] = ibm;
-              misc[41] = fbm;
-              misc[42] = t1m;
-              misc[43] = incm;
-            }
-          }
-          __syncthreads();
-          const uint32_t ibm = misc[40], fbm = misc[41], t1m = misc[42], incm = misc[43];
-          dirty = ibm | fbm;
-          const uint32_t sp_s = ent & 0x7FFFFFFFu;
-          // ---- Type Ib (capi.c:181-190), in rounds of IBS clauses: the picks
-          // of each clause counted per bit in two binary levels, larger counts
-          // as overflow entries worth 4 each (saturating subtraction is
-          // order-free), then applied by the owners of the words ----------------
-          for (uint32_t rest = ibm; rest;) {
-            uint32_t grp = 0;
-            for (int q = 0; q < IBS && rest; q++) {
-              grp |= rest & (0u - rest);
-              rest &= rest - 1u;
-            }
-            const uint32_t npk = C.s_picks, nq = (npk + 3) >> 2;
-            uint32_t slot = 0;
-            for (uint32_t cm = grp; cm; cm &= cm - 1, slot++) {
-              const uint32_t c = __ffs(cm) - 1;
-              uint32_t *l0 = lev + slot * 2 * Wpmax, *l1 = l0 + Wpmax;
-              for (uint32_t q = tid; q < nq; q += NT) {
-                uint32_t r[4];
-                philox(sp_s, ee, g, ST_IB | (c << 20) | q, M.seed, r);
+          const uint32_t here = misc[8 + lane];  // SP_SC * SPW = 32 counts
 #pragma unroll
-                for (uint32_t z = 0; z < 4; z++) {
-                  if (4 * q + z < npk) {
-                    const uint32_t bit = __umulhi(r[z], C.input_bits);
-                    const uint32_t w = bit >> 5, mk = 1u << (bit & 31);
-                    if (atomicXor(&l0[w], mk) & mk) {
-                      if (atomicXor(&l1[w], mk) & mk) {
-                        const uint32_t at = atomicAdd(&misc[48 + slot], 1u);
-                        if (at < ovf_cap) ovf[slot * ovf_cap + at] = bit;
-                      }
-                    }
-                  }
+          for (uint32_t j = 0; j < SP_SC; j++) {
+            const uint32_t before = __reduce_add_sync(FULL, lane < j * SPW + warp ? here : 0);
+            if ((bal[j] >> lane) & 1u)
+              list[cnt + before + __popc(bal[j] & ((1u << lane) - 1u))] = s[j] | (y[j] << 31);
+          }
+          cnt += __reduce_add_sync(FULL, here);
+          at += SP_SC * SP_NT;
+          __syncthreads();
+        }
+        nsteps += cnt;
+        // rows [from, to) of the list into their ring slots, by all threads
+        auto fetch = [&](uint32_t from, uint32_t to) {
+          const uint32_t q4 = Wp >> 2;
+          for (uint32_t a = from + (tid >> 4); a < to; a += SP_NT / 16) {
+            const uint32_t *src = xbase + (uint64_t)(list[a] & 0x7FFFFFFFu) * Wp;
+            uint32_t *dst = ring + (a % R) * SW;
+            for (uint32_t q = tid & 15; q < q4; q += 16) cp_async_words<16>(dst + 4 * q, src + 4 * q);
+          }
+          cp_commit();
+        };
+        uint32_t fetched = cnt < (uint32_t)R ? cnt : (uint32_t)R;
+        fetch(0, fetched);
+        for (uint32_t g0 = 0; g0 < cnt; g0 += SP_NT) {
+          if (g0) __syncthreads();
+          if (g0 + tid < cnt) vote_thresholds(list[g0 + tid], ee, g, M.T, seed, thr + tid * 8);
+          if (!g0) cp_wait<0>();
+          __syncthreads();
+          const uint32_t ge = cnt - g0 < SP_NT ? cnt : g0 + SP_NT;
+          for (uint32_t b = g0; b < ge;) {
+            const uint32_t be = b + win < ge ? b + win : ge;  // the round's end
+            // ---- this warp's sample of the round -------------------------------
+            const uint32_t a = b + warp;
+            uint32_t r = 0;
+            if (a < be) {
+              const bool pa = list[a] >> 31;
+              const int32_t tc = thr[(a - g0) * 8 + cl];
+              const uint32_t L = lits[cl];
+              const uint32_t *xs = ring + (a % R) * SW + 2 * lane;
+              uint32_t f[8] = {};
+#pragma unroll
+              for (int k = 0; k < NK; k++) {
+                uint2 x = *(const uint2 *)(xs + 64 * k);
+                x.x |= ~em[k][0];
+                x.y |= ~em[k][1];
+#pragma unroll
+                for (int c = 0; c < 8; c++) {
+                  const uint2 t = *(const uint2 *)(planes + (c * 8 + M7) * SW + 2 * lane + 64 * k);
+                  f[c] += __popc(t.x & ~x.x) + __popc(t.y & ~x.y);
                 }
               }
+              uint32_t pk[4];
+#pragma unroll
+              for (int c = 0; c < 4; c++)
+                pk[c] = __reduce_add_sync(FULL, f[2 * c] + (f[2 * c + 1] << 16));
+              const uint32_t pr =
+                  (lane & 4) ? ((lane & 2) ? pk[3] : pk[2]) : ((lane & 2) ? pk[1] : pk[0]);
+              const uint32_t F = (lane & 1) ? pr >> 16 : pr & 0xFFFFu;
+              // votes (capi.c:110-118), signed by clause parity (:148-161)
+              int32_t vote = (int32_t)(L == 0 || L > tol ? tol : L) - (int32_t)F;
+              vote = vote < 0 ? 0 : vote;
+              const int32_t v = (int32_t)__reduce_add_sync(FULL, (uint32_t)(vote * sign));
+              const uint32_t fm = __ballot_sync(FULL, (pa ? v : -v) < tc) & 0xFFu;
+              if (fm) {
+                const uint32_t vt = __ballot_sync(FULL, vote > 0);
+                const uint32_t inc = __ballot_sync(FULL, L <= maxlit);
+                const uint32_t t1 = pa ? 0x55u : 0xAAu;  // Type I clauses
+                // Type Ib (capi.c:181-190), Type Ia and II, Type Ia increments
+                r = (fm & t1 & ~vt) | (fm & vt) << 8 | (fm & vt & t1 & inc & 0xFFu) << 16;
+              }
             }
+            if (lane == 0) res[par * SPW + warp] = r;
+            cp_wait<AHEAD>();
             __syncthreads();
-#pragma unroll
-            for (int c = 0; c < 8; c++) {
-              if (!((grp >> c) & 1u) || !mine) continue;
-              uint32_t p[WPT][M7];
-              gather(c, p);
-              const uint32_t sl2 = __popc(grp & ((1u << c) - 1u));
-              uint32_t *l0 = lev + sl2 * 2 * Wpmax + w0, *l1 = l0 + Wpmax;
-              uint32_t m0[WPT], m1[WPT], zero[WPT];
-              WVec<WPT>::ld(l0, m0);
-              WVec<WPT>::ld(l1, m1);
-#pragma unroll
-              for (int q = 0; q < WPT; q++) zero[q] = 0;
-              WVec<WPT>::st(l0, zero);
-              WVec<WPT>::st(l1, zero);
-#pragma unroll
-              for (int q = 0; q < WPT; q++) {
-                rg_sub_pow2<M7>(p[q], act[c][q], M7, 0, m0[q], am[q]);
-                rg_sub_pow2<M7>(p[q], act[c][q], M7, 1, m1[q], am[q]);
+            // rows behind this round are done with: refill their slots
+            {
+              const uint32_t to = cnt - b < (uint32_t)R ? cnt : b + R;
+              fetch(fetched, to);
+              fetched = to;
+            }
+            // ---- feedback of the round's samples, in order -----------------------
+            const uint32_t rs = res[par * SPW + cl];
+            par ^= 1u;
+            uint32_t next = be;
+            for (uint32_t pend = __ballot_sync(FULL, rs != 0) & 0xFFu; pend; pend &= pend - 1) {
+              const uint32_t w = __ffs(pend) - 1;
+              const uint32_t rw = __shfl_sync(FULL, rs, w);
+              const uint32_t ent = list[b + w];
+              const uint32_t ibm = rw & 0xFFu, fbm = (rw >> 8) & 0xFFu, incm = rw >> 16;
+              const uint32_t t1 = (ent >> 31) ? 0x55u : 0xAAu;
+              uint32_t *oc = misc + 48 + opar * 4;
+              if (ibm) {
+                draw_picks<SP_NT, SW>(ibm, ent & 0x7FFFFFFFu, ee, g, seed, npk, nq, input_bits, lev,
+                                      ovf, oc, ovf_cap);
+                __syncthreads();
+                opar ^= 1u;
+                if (tid < 4) misc[48 + opar * 4 + tid] = 0;  // for the next pass with picks
               }
-              const uint32_t no = min(misc[48 + sl2], ovf_cap);
-              for (uint32_t t = 0; t < no; t++) {
-                const uint32_t bit = ovf[sl2 * ovf_cap + t], w = bit >> 5;
+              if ((ibm | fbm) & jbit) {
+                const bool is1 = (t1 & jbit) != 0, incx = (incm & jbit) != 0;
+                const uint32_t slot = __popc(ibm & (jbit - 1u));
+                const uint32_t *xs = ring + ((b + w) % R) * SW + 2 * lane;
+#pragma unroll 1
+                for (int k = 0; k < NK; k++) {
+                  uint32_t p[M7][2], ac[2], x[2], mv[2], ma[2];
 #pragma unroll
-                for (int q = 0; q < WPT; q++)
-                  if (w == w0 + q) rg_sub_pow2<M7>(p[q], act[c][q], M7, 2, 1u << (bit & 31), am[q]);
+                  for (int bb = 0; bb < M7; bb++) WVec<2>::ld(own + bb * SW + 64 * k, p[bb]);
+                  WVec<2>::ld(own + M7 * SW + 64 * k, ac);
+                  WVec<2>::ld(xs + 64 * k, x);
+#pragma unroll
+                  for (int q = 0; q < 2; q++) {
+                    if (NK == 1) {
+                      mv[q] = vm[0][q];
+                      ma[q] = am[0][q];
+                    } else {
+                      mv[q] = word_mask(64 * k + 2 * lane + q, W, C.vmask);
+                      ma[q] = word_mask(64 * k + 2 * lane + q, W, C.amask);
+                    }
+                  }
+                  if (ibm & jbit) {
+                    uint32_t *l0 = lev + slot * (2 * SW) + 2 * lane + 64 * k, *l1 = l0 + SW;
+                    uint32_t m0[2], m1[2];
+                    const uint32_t zero[2] = {};
+                    WVec<2>::ld(l0, m0);
+                    WVec<2>::ld(l1, m1);
+                    WVec<2>::st(l0, zero);
+                    WVec<2>::st(l1, zero);
+                    // an overflow entry is worth 4: twice a level-1 count
+                    const uint32_t no = 2 * min(oc[slot], ovf_cap);
+                    for (uint32_t t = 0;; t++) {
+                      count_sub(p, ac, m0, m1, ma);
+                      if (t >= no) break;
+                      const uint32_t bit = ovf[slot * ovf_cap + (t >> 1)];
+#pragma unroll
+                      for (int q = 0; q < 2; q++) {
+                        m0[q] = 0;
+                        m1[q] = (bit >> 5) == 64 * k + 2 * lane + q ? 1u << (bit & 31) : 0u;
+                      }
+                    }
+                  } else {
+                    // Type Ia (capi.c:177-180): inc where x = 1 (if L <=
+                    // maximum), dec where x = 0 and not included.  Type II
+                    // (capi.c:192-196): inc where x = 0 and not included.
+                    uint32_t c0[2], dm[2];
+#pragma unroll
+                    for (int q = 0; q < 2; q++) {
+                      const uint32_t nx = ~(x[q] | included(p, ac[q], q, ib)) & mv[q];
+                      c0[q] = nx | (incx ? x[q] & mv[q] : 0u);
+                      dm[q] = is1 ? nx : 0u;
+                    }
+                    count_step(p, ac, c0, dm, ma);
+                  }
+#pragma unroll
+                  for (int bb = 0; bb < M7; bb++) WVec<2>::st(own + bb * SW + 64 * k, p[bb]);
+                  WVec<2>::st(own + M7 * SW + 64 * k, ac);
+                }
               }
-              scatter(c, p);
+              if (ibm || incm || (fbm & ~t1) || ib > 1) {
+                // an action may have moved: the later results no longer hold
+                if ((ibm | fbm) & jbit) recount();
+                next = b + w + 1;
+                __syncthreads();
+                break;
+              }
             }
-            if (rest) {
-              // another round reuses the slots: every thread has read the
-              // overflow counts before they are reset
-              __syncthreads();
-              if (tid < IBS) misc[48 + tid] = 0;
-              __syncthreads();
-            }
-          }
-          // ---- Type Ia / II of this thread's words of every fed-back clause --
-#pragma unroll
-          for (int c = 0; c < 8; c++) {
-            if (!((fbm >> c) & 1u) || !mine) continue;
-            uint32_t p[WPT][M7];
-            gather(c, p);
-            const bool t1 = (t1m >> c) & 1u, incx = (incm >> c) & 1u;
-#pragma unroll
-            for (int q = 0; q < WPT; q++) {
-              // Type Ia (capi.c:177-180): inc where x=1 (if L <= maximum),
-              // dec where x=0 and not included.  Type II (capi.c:192-196):
-              // inc where x=0 and not included.
-              const uint32_t nx = ~x[q] & ~rg_included<M7>(p[q], act[c][q], M7, M.ib) & vm[q];
-              if (t1 && incx)
-                rg_add<M7>(p[q], act[c][q], M7, x[q] & vm[q], nx, am[q]);
-              else if (t1)
-                rg_dec<M7>(p[q], act[c][q], M7, nx, am[q]);
-              else
-                rg_inc<M7>(p[q], act[c][q], M7, nx, am[q]);
-            }
-            scatter(c, p);
+            // a round that ended early is followed by one that little longer
+            // (evaluations thrown away take issue slots from other units), a
+            // full one by one of twice its length
+            const uint32_t grown = next < be ? next - b + 1 : 2 * win;
+            win = grown < SPW ? grown : SPW;
+            b = next;
           }
         }
-        if (!aborted) gs += nact;
+        cp_wait<0>();
         __syncthreads();
       }
     }
-    if (aborted) break;
     // ---- the unit's automata back to global memory ----------------------------
 #pragma unroll
-    for (int c = 0; c < 8; c++) {
-      if (mine) {
-        WVec<WPT>::st(gact + c * Wp + w0, act[c]);
+    for (int k = 0; k < NK; k++) {
+      if (64 * k + 2 * lane >= Wp) continue;
 #pragma unroll
-        for (int b = 0; b < RP; b++) WVec<WPT>::st(gcnt + (c * M7 + b) * Wp + w0, pl[c][b]);
-      }
+      for (int b = 0; b < 8; b++)
+        *(uint2 *)((b < M7 ? gcnt + b * Wp : gact) + 64 * k) = *(const uint2 *)(own + b * SW + 64 * k);
     }
-    for (uint32_t i = tid; i < (uint32_t)(M7 - RP) * 8 * Wp; i += NT) {
-      const uint32_t bb = i / (8 * Wp), rem = i - bb * 8 * Wp, c = rem / Wp, w = rem - c * Wp;
-      gcnt[(c * M7 + RP + bb) * Wp + w] = splanes[i];
-    }
+    if (tid == 0 && nsteps) atomicAdd((unsigned long long *)(err + 2), (unsigned long long)nsteps);
     __syncthreads();
   }
-  if (aborted && tid == 0) {
-    // wait (bounded) for this CTA's copies still in flight before exiting
-    for (uint32_t k = gs; k < issued; k++) mbar_wait(&bars[k % TM_RING], (k / TM_RING) & 1u);
-  }
-  __syncthreads();
 }
 
 // ---- configurations ----------------------------------------------------------
-// id (1-based): threads per unit, words per thread, register planes, CTAs
-// per SM the registers are sized for, Type Ib slots
-#define TM_WPT_CONFIGS(X)   \
-  X(1, 512, 2, 2, 1, 2)     \
-  X(2, 256, 1, 0, 3, 2)     \
-  X(3, 256, 2, 2, 2, 2)     \
-  X(4, 128, 2, 1, 4, 2)     \
-  X(5, 64, 1, 0, 8, 2)      \
-  X(6, 32, 2, 0, 14, 2)     \
-  X(7, 32, 2, 1, 14, 2)
+// id (1-based).  k_train_wpt: W(threads per unit, words per thread, words
+// per row slot, register planes, CTAs per SM the registers are sized for);
+// k_train_spec: S(words per row slot, ring slots, CTAs per SM).
+#define TM_WPT_CONFIGS(W, S) \
+  W(1, 256, 4, 1024, 4, 1)   \
+  S(2, 256, 32, 1)           \
+  W(3, 128, 4, 512, 4, 2)    \
+  W(4, 128, 2, 256, 4, 4)    \
+  S(5, 64, 32, 3)            \
+  W(6, 32, 2, 64, 0, 16)     \
+  W(7, 32, 2, 56, 0, 16)     \
+  W(8, 32, 1, 32, 0, 20)     \
+  S(9, 128, 32, 2)           \
+  W(10, 64, 2, 128, 0, 8)    \
+  W(11, 256, 4, 1024, 3, 1)
 
 struct WptConfig {
-  int nt, wpt, rp, minb, ibs;
+  int ring;  // ring slots of k_train_spec, 0: k_train_wpt
+  int nt, sw, rp;
 };
 static const WptConfig kWpt[] = {
-#define TM_WPT_ROW(ID, NT, WPT, RP, MINB, IBS) {NT, WPT, RP, MINB, IBS},
-    TM_WPT_CONFIGS(TM_WPT_ROW)
-#undef TM_WPT_ROW
+#define TM_W(ID, NT, WPT, SW, RP, MINB) {0, NT, SW, RP},
+#define TM_S(ID, SW, R, MINB) {R, (int)SP_NT, SW, 0},
+    TM_WPT_CONFIGS(TM_W, TM_S)
+#undef TM_W
+#undef TM_S
 };
 constexpr int kWptCount = (int)(sizeof(kWpt) / sizeof(kWpt[0]));
 
-int wpt_configs() { return kWptCount; }
-
 static uint32_t wpt_ovf_cap(uint32_t smax) { return smax / 4 > 0 ? smax / 4 : 1; }
 
-template <int NT, int WPT, int RP, int MINB, int IBS>
-static int wpt_occ(size_t bytes) {
-  cudaFuncSetAttribute(k_train_wpt<NT, WPT, RP, MINB, IBS>,
-                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+static size_t wpt_bytes(const WptConfig &k, uint32_t smax) {
+  const uint32_t oc = wpt_ovf_cap(smax);
+  return k.ring ? spec_layout(k.sw, k.ring, oc).total
+                : wpt_layout(k.nt, k.sw, k.rp, 4, oc).total;
+}
+
+template <class F>
+static int wpt_occ(F kernel, int threads, size_t bytes) {
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   int nb = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_train_wpt<NT, WPT, RP, MINB, IBS>, NT,
-                                                bytes);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, threads, bytes);
   return nb;
 }
 
@@ -506,36 +1145,72 @@ static int wpt_occ(size_t bytes) {
 int train_wpt_occupancy(int id, uint32_t Wpmax, uint32_t smax, size_t *smem_bytes) {
   if (id < 1 || id > kWptCount) return 0;
   const WptConfig &k = kWpt[id - 1];
-  if (Wpmax > (uint32_t)(k.nt * k.wpt) || Wpmax % k.wpt) return 0;
-  uint32_t o[10];
-  wpt_layout(Wpmax, k.nt, k.rp, k.ibs, wpt_ovf_cap(smax), o);
-  *smem_bytes = o[9];
+  if (Wpmax > (uint32_t)k.sw) return 0;
+  const size_t bytes = wpt_bytes(k, smax);
+  *smem_bytes = bytes;
   switch (id) {
-#define TM_WPT_OCC(ID, NT, WPT, RP, MINB, IBS) \
-  case ID: return wpt_occ<NT, WPT, RP, MINB, IBS>(o[9]);
-    TM_WPT_CONFIGS(TM_WPT_OCC)
-#undef TM_WPT_OCC
+#define TM_W(ID, NT, WPT, SW, RP, MINB) \
+  case ID: return wpt_occ(k_train_wpt<NT, WPT, SW, RP, MINB>, NT, bytes);
+#define TM_S(ID, SW, R, MINB) \
+  case ID: return wpt_occ(k_train_spec<SW, R, MINB>, SP_NT, bytes);
+    TM_WPT_CONFIGS(TM_W, TM_S)
+#undef TM_W
+#undef TM_S
   }
   return 0;
 }
 
+// The configurations worth a launch of `units` units on `sms` SMs, rows of at
+// most Wpmax words (ids, best guess first; 0 to `max` of them).
+//   k_train_wpt with the smallest row slot that holds the rows: smaller slots
+//     hold more units per SM (search rows of 49 words: 25.7 ms in 56-word
+//     slots, 27.5 ms in 64-word ones).  For rows above 512 words three register
+//     planes when the shared memory allows it (105.1 against 110.1 ms on the
+//     large sparse classifier, 6,000 samples x 2), else four.
+//   k_train_spec up to 6 units per SM and 256 words: with few units the chain
+//     of one unit's samples is what takes the time (plain classifier, 320
+//     units: 2.8 ms against 6.6 ms), with many the evaluations it throws away
+//     (search rows, 15,000 units: 67.8 against 25.7 ms).
+int wpt_choices(uint32_t Wpmax, uint32_t smax, uint32_t units, int sms, int optin, int *ids,
+                int max) {
+  int n = 0;
+  for (int spec = 0; spec < 2; spec++) {
+    if (spec && units > 6u * (uint32_t)sms) break;
+    int best = 0;
+    for (int id = 1; id <= kWptCount; id++) {
+      const WptConfig &k = kWpt[id - 1];
+      if ((k.ring != 0) != (spec != 0) || Wpmax > (uint32_t)k.sw) continue;
+      if (wpt_bytes(k, smax) > (size_t)optin) continue;
+      if (best && kWpt[best - 1].sw < k.sw) continue;
+      if (best && kWpt[best - 1].sw == k.sw && kWpt[best - 1].rp <= k.rp) continue;
+      best = id;
+    }
+    if (best && n < max) ids[n++] = best;
+  }
+  return n;
+}
+
 cudaError_t launch_train_wpt(int id, const TrainDev *machines, const WorkItem *work,
                              uint32_t nwork, uint32_t *counter, uint32_t e_begin, uint32_t e_end,
-                             uint32_t Wpmax, uint32_t smax, uint32_t wait_limit, int grid,
-                             uint32_t *err, cudaStream_t st) {
-  if (id < 1 || id > kWptCount) return cudaErrorInvalidValue;
-  const WptConfig &k = kWpt[id - 1];
-  const uint32_t ovf_cap = wpt_ovf_cap(smax);
-  uint32_t o[10];
-  wpt_layout(Wpmax, k.nt, k.rp, k.ibs, ovf_cap, o);
+                             uint32_t Wpmax, uint32_t smax, int grid, uint32_t *err,
+                             cudaStream_t st) {
+  if (id < 1 || id > kWptCount || Wpmax > (uint32_t)kWpt[id - 1].sw) return cudaErrorInvalidValue;
+  const size_t bytes = wpt_bytes(kWpt[id - 1], smax);
+  const uint32_t oc = wpt_ovf_cap(smax);
   switch (id) {
-#define TM_WPT_LAUNCH(ID, NT, WPT, RP, MINB, IBS)                                            \
-  case ID:                                                                                   \
-    k_train_wpt<NT, WPT, RP, MINB, IBS><<<grid, NT, o[9], st>>>(                             \
-        machines, work, nwork, counter, e_begin, e_end, Wpmax, ovf_cap, wait_limit, err);    \
+#define TM_W(ID, NT, WPT, SW, RP, MINB)                                          \
+  case ID:                                                                       \
+    k_train_wpt<NT, WPT, SW, RP, MINB><<<grid, NT, bytes, st>>>(                 \
+        machines, work, nwork, counter, e_begin, e_end, oc, err);                \
     break;
-    TM_WPT_CONFIGS(TM_WPT_LAUNCH)
-#undef TM_WPT_LAUNCH
+#define TM_S(ID, SW, R, MINB)                                                    \
+  case ID:                                                                       \
+    k_train_spec<SW, R, MINB><<<grid, SP_NT, bytes, st>>>(                       \
+        machines, work, nwork, counter, e_begin, e_end, oc, err);                \
+    break;
+    TM_WPT_CONFIGS(TM_W, TM_S)
+#undef TM_W
+#undef TM_S
   }
   return cudaGetLastError();
 }
