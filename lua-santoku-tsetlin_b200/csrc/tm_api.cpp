@@ -51,15 +51,25 @@ static int fail(int code, const char *fmt, ...) {
 // of create / train / predict can be tested without exhausting a GPU.
 static std::atomic<int64_t> g_fail_alloc{-1};
 
-cudaError_t tmb_dev_malloc(void **p, size_t n) {
+bool tmb_alloc_fails() {
   int64_t c = g_fail_alloc.load();
   while (c >= 0 && !g_fail_alloc.compare_exchange_weak(c, c - 1)) {
   }
-  if (c == 0) {
+  return c == 0;
+}
+
+cudaError_t tmb_dev_malloc(void **p, size_t n) {
+  if (tmb_alloc_fails()) {
     *p = nullptr;
     return cudaErrorMemoryAllocation;
   }
-  return cudaMalloc(p, n);
+  cudaError_t e = cudaMalloc(p, n);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    tmb_scratch_trim();
+    e = cudaMalloc(p, n);
+  }
+  return e;
 }
 
 extern "C" int tm_debug_fail_alloc(int64_t after) {

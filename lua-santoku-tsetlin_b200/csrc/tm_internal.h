@@ -320,5 +320,9 @@ int tmb_fail(int code, const char *msg);
 // null when the device has no GEMM encoding or the machine is
 // individualized.  The bytes stay valid until the automata change.
 int tmb_machine_act8(tm_machine *m, tmb::MachineView *v);
-// cudaMalloc behind the failure injection of tm_debug_fail_alloc
+// whether the failure injection of tm_debug_fail_alloc fails this allocation
+bool tmb_alloc_fails();
+// gives the scratch pool's unused memory of the current device back (tm_util.cu)
+void tmb_scratch_trim();
+// cudaMalloc behind it
 cudaError_t tmb_dev_malloc(void **p, size_t n);
