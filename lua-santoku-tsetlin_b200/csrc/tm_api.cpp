@@ -156,6 +156,9 @@ struct tm_machine {
   // by the round's machines one after another, and the holdout bytes of
   // each distinct holdout row layout
   DevBuf search_act8;
+  // vote sums and CTA count of k_predict_few, zero between calls
+  DevBuf few;
+  int sms = 0;  // of the device, once asked
   std::vector<DevBuf> search_x8;
   // the autotuner's snapshot of the automata between its trials
   DevBuf tune_snap;
@@ -440,7 +443,7 @@ extern "C" void tm_destroy(tm_machine *m) {
   for (DevBuf *b : {&m->x, &m->tx, &m->raw, &m->labels, &m->codes, &m->perm, &m->perm_scratch, &m->sums,
                     &m->outc, &m->work, &m->tdev, &m->cls_job, &m->errf, &m->ckpt, &m->search,
                     &m->search_truth, &m->act8, &m->x8, &m->gemm_c, &m->gemm_ws,
-                    &m->search_act8, &m->tune_snap})
+                    &m->search_act8, &m->tune_snap, &m->few})
     b->release();
   for (DevBuf &b : m->search_x8) b.release();
   if (m->ev0) cudaEventDestroy(m->ev0);
@@ -2031,6 +2034,94 @@ static int predict_gemm(tm_machine *m, uint64_t n) {
   }
 }
 
+// A predict of at most TM_SMALL_N_MAX samples of a dense machine: one launch
+// per 16 samples from the byte rows to the outputs (k_predict_few).  Requests
+// from host memory of up to 3,840 bytes travel in the kernel's parameters,
+// larger ones through the machine's pinned buffer and a copy; the outputs come
+// back through the pinned buffer.
+static int predict_few(tm_machine *m, const uint8_t *problems, uint64_t n, int64_t *out_classes,
+                       uint8_t *out_codes, int64_t *out_scores, bool on_device) {
+  const ClassDev &c0 = m->cls[0];
+  const uint64_t sums_b = 16ull * m->classes * 4;
+  if (m->few.cap < sums_b + 16) {
+    CK(m->few.ensure(sums_b + 16));
+    CK(cudaMemsetAsync(m->few.p, 0, m->few.cap, m->st));
+  }
+  int rc = ensure_lits(m);
+  if (rc) return rc;
+  const uint64_t nch = m->n_chunks[0], inb = n * nch;
+  const uint64_t clsb = n * 8, codb = n * m->class_chunks, scb = n * m->classes * 8;
+  PredictFew f{};
+  f.act = m->d_act;
+  f.lits = m->d_lits;
+  f.C = c0;
+  f.classes = m->classes;
+  f.clauses = m->clauses;
+  f.tol = m->tol;
+  f.row_bytes = (uint32_t)nch;
+  f.sums = m->few.as<int32_t>();
+  f.done = (uint32_t *)(m->few.as<uint8_t>() + sums_b);
+  f.type = m->type;
+  f.device = m->device;
+  if (!m->sms) m->sms = num_sms(m->device);
+  f.sms = m->sms;
+  f.in = problems;
+  uint8_t *po = nullptr;  // outputs in pinned memory: classes or codes, then scores
+  const uint64_t first = out_classes ? clsb : codb, sc_at = (first + 7) & ~7ull;
+  const uint64_t outb = sc_at + (out_scores ? scb : 0);
+  if (!on_device) {
+    uint8_t *pb = nullptr;
+    if (inb <= sizeof f.inl && n <= predict_few_group(c0.Wp)) {
+      f.in = nullptr;
+      memcpy(f.inl.w, problems, inb);
+    } else {
+      pb = pin_stage(m, inb);
+      if (pb) memcpy(pb, problems, inb);
+      CK(m->raw.ensure(std::max<uint64_t>(inb, 16)));
+      CK(cudaMemcpyAsync(m->raw.p, pb ? pb : problems, inb, cudaMemcpyHostToDevice, m->st));
+      f.in = m->raw.as<uint8_t>();
+    }
+    uint8_t *o = nullptr;
+    if (outb <= TM_PIN_STAGE && (pb || pin_stage(m, 0))) {
+      po = o = m->pin + TM_PIN_STAGE;
+    } else {
+      CK(m->outc.ensure(outb + 64));
+      o = m->outc.as<uint8_t>();
+    }
+    f.out_classes = out_classes ? (int64_t *)o : nullptr;
+    f.out_codes = out_codes ? o : nullptr;
+    f.out_scores = out_scores ? (int64_t *)(o + sc_at) : nullptr;
+  } else {
+    f.out_classes = out_classes;
+    f.out_codes = out_codes;
+    f.out_scores = out_scores;
+  }
+  if (m->timing) CK(cudaEventRecord(m->ev0, m->st));
+  CK(launch_predict_few(f, (uint32_t)n, m->st));
+  const uint32_t group = predict_few_group(c0.Wp);
+  note_launch(m, (n + group - 1) / group);
+  if (m->timing) CK(cudaEventRecord(m->ev1, m->st));
+  m->stats.predict_launches++;
+  m->stats.predict_gemm = 0;
+  if (!on_device && !po) {
+    if (out_classes) CK(cudaMemcpyAsync(out_classes, f.out_classes, clsb, cudaMemcpyDeviceToHost, m->st));
+    if (out_codes) CK(cudaMemcpyAsync(out_codes, f.out_codes, codb, cudaMemcpyDeviceToHost, m->st));
+    if (out_scores) CK(cudaMemcpyAsync(out_scores, f.out_scores, scb, cudaMemcpyDeviceToHost, m->st));
+  }
+  CK(cudaStreamSynchronize(m->st));
+  if (po) {
+    if (out_classes) memcpy(out_classes, f.out_classes, clsb);
+    if (out_codes) memcpy(out_codes, f.out_codes, codb);
+    if (out_scores) memcpy(out_scores, f.out_scores, scb);
+  }
+  if (m->timing) {
+    float ms = 0;
+    CK(cudaEventElapsedTime(&ms, m->ev0, m->ev1));
+    m->stats.predict_kernel_ms += ms;
+  }
+  return TM_OK;
+}
+
 static int predict_common(tm_machine *m, const uint8_t *problems, const int64_t *dim_offsets,
                           uint64_t n, int64_t *out_classes, uint8_t *out_codes,
                           int64_t *out_scores, bool on_device) {
@@ -2040,6 +2131,8 @@ static int predict_common(tm_machine *m, const uint8_t *problems, const int64_t 
   if (n >= (1ull << 31)) return fail(TM_ERR_ARG, "predict: too many samples");
   if (n == 0) return TM_OK;
   DevGuard g(m->device);
+  if (n <= TM_SMALL_N_MAX && !m->individualized && predict_few_group(m->cls[0].Wp))
+    return predict_few(m, problems, n, out_classes, out_codes, out_scores, on_device);
   std::vector<ClassDev> cls;
   const uint64_t sb = n * m->classes * 4;
   CK(m->sums.ensure(sb));

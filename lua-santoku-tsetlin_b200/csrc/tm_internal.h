@@ -217,6 +217,32 @@ cudaError_t launch_serve_finalize(const ServeJob *jobs_dev, uint32_t njobs, cuda
 // Predicts of at most this many samples read each clause row once with one
 // warp per row (k_predict_small) instead of the 64 x 64 tiles.
 constexpr uint32_t TM_SMALL_N_MAX = 32;
+// A predict of at most TM_SMALL_N_MAX samples of a dense machine from byte
+// rows to outputs, one launch per group of samples (k_predict_few).  `in` and
+// the outputs may be device memory or pinned host memory; without `in` the
+// rows are in `inl` (one launch).  sums (16 x classes) and done are zero
+// between calls: the kernel leaves them so.
+struct FewRows {
+  uint32_t w[960];
+};
+constexpr uint32_t TM_FEW_SMEM = 72 << 10;  // staged rows of a launch: two CTAs per SM
+struct PredictFew {
+  const uint32_t *act;
+  const int32_t *lits;
+  ClassDev C;  // the layout all classes share (offsets of class 0)
+  uint32_t classes, clauses, tol, row_bytes;
+  const uint8_t *in;
+  int32_t *sums;
+  uint32_t *done;
+  int32_t type;
+  int64_t *out_classes;
+  uint8_t *out_codes;
+  int64_t *out_scores;
+  int device, sms;
+  FewRows inl;
+};
+uint32_t predict_few_group(uint32_t Wp);
+cudaError_t launch_predict_few(const PredictFew &f, uint32_t n, cudaStream_t st);
 // k_lits with an optional gate (skipped while *gate == 0)
 cudaError_t launch_lits_gated(const uint32_t *act, const ClassDev *cls, uint32_t classes,
                               uint32_t clauses, int32_t *lits, const uint32_t *gate,

@@ -12,6 +12,8 @@
 #include <cooperative_groups.h>
 #include <cub/cub.cuh>
 
+#include <atomic>
+
 #include "tm_device.cuh"
 
 namespace tmb {
@@ -1449,6 +1451,321 @@ __global__ void __launch_bounds__(256, NS <= 2 ? 3 : 2)
     small_vote<NS>(f, lits[(uint64_t)h * clauses + c], c, tol, ns, lane, part);
   }
   if (lane < ns && part != 0) atomicAdd(&sums[(uint64_t)(s0 + lane) * classes + h], part);
+}
+
+// ---------------------------------------------------------------------------
+// k_predict_few: a whole predict of at most 16 samples of a dense machine in
+// one launch -- byte rows in, classes / codes / scores out.  Every CTA stages
+// the samples' rows in shared memory from the caller's bytes (bits that do not
+// count for a row's end set, so that no mask is needed later); its warps
+// evaluate contiguous ranges of the flattened (class, clause) order, CR rows
+// at a time (a sample's words are read once for CR clauses).  A lane's action
+// words stream through a ring of its own in shared memory, DEPTH copies of 16
+// bytes ahead, across rows: HBM stays busy while the counts are formed, and no
+// register waits for a load.  Votes are added to sums, and the last CTA to
+// finish forms the outputs and leaves sums and the CTA count at zero for the
+// next call.  Small requests from host memory travel in the kernel's
+// parameters and the outputs may be pinned host memory, so that a one-sample
+// call is one launch (rows read from pinned memory by every CTA took 20 us).
+// Bound by HBM for few samples on machines beyond L2 (each action word is read
+// once), by LOP3 (64 % of the ALU pipe at 5 samples) above, by launch latency
+// on small machines.  Whole calls from host memory, before (repack, the
+// row-per-warp kernel reading rows through L1, finalize, two copies) -> now:
+// plain classifier, one sample 36.3 -> 24.0 us; large sparse classifier, five
+// samples 133 -> 81 us.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ uint32_t maj3(uint32_t a, uint32_t b, uint32_t c) {
+  uint32_t d;
+  asm("lop3.b32 %0, %1, %2, %3, 0xE8;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+  return d;
+}
+__device__ __forceinline__ uint32_t xor3(uint32_t a, uint32_t b, uint32_t c) {
+  uint32_t d;
+  asm("lop3.b32 %0, %1, %2, %3, 0x96;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+  return d;
+}
+
+constexpr int FEW_DEPTH = 8;  // copies in flight per lane
+
+// U: steps of the row loop unrolled, so that ring slots and the choice of
+// counting are fixed per step (4 for rows of more than 3 steps; rows are then
+// padded to whole groups of U steps), or 1.
+template <int NS, int CR, int U>
+__global__ void __launch_bounds__(256, NS <= 2 ? 4 : (NS <= 5 ? 3 : 2))
+    k_predict_few(const uint32_t *__restrict__ act, const int32_t *__restrict__ lits,
+                  const ClassDev C, uint32_t classes, uint32_t clauses, uint32_t tol,
+                  const uint8_t *__restrict__ in, uint32_t row_bytes, uint32_t ns,
+                  uint32_t per_warp, int32_t *__restrict__ sums, uint32_t *__restrict__ done,
+                  int32_t type, int64_t *out_classes, uint8_t *out_codes, int64_t *out_scores,
+                  const __grid_constant__ FewRows inl) {
+  extern __shared__ __align__(16) uint32_t fsm[];
+  __shared__ bool last;
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t Wp = C.Wp, W = C.W, Q = Wp >> 2, KQ = ((Q + 31) / 32 + U - 1) / U * U;
+  static_assert(U == 1 || (U * CR) % FEW_DEPTH == 0 || FEW_DEPTH % (U * CR) == 0, "ring slots");
+  // [FEW_DEPTH][thread] 16-byte ring slots, then the samples' rows
+  uint4 *ring = (uint4 *)fsm + threadIdx.x;
+  uint32_t *xs = fsm + FEW_DEPTH * 256 * 4;
+  const uint64_t total = (uint64_t)classes * clauses;
+  uint64_t q = (((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * per_warp;
+  const uint64_t qe = q < total ? (q + per_warp < total ? q + per_warp : total) : q;
+  // the copy stream: rows q .. qe - 1 in groups of CR, per group KQ steps of
+  // one copy per row
+  const uint4 *fr = (const uint4 *)(act + q * Wp) + lane;  // row of the next copy's group
+  uint32_t fk = 0, left = (uint32_t)(qe - q);
+  int slot_in = 0, slot_out = 0;
+  // one step's copies (rows of the group past the range and words past the
+  // row are not read) into slots `slot` ..
+  auto push = [&](int slot) {
+#pragma unroll
+    for (int r = 0; r < CR; r++)
+      if ((uint32_t)r < left && lane + 32 * fk < Q)
+        cp_async16(ring + (slot + r) * 256, fr + r * Q + 32 * fk, true);
+    cp_async_commit();
+    if (++fk == KQ) {
+      fk = 0;
+      fr += CR * Q;
+      left = left > CR ? left - CR : 0;
+    }
+  };
+  constexpr int STEPS = FEW_DEPTH / CR;  // steps the ring holds
+  auto wrap = [](int s) { return s >= FEW_DEPTH ? s - FEW_DEPTH : s; };
+#pragma unroll
+  for (int k = 0; k < STEPS - 1; k++) push(k * CR);
+  slot_in = (STEPS - 1) * CR;
+  {
+    const bool words = ((row_bytes | (uint32_t)(uintptr_t)in) & 3) == 0;
+    const uint8_t *small = (const uint8_t *)inl.w;  // rows in the kernel's parameters
+#pragma unroll
+    for (uint32_t s = 0; s < NS; s++) {
+      const uint8_t *row = in + (uint64_t)s * row_bytes;
+      for (uint32_t w = threadIdx.x; w < Wp; w += blockDim.x) {
+        uint32_t v = 0xFFFFFFFFu;
+        if (s < ns && w < W) {
+          if (in && words) {
+            v = ((const uint32_t *)row)[w];
+          } else {
+            v = 0;
+#pragma unroll
+            for (uint32_t b = 0; b < 4; b++)
+              if (4 * w + b < row_bytes)
+                v |= (uint32_t)(in ? row[4 * w + b] : small[s * row_bytes + 4 * w + b]) << (8 * b);
+          }
+          if (w + 1 == W) v |= ~C.emask;  // evaluation mask (capi.c:104-106)
+        }
+        xs[s * Wp + w] = v;
+      }
+    }
+    __syncthreads();
+  }
+  const uint4 *x4 = (const uint4 *)xs;
+  uint32_t h = 0, c = 0;
+  if (q < total) {
+    h = (uint32_t)(q / clauses);
+    c = (uint32_t)(q - (uint64_t)h * clauses);
+  }
+  constexpr bool CSA = NS >= 3;
+  int32_t part = 0;  // lane s < ns: sample s's votes of class h
+  while (q < qe) {
+    const uint32_t nr = (uint32_t)(qe - q < CR ? qe - q : CR);
+    uint32_t f[CR][NS], ones[CR][NS], twos[CR][NS];
+    int32_t Ls[CR];  // literal counts, loaded ahead of the rows
+#pragma unroll
+    for (int r = 0; r < CR; r++) {
+      Ls[r] = lits[q + ((uint32_t)r < nr ? r : 0)];
+#pragma unroll
+      for (int s = 0; s < NS; s++) f[r][s] = ones[r][s] = twos[r][s] = 0;
+    }
+    for (uint32_t k0 = 0; k0 < KQ; k0 += U) {
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const uint32_t k = k0 + u;
+        // the ring's slots: fixed per unrolled step, else carried along
+        const int si = U > 1 ? ((u + STEPS - 1) * CR) % FEW_DEPTH : slot_in;
+        const int so = U > 1 ? (u * CR) % FEW_DEPTH : slot_out;
+        push(si);
+        cp_async_wait<STEPS - 1>();
+        if (U == 1) {
+          slot_in = wrap(slot_in + CR);
+          slot_out = wrap(slot_out + CR);
+        }
+        const uint32_t kq = lane + 32 * k;
+        const bool in_row = kq < Q;
+        uint4 a[CR];
+#pragma unroll
+        for (int r = 0; r < CR; r++)
+          a[r] = in_row && (uint32_t)r < nr ? ring[(so + r) * 256] : make_uint4(0u, 0u, 0u, 0u);
+        const uint32_t xq = in_row ? kq : 0;  // past the row: a is zero, any x word will do
+        const bool csa = CSA && (U > 1 ? (u & 3) != 2 : (k & 3) != 2);
+#pragma unroll
+        for (int s = 0; s < NS; s++) {
+          const uint4 v = x4[s * Q + xq];
+#pragma unroll
+          for (int r = 0; r < CR; r++) {
+            const uint32_t t0 = a[r].x & ~v.x, t1 = a[r].y & ~v.y;
+            const uint32_t t2 = a[r].z & ~v.z, t3 = a[r].w & ~v.w;
+            if (csa) {
+              // (ones, twos) hold bit-sliced partial counts of weight 1 and
+              // 2; only the weight-4 carries are popcounted
+              const uint32_t o = ones[r][s], tw = twos[r][s];
+              const uint32_t h1 = maj3(o, t0, t1), o1 = xor3(o, t0, t1);
+              const uint32_t h2 = maj3(o1, t2, t3);
+              ones[r][s] = xor3(o1, t2, t3);
+              f[r][s] += 4 * __popc(maj3(tw, h1, h2));
+              twos[r][s] = xor3(tw, h1, h2);
+            } else {
+              f[r][s] += __popc(t0) + __popc(t1) + __popc(t2) + __popc(t3);
+            }
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < CR; r++) {
+      if ((uint32_t)r < nr) {
+        if (c == clauses) {  // the class ends within the group
+          if (lane < ns && part != 0) atomicAdd(&sums[lane * classes + h], part);
+          part = 0;
+          h++;
+          c = 0;
+        }
+        const int32_t L = Ls[r];
+#pragma unroll
+        for (int s = 0; s < NS; s++) {
+          if (CSA) f[r][s] += 2 * __popc(twos[r][s]) + __popc(ones[r][s]);
+          const int32_t F = (int32_t)__reduce_add_sync(0xFFFFFFFFu, f[r][s]);
+          // votes (capi.c:110-118), signed by clause parity (:148-161)
+          int32_t vote = (L == 0 || L > (int32_t)tol ? (int32_t)tol : L) - F;
+          vote = vote < 0 ? 0 : vote;
+          if (lane == (uint32_t)s) part += (c & 1) ? -vote : vote;
+        }
+        c++;
+      }
+    }
+    q += nr;
+  }
+  if (lane < ns && part != 0) atomicAdd(&sums[lane * classes + h], part);
+  cp_async_wait<0>();
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(done, 1u) + 1 == gridDim.x;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  // outputs (k_finalize's rules, capi.c:934-942, 982-990)
+  if (out_scores)
+    for (uint32_t i = threadIdx.x; i < ns * classes; i += blockDim.x)
+      out_scores[i] = __ldcg(&sums[i]);
+  if (type == 0 && out_classes) {
+    // one warp per sample: the largest sum, ties to the lowest class
+    for (uint32_t s = threadIdx.x >> 5; s < ns; s += blockDim.x >> 5) {
+      int32_t best = INT32_MIN;
+      uint32_t bc = 0xFFFFFFFFu;
+      for (uint32_t i = lane; i < classes; i += 32) {
+        const int32_t v = __ldcg(&sums[s * classes + i]);
+        if (bc == 0xFFFFFFFFu || v > best) {
+          best = v;
+          bc = i;
+        }
+      }
+#pragma unroll
+      for (int d = 16; d; d >>= 1) {
+        const int32_t ov = __shfl_xor_sync(0xFFFFFFFFu, best, d);
+        const uint32_t oc = __shfl_xor_sync(0xFFFFFFFFu, bc, d);
+        if (oc != 0xFFFFFFFFu && (bc == 0xFFFFFFFFu || ov > best || (ov == best && oc < bc))) {
+          best = ov;
+          bc = oc;
+        }
+      }
+      if (lane == 0) out_classes[s] = bc;
+    }
+  }
+  if (type == 1 && out_codes) {
+    const uint32_t nb = (classes + 7) >> 3;
+    for (uint32_t i = threadIdx.x; i < ns * nb; i += blockDim.x) {
+      const uint32_t s = i / nb, b = i - s * nb;
+      uint32_t byte = 0;
+      for (uint32_t k = 0; k < 8 && b * 8 + k < classes; k++)
+        byte |= (__ldcg(&sums[s * classes + b * 8 + k]) > 0 ? 1u : 0u) << k;
+      out_codes[i] = (uint8_t)byte;
+    }
+  }
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < ns * classes; i += blockDim.x) sums[i] = 0;
+  if (threadIdx.x == 0) *done = 0;
+}
+
+// One launch of k_predict_few: one wave of resident CTAs, each warp with an
+// equal share of the machine's clauses.
+template <int NS, int CR, int U>
+static cudaError_t few_launch_u(const PredictFew &f, uint32_t s0, uint32_t ns, cudaStream_t st) {
+  // resident CTAs per SM at the last shared-memory size, per device (the
+  // limit is raised to the most any call asks for when it is first used)
+  static std::atomic<uint64_t> seen[64];
+  std::atomic<uint64_t> &sc = seen[f.device & 63];
+  const uint64_t smem = FEW_DEPTH * 256 * 16 + (uint64_t)NS * f.C.Wp * 4;
+  const uint64_t got = sc.load(std::memory_order_relaxed);
+  int occ = (int)(got & 0xFF);
+  if (got >> 8 != smem || !occ) {
+    cudaError_t e = cudaFuncSetAttribute(k_predict_few<NS, CR, U>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)TM_FEW_SMEM + FEW_DEPTH * 256 * 16);
+    if (e == cudaSuccess)
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_predict_few<NS, CR, U>, 256, smem);
+    if (e != cudaSuccess) return e;
+    if (occ <= 0) occ = 1;
+    sc.store(smem << 8 | (uint64_t)occ, std::memory_order_relaxed);
+  }
+  const uint64_t total = (uint64_t)f.classes * f.clauses;
+  const uint64_t resident = (uint64_t)f.sms * occ * 8;
+  uint64_t per = (total + resident - 1) / resident;
+  if (per > 1) per = (per + CR - 1) / CR * CR;  // whole groups of CR rows
+  const uint64_t used = (total + per - 1) / per;
+  const uint32_t nb = (f.classes + 7) >> 3;
+  k_predict_few<NS, CR, U><<<(unsigned)((used + 7) / 8), 256, smem, st>>>(
+      f.act, f.lits, f.C, f.classes, f.clauses, f.tol,
+      f.in ? f.in + (uint64_t)s0 * f.row_bytes : nullptr, f.row_bytes, ns, (uint32_t)per, f.sums, f.done, f.type,
+      f.out_classes ? f.out_classes + s0 : nullptr,
+      f.out_codes ? f.out_codes + (uint64_t)s0 * nb : nullptr,
+      f.out_scores ? f.out_scores + (uint64_t)s0 * f.classes : nullptr, f.inl);
+  return cudaGetLastError();
+}
+
+template <int NS, int CR>
+static cudaError_t few_launch(const PredictFew &f, uint32_t s0, uint32_t ns, cudaStream_t st) {
+  constexpr int U = 8 / (CR * 2) * 2;  // a whole ring of steps for CR 2, half of one for CR 1
+  return f.C.Wp > 3 * 128 ? few_launch_u<NS, CR, U>(f, s0, ns, st)
+                          : few_launch_u<NS, CR, 1>(f, s0, ns, st);
+}
+
+// Samples per launch for rows of Wp words (0: the rows do not fit): 16, or as
+// many rows as TM_FEW_SMEM holds, rounded down to a size with a kernel.
+uint32_t predict_few_group(uint32_t Wp) {
+  const uint64_t fit = TM_FEW_SMEM / (4ull * Wp);
+  for (uint32_t ns : {16u, 12u, 8u, 7u, 6u, 5u, 4u, 3u, 2u, 1u})
+    if (fit >= ns) return ns;
+  return 0;
+}
+
+cudaError_t launch_predict_few(const PredictFew &f, uint32_t n, cudaStream_t st) {
+  const uint32_t group = predict_few_group(f.C.Wp);
+  if (!group) return cudaErrorInvalidValue;
+  for (uint32_t s0 = 0; s0 < n; s0 += group) {
+    const uint32_t ns = n - s0 < group ? n - s0 : group;
+    cudaError_t e;
+    if (ns <= 1) e = few_launch<1, 2>(f, s0, ns, st);
+    else if (ns == 2) e = few_launch<2, 2>(f, s0, ns, st);
+    else if (ns == 3) e = few_launch<3, 2>(f, s0, ns, st);
+    else if (ns == 4) e = few_launch<4, 2>(f, s0, ns, st);
+    else if (ns == 5) e = few_launch<5, 2>(f, s0, ns, st);
+    else if (ns == 6) e = few_launch<6, 2>(f, s0, ns, st);
+    else if (ns == 7) e = few_launch<7, 2>(f, s0, ns, st);
+    else if (ns == 8) e = few_launch<8, 2>(f, s0, ns, st);
+    else if (ns <= 12) e = few_launch<12, 1>(f, s0, ns, st);
+    else e = few_launch<16, 1>(f, s0, ns, st);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
 // Many small predict jobs (at most 16 samples each, any machines) in one
