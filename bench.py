@@ -478,7 +478,7 @@ def run_ours(args, w):
         ops = 2.0 * w["classes"] * w["clauses"] * (hi_s - lo_s) * 32 * words
         t_s = st["predict_kernel_ms"] / max(1, st["predict_launches"]) / 1e3 + 1e-12
         out["kernels"].update({
-            "predict_path": "int8 GEMM" if st["predict_gemm"] == 1 else "e4m3 GEMM",
+            "predict_path": "int8 GEMM" if st["predict_gemm"] == 1 else "e2m1 vote kernel",
             "predict_tensor_ops_per_s": ops / t_s,
             "predict_tensor_peak_ops_per_s": 4.5e15,
             "predict_tensor_peak_source": "nominal dense 8-bit rate of a B200 (no measured "

@@ -104,6 +104,26 @@ struct DevBuf {
   T *as() const { return (T *)p; }
 };
 
+// Grow-only buffer of the library's stream-ordered pool, used on one stream.
+struct PoolBuf {
+  void *p = nullptr;
+  size_t cap = 0;
+  cudaError_t ensure(size_t n, cudaStream_t st) {
+    if (n <= cap) return cudaSuccess;
+    release(st);
+    cudaError_t e = tmb_pool_alloc(&p, n, st);
+    if (e == cudaSuccess) cap = n;
+    return e;
+  }
+  void release(cudaStream_t st) {
+    tmb_pool_free(p, st);
+    p = nullptr;
+    cap = 0;
+  }
+  template <class T>
+  T *as() const { return (T *)p; }
+};
+
 // ---------------------------------------------------------------------------
 // machine
 // ---------------------------------------------------------------------------
@@ -151,6 +171,9 @@ struct tm_machine {
   // clause x sample products and the library's workspace
   DevBuf act8, x8, gemm_c, gemm_ws;
   bool act8_valid = false;
+  // the actions and a chunk of samples as 4-bit floats (k_votes)
+  PoolBuf act4, x4;
+  bool act4_valid = false;
   int act8_kind = 0;
   // (owner of a search round) the GEMM predict's action-byte scratch, shared
   // by the round's machines one after another, and the holdout bytes of
@@ -165,7 +188,8 @@ struct tm_machine {
   // pinned staging of small host requests (TM_PIN_STAGE bytes each way):
   // inputs go host -> pin -> device, outputs device -> pin -> host, so that
   // a one-sample predict makes no pageable (synchronously staged) copy.
-  // pin_ev marks the end of the last copy out of the input half.
+  // pin_ev marks the end of the last copy out of the input half.  The output half
+  // ends with a status word that k_votes sets.
   uint8_t *pin = nullptr;
   cudaEvent_t pin_ev = nullptr;
   bool pin_pending = false;
@@ -176,6 +200,7 @@ struct tm_machine {
 static void invalidate_derived(tm_machine *m) {
   m->lits_valid = false;
   m->act8_valid = false;
+  m->act4_valid = false;
 }
 
 // ---- large-batch predict as a GEMM ------------------------------------------
@@ -199,7 +224,21 @@ static int gemm_kind_of(int dev) {
 }
 
 
+// Whether large predicts run as k_votes (4-bit floats), the default;
+// TSETLIN_B200_GEMM=int8|fp8 asks for the library's 8-bit GEMM, off for the
+// bitwise kernels.
+static bool votes_wanted() {
+  static const bool on = [] {
+    const char *e = getenv("TSETLIN_B200_GEMM");
+    return !e || !*e || !strcmp(e, "fp4");
+  }();
+  return on;
+}
+
 constexpr uint64_t TM_PIN_STAGE = 256 << 10;
+// the output half ends with the status word of k_votes (a larger block would
+// leave the 512 KB that the driver serves from one chunk: 1.3 ms instead of 6 us)
+constexpr uint64_t TM_PIN_OUT = TM_PIN_STAGE - 64;
 
 // The input half of the machine's pinned staging buffer, ready to be
 // written, or null when the request is too large for it (or pinned memory
@@ -445,6 +484,8 @@ extern "C" void tm_destroy(tm_machine *m) {
                     &m->search_truth, &m->act8, &m->x8, &m->gemm_c, &m->gemm_ws,
                     &m->search_act8, &m->tune_snap, &m->few})
     b->release();
+  m->act4.release(m->st);
+  m->x4.release(m->st);
   for (DevBuf &b : m->search_x8) b.release();
   if (m->ev0) cudaEventDestroy(m->ev0);
   if (m->ev1) cudaEventDestroy(m->ev1);
@@ -2082,7 +2123,7 @@ static int predict_few(tm_machine *m, const uint8_t *problems, uint64_t n, int64
       f.in = m->raw.as<uint8_t>();
     }
     uint8_t *o = nullptr;
-    if (outb <= TM_PIN_STAGE && (pb || pin_stage(m, 0))) {
+    if (outb <= TM_PIN_OUT && (pb || pin_stage(m, 0))) {
       po = o = m->pin + TM_PIN_STAGE;
     } else {
       CK(m->outc.ensure(outb + 64));
@@ -2122,6 +2163,56 @@ static int predict_few(tm_machine *m, const uint8_t *problems, uint64_t n, int64
   return TM_OK;
 }
 
+// Whether a predict of n samples runs as k_votes: dense machines within its
+// exact range, past the few-sample kernel, and 2^25 clause x sample x row-word
+// tests or more: the bitwise tiles take about 10 us for those, the expansions
+// and the products' fixed cost as long.
+static bool votes_path(tm_machine *m, uint64_t n) {
+  if (m->individualized || n <= TM_SMALL_N_MAX || !votes_wanted()) return false;
+  const uint64_t M = (uint64_t)m->classes * m->clauses, W = m->cls[0].W;
+  return m->tol <= TM_VOTES_TOL && W < (1u << 19) && M < (1ull << 31) && M * n * W >= (1ull << 25);
+}
+
+// The vote sums of n byte rows through k_votes (m->sums, cleared here); 1 when
+// its status word cannot be had (nothing was queued).
+static int predict_votes(tm_machine *m, const uint8_t *rows, uint64_t n, bool on_device) {
+  const ClassDev &c0 = m->cls[0];
+  const uint64_t M = (uint64_t)m->classes * m->clauses, K = (uint64_t)c0.W * 16;
+  const uint64_t nch = m->n_chunks[0];
+  if (!pin_stage(m, 0)) return 1;
+  if (!m->sms) m->sms = num_sms(m->device);
+  uint32_t *status = (uint32_t *)(m->pin + TM_PIN_STAGE + TM_PIN_OUT);
+  *status = 0;
+  if (!on_device) {
+    CK(m->raw.ensure(n * nch));
+    uint8_t *pb = pin_stage(m, n * nch);
+    if (pb) memcpy(pb, rows, n * nch);
+    CK(cudaMemcpyAsync(m->raw.p, pb ? pb : rows, n * nch, cudaMemcpyHostToDevice, m->st));
+    rows = m->raw.as<uint8_t>();
+  }
+  if (!m->act4_valid) {
+    CK(m->act4.ensure(M * K, m->st));
+    // dense machines: the classes' clause rows follow each other
+    CK(launch_expand_fp4(m->d_act + c0.act_off, M, c0.Wp, c0.W, c0.emask, m->act4.as<uint8_t>(),
+                         m->st));
+    note_launch(m, 1);
+    m->act4_valid = true;
+  }
+  // samples per launch: at most 512 MB of operand, whole tiles of 256
+  const uint64_t nc = std::max<uint64_t>(256, ((512ull << 20) / K) / 256 * 256);
+  CK(m->x4.ensure(std::min<uint64_t>(nc, n) * K, m->st));
+  for (uint64_t s0 = 0; s0 < n; s0 += nc) {
+    const uint64_t k = std::min<uint64_t>(nc, n - s0);
+    int32_t *sums = m->sums.as<int32_t>() + s0 * m->classes;
+    CK(launch_expand_fp4_bytes(rows + s0 * nch, k, (uint32_t)nch, c0.W, m->x4.as<uint8_t>(),
+                               (uint32_t *)sums, k * m->classes, m->st));
+    CK(launch_votes(m->device, m->sms, m->act4.as<uint8_t>(), m->x4.as<uint8_t>(), m->classes,
+                    m->clauses, c0.W, m->tol, m->d_lits, (uint32_t)k, sums, nullptr, status, m->st));
+    note_launch(m, 2);
+  }
+  return TM_OK;
+}
+
 static int predict_common(tm_machine *m, const uint8_t *problems, const int64_t *dim_offsets,
                           uint64_t n, int64_t *out_classes, uint8_t *out_codes,
                           int64_t *out_scores, bool on_device) {
@@ -2136,22 +2227,29 @@ static int predict_common(tm_machine *m, const uint8_t *problems, const int64_t 
   std::vector<ClassDev> cls;
   const uint64_t sb = n * m->classes * 4;
   CK(m->sums.ensure(sb));
-  // the repack launch also clears the vote sums
-  int rc = stage_rows(m, m->x, problems, dim_offsets, n, on_device, cls, m->sums.as<uint32_t>(),
-                      sb / 4);
-  if (rc) return rc;
-  // a dense machine's rows start at offset 0 for every class: its resident
-  // class table already describes them
-  if (m->individualized) {
-    rc = upload_cls(m, m->d_cls, cls);
-    if (rc) return rc;
-  }
-  rc = ensure_lits(m);
+  int rc = ensure_lits(m);
   if (rc) return rc;
   if (m->timing) CK(cudaEventRecord(m->ev0, m->st));
-  int gr = gemm_wanted(m, n) ? predict_gemm(m, n) : 1;
+  bool votes = votes_path(m, n);
+  int gr = votes ? predict_votes(m, problems, n, on_device) : 1;
   if (gr < 0) return gr;
-  m->stats.predict_gemm = gr == 0 ? m->act8_kind : 0;
+  votes = gr == 0;
+  if (gr == 1) {
+    // the repack launch also clears the vote sums
+    rc = stage_rows(m, m->x, problems, dim_offsets, n, on_device, cls, m->sums.as<uint32_t>(),
+                    sb / 4);
+    if (rc) return rc;
+    // a dense machine's rows start at offset 0 for every class: its resident
+    // class table already describes them
+    if (m->individualized) {
+      rc = upload_cls(m, m->d_cls, cls);
+      if (rc) return rc;
+    }
+    if (m->timing) CK(cudaEventRecord(m->ev0, m->st));  // the evaluation alone
+    gr = gemm_wanted(m, n) ? predict_gemm(m, n) : 1;
+    if (gr < 0) return gr;
+  }
+  m->stats.predict_gemm = gr ? 0 : (votes ? TM_GEMM_FP8 : m->act8_kind);
   if (gr == 1) {
     CK(launch_predict(m->d_act, m->d_lits, m->d_cls, nullptr, m->classes, m->clauses, m->tol,
                       m->x.as<uint32_t>(), (uint32_t)n, m->sums.as<int32_t>(), m->st));
@@ -2180,7 +2278,7 @@ static int predict_common(tm_machine *m, const uint8_t *problems, const int64_t 
   // small results come back through the output half of the pinned buffer
   uint8_t *po = nullptr;
   const uint64_t outb = (out_classes ? clsb : 0) + (out_codes ? codb : 0) + (out_scores ? scb : 0);
-  if (!on_device && outb <= TM_PIN_STAGE && pin_stage(m, 0)) po = m->pin + TM_PIN_STAGE;
+  if (!on_device && outb <= TM_PIN_OUT && pin_stage(m, 0)) po = m->pin + TM_PIN_STAGE;
   if (!on_device) {
     uint8_t *q = po;
     auto back = [&](void *dst, const void *src, uint64_t b) -> cudaError_t {
@@ -2194,6 +2292,8 @@ static int predict_common(tm_machine *m, const uint8_t *problems, const int64_t 
     if (out_scores) CK(back(out_scores, dsc, scb));
   }
   CK(cudaStreamSynchronize(m->st));
+  if (votes && *(volatile uint32_t *)(m->pin + TM_PIN_STAGE + TM_PIN_OUT))
+    return fail(TM_ERR_DEVICE, "predict: a wait of the vote kernel ran out");
   if (po) {
     const uint8_t *q = po;
     if (out_classes) memcpy(out_classes, q, clsb), q += clsb;

@@ -156,6 +156,20 @@ cudaError_t launch_train_wpt(int id, const TrainDev *machines, const WorkItem *w
                              uint32_t nwork, uint32_t *counter, uint32_t e_begin, uint32_t e_end,
                              uint32_t Wpmax, uint32_t smax, int grid, uint32_t *err,
                              cudaStream_t st);
+// Large-batch predict in one tensor-core kernel (tm_votes.cu): bit rows as
+// 4-bit floats (16 bytes per word), and the vote sums of n samples x classes
+// added to `sums`.  Exact for clause tolerances up to TM_VOTES_TOL and rows
+// of fewer than 2^24 literals.  `err` (device or pinned) is set to 1 when a
+// bounded wait ran out.
+constexpr uint32_t TM_VOTES_TOL = 65536;
+cudaError_t launch_expand_fp4(const uint32_t *src, uint64_t rows, uint32_t stride, uint32_t W,
+                              uint32_t last_mask, uint8_t *dst, cudaStream_t st);
+cudaError_t launch_expand_fp4_bytes(const uint8_t *src, uint64_t rows, uint32_t row_bytes,
+                                    uint32_t W, uint8_t *dst, uint32_t *zero, uint64_t zero_words,
+                                    cudaStream_t st);
+cudaError_t launch_votes(int dev, int sms, const uint8_t *act4, const uint8_t *x4, uint32_t classes,
+                         uint32_t clauses, uint32_t W, uint32_t tol, const int32_t *lits, uint32_t n,
+                         int32_t *sums, const uint32_t *gate, uint32_t *err, cudaStream_t st);
 cudaError_t launch_lits(const uint32_t *act, const ClassDev *cls, uint32_t classes,
                         uint32_t clauses, int32_t *lits, cudaStream_t st);
 cudaError_t launch_predict(const uint32_t *act, const int32_t *lits, const ClassDev *cls,
@@ -350,5 +364,8 @@ int tmb_machine_act8(tm_machine *m, tmb::MachineView *v);
 bool tmb_alloc_fails();
 // gives the scratch pool's unused memory of the current device back (tm_util.cu)
 void tmb_scratch_trim();
+// stream-ordered memory of that pool, for buffers used on one stream only
+cudaError_t tmb_pool_alloc(void **p, size_t n, cudaStream_t st);
+void tmb_pool_free(void *p, cudaStream_t st);
 // cudaMalloc behind it
 cudaError_t tmb_dev_malloc(void **p, size_t n);

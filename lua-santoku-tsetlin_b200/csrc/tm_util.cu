@@ -29,10 +29,10 @@
 
 namespace {
 
-// Scratch of one call.  The metric and packing calls work on the legacy
-// stream; their scratch comes from a pool of the library's own per device,
-// in stream order, so that a call does not pay for cudaMalloc and cudaFree
-// (224 us of a 20,000-code score went to them and to idle waits).  The pool
+// Scratch memory of calls, in stream order, from a pool of the library's own
+// per device, so that a call (the metrics and the packing, on the legacy
+// stream) or a new machine's first predict does not pay for cudaMalloc and
+// cudaFree (they took most of the 224 us of a 20,000-code score).  The pool
 // keeps at most TM_SCRATCH_KEEP bytes between calls and gives them back when
 // an allocation of the library fails.
 constexpr uint64_t TM_SCRATCH_KEEP = 256ull << 20;
@@ -70,32 +70,31 @@ void tmb_scratch_trim() {
   cudaMemPoolTrimTo(g_pool[dev], 0);
 }
 
+cudaError_t tmb_pool_alloc(void **p, size_t n, cudaStream_t st) {
+  *p = nullptr;
+  if (tmb_alloc_fails()) return cudaErrorMemoryAllocation;
+  cudaMemPool_t pool = scratch_pool();
+  if (!pool) return cudaErrorNotSupported;
+  cudaError_t e = cudaMallocFromPoolAsync(p, n, pool, st);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    tmb_scratch_trim();
+    e = cudaMallocFromPoolAsync(p, n, pool, st);
+  }
+  if (e != cudaSuccess) *p = nullptr;
+  return e;
+}
+
+void tmb_pool_free(void *p, cudaStream_t st) {
+  if (p) cudaFreeAsync(p, st);
+}
+
 namespace {
 
 struct DevScratch {
   void *p = nullptr;
-  bool pooled = false;
-  cudaError_t ensure(size_t n) {
-    if (tmb_alloc_fails()) return cudaErrorMemoryAllocation;
-    cudaMemPool_t pool = scratch_pool();
-    if (pool) {
-      cudaError_t e = cudaMallocFromPoolAsync(&p, n, pool, 0);
-      if (e == cudaErrorMemoryAllocation) {
-        cudaGetLastError();
-        tmb_scratch_trim();
-        e = cudaMallocFromPoolAsync(&p, n, pool, 0);
-      }
-      if (e == cudaSuccess) pooled = true;
-      else p = nullptr;
-      return e;
-    }
-    return cudaMalloc(&p, n);
-  }
-  ~DevScratch() {
-    if (!p) return;
-    if (pooled) cudaFreeAsync(p, 0);
-    else cudaFree(p);
-  }
+  cudaError_t ensure(size_t n) { return tmb_pool_alloc(&p, n, 0); }
+  ~DevScratch() { tmb_pool_free(p, 0); }
 };
 
 }  // namespace
