@@ -175,14 +175,14 @@ struct tm_machine {
   PoolBuf act4, x4;
   bool act4_valid = false;
   int act8_kind = 0;
-  // (owner of a search round) the GEMM predict's action-byte scratch, shared
-  // by the round's machines one after another, and the holdout bytes of
+  // (owner of a search round) the vote kernel's copy of the actions, shared
+  // by the round's machines one after another, and the expanded holdout of
   // each distinct holdout row layout
-  DevBuf search_act8;
+  DevBuf search_act4;
   // vote sums and CTA count of k_predict_few, zero between calls
   DevBuf few;
   int sms = 0;  // of the device, once asked
-  std::vector<DevBuf> search_x8;
+  std::vector<DevBuf> search_x4;
   // the autotuner's snapshot of the automata between its trials
   DevBuf tune_snap;
   // pinned staging of small host requests (TM_PIN_STAGE bytes each way):
@@ -264,10 +264,6 @@ static uint8_t *pin_stage(tm_machine *m, uint64_t bytes) {
   }
   return m->pin;
 }
-
-// Kernels launched by a CUB 64-bit radix sort of pairs: upsweep histogram,
-// exclusive scan and one onesweep pass per 8-bit digit.
-static const uint64_t kSortKernels = 10;
 
 static void note_launch(tm_machine *m, uint64_t k) { m->stats.kernel_launches += k; }
 
@@ -482,11 +478,11 @@ extern "C" void tm_destroy(tm_machine *m) {
   for (DevBuf *b : {&m->x, &m->tx, &m->raw, &m->labels, &m->codes, &m->perm, &m->perm_scratch, &m->sums,
                     &m->outc, &m->work, &m->tdev, &m->cls_job, &m->errf, &m->ckpt, &m->search,
                     &m->search_truth, &m->act8, &m->x8, &m->gemm_c, &m->gemm_ws,
-                    &m->search_act8, &m->tune_snap, &m->few})
+                    &m->search_act4, &m->tune_snap, &m->few})
     b->release();
   m->act4.release(m->st);
   m->x4.release(m->st);
-  for (DevBuf &b : m->search_x8) b.release();
+  for (DevBuf &b : m->search_x4) b.release();
   if (m->ev0) cudaEventDestroy(m->ev0);
   if (m->ev1) cudaEventDestroy(m->ev1);
   if (m->pin_ev) cudaEventDestroy(m->pin_ev);
@@ -1133,6 +1129,23 @@ static int choose_plan(std::vector<TrainJob> &jobs, const std::vector<TrainDev> 
   return TM_OK;
 }
 
+// Queues epoch orders on the owner's stream, with scratch for the large ones:
+// as many at a time as fit 256 MB.
+static int queue_orders(tm_machine *m0, std::vector<OrderJob> &orders, const uint32_t *epoch_dev,
+                        uint64_t *launches) {
+  size_t one = 0, all = 0;
+  for (const OrderJob &J : orders) {
+    const size_t b = order_scratch_bytes(J.n);
+    one = std::max(one, b);
+    all += b;
+  }
+  const size_t want = std::max(one, std::min<size_t>(all, 256u << 20));
+  if (want) CK(m0->perm_scratch.ensure(want));
+  CK(launch_orders(orders.data(), orders.size(), m0->perm_scratch.p, m0->perm_scratch.cap, m0->st,
+                   epoch_dev, launches));
+  return TM_OK;
+}
+
 // Runs local epochs [e0, e1) of every job in one launch (units of all jobs
 // share the grid).  Permutations are built per job for those epochs.
 static int run_epochs(std::vector<TrainJob> &jobs, uint32_t e0, uint32_t e1, tm_machine *owner) {
@@ -1154,19 +1167,14 @@ static int run_epochs(std::vector<TrainJob> &jobs, uint32_t e0, uint32_t e1, tm_
     }
   }
   CK(m0->perm.ensure(std::max<uint64_t>(pwords, 4) * 4));
-  uint32_t maxn = 0;
-  for (auto &j : jobs) maxn = std::max<uint32_t>(maxn, (uint32_t)j.a->samples);
-  const size_t psb = perm_scratch_bytes(std::max<uint32_t>(maxn, 1));
-  CK(m0->perm_scratch.ensure(psb));
-  for (auto &kv : pidx) {
-    const uint64_t seed = kv.first.first, n = kv.first.second;
-    for (uint32_t e = e0; e < e1; e++) {
-      // the draw-contract epoch index is local epoch e (epoch_base 0)
-      CK(launch_perm(seed, e, (uint32_t)n, m0->perm.as<uint32_t>() + kv.second + (e - e0) * n,
-                     m0->perm_scratch.p, m0->perm_scratch.cap, st));
-      note_launch(m0, 1 + kSortKernels);
-    }
-  }
+  std::vector<OrderJob> orders;
+  for (auto &kv : pidx)
+    for (uint32_t e = e0; e < e1; e++)  // the draw-contract epoch index is local epoch e
+      orders.push_back(OrderJob{kv.first.first,
+                                m0->perm.as<uint32_t>() + kv.second + (uint64_t)(e - e0) * kv.first.second,
+                                nullptr, nullptr, (uint32_t)kv.first.second, e});
+  int orc = queue_orders(m0, orders, nullptr, &m0->stats.kernel_launches);
+  if (orc) return orc;
   std::vector<TrainDev> td;
   std::vector<WorkItem> work;
   TrainShape sh{};
@@ -1421,6 +1429,8 @@ static int train_batch_impl(tm_machine *const *ms, const tm_train_args *args, ui
 // with one host synchronisation.  Every kernel reads the machine's `live`
 // flag, so stopped machines drop out of the replays without a new graph.
 // ---------------------------------------------------------------------------
+static bool votes_path(tm_machine *m, uint64_t n);
+
 static int search_round(tm_machine *const *ms, const tm_train_args *args, uint32_t count,
                         const tm_search_args *sa) {
   tm_machine *m0 = ms[0];
@@ -1489,88 +1499,55 @@ static int search_round(tm_machine *const *ms, const tm_train_args *args, uint32
     CK(cudaMemsetAsync(m->sums.p, 0, nt * m->classes * 4, st));
     if (sa->patience) CK(m->ckpt.ensure(std::max<uint64_t>(m->act_words, 4) * 4));
   }
-  // ---- the holdout predict of large dense machines as the 8-bit GEMM ---------
-  // Their holdout rows are expanded to bytes once; in every epoch the graph
-  // expands the trained actions and runs the products and the vote epilogue
-  // (gated by the machine's live flag, like the bitwise predict).  Each
-  // product width is tried once here, outside the capture: a machine whose
-  // shape the library cannot take keeps the bitwise predict.
-  const int gkind = gemm_kind_of(m0->device);
-  const size_t gws = 32u << 20;
-  std::vector<char> use_gemm(count, 0);
-  std::vector<uint64_t> gchunk(count, 0);
-  std::vector<uint8_t *> gx8(count, nullptr);
+  // ---- the holdout predict of large dense machines as k_votes ---------------
+  // Their holdout rows are expanded to 4-bit floats once; in every epoch the
+  // graph expands the trained actions and runs the vote kernel (gated by the
+  // machine's live flag, like the bitwise predict).
+  std::vector<char> use_votes(count, 0);
+  std::vector<const uint8_t *> vx4(count, nullptr);
+  if (!m0->sms) m0->sms = num_sms(m0->device);
   {
-    uint64_t cmax = 0;
-    for (uint32_t i = 0; i < count; i++) {
-      tm_machine *m = ms[i];
-      const ClassDev &c0 = m->cls[0];
-      const uint64_t M = (uint64_t)m->classes * m->clauses;
-      if (gkind <= 0 || m->individualized || nt <= TM_SMALL_N_MAX ||
-          M * nt * c0.W < (1ull << 28))
-        continue;
-      uint64_t nc = ((512ull << 20) / (4 * M)) / 64 * 64;
-      nc = std::max<uint64_t>(nc, 64);
-      gchunk[i] = nc;
-      cmax = std::max<uint64_t>(cmax, gemm_bucket(std::min<uint64_t>(nc, nt), nc) * M * 4);
-      use_gemm[i] = 1;
-    }
     uint64_t amax = 0;
-    for (uint32_t i = 0; i < count; i++)
-      if (use_gemm[i])
-        amax = std::max<uint64_t>(amax, (uint64_t)ms[i]->classes * ms[i]->clauses *
-                                            ms[i]->cls[0].W * 32);
-    if (cmax) {
-      CK(m0->gemm_c.ensure(cmax));
-      CK(m0->gemm_ws.ensure(gws));
-      CK(m0->search_act8.ensure(amax));
-    }
-    // one byte copy of the holdout per distinct row layout (the machines'
-    // staged rows of one source, feature count and row width are the same)
-    std::map<std::tuple<const void *, uint64_t, uint32_t, uint32_t>, size_t> x8_of;
+    // one copy of the holdout per distinct row layout (the machines' staged
+    // rows of one source, feature count and row width are the same)
+    std::map<std::tuple<const void *, uint64_t, uint32_t, uint32_t>, size_t> x4_of;
     for (uint32_t i = 0; i < count; i++) {
-      if (!use_gemm[i]) continue;
       tm_machine *m = ms[i];
       const ClassDev &c0 = m->cls[0];
-      const uint64_t K = (uint64_t)c0.W * 32;
+      const uint64_t M = (uint64_t)m->classes * m->clauses, K = (uint64_t)c0.W * 16;
+      // beside the launch of all small machines' tiles, a machine's own two
+      // launches pay from more work on than in a predict of its own
+      if (!votes_path(m, nt) || M * nt * c0.W < (1ull << 27) || nt * K > (2ull << 30)) continue;
+      use_votes[i] = 1;
+      amax = std::max<uint64_t>(amax, M * K);
       const void *src = sa->test_each && sa->test_each[i] ? (const void *)sa->test_each[i]
                                                           : (const void *)sa->test_problems;
       const auto key = std::make_tuple(src, (uint64_t)m->features, c0.Wp, c0.W);
-      if (x8_of.count(key)) continue;
-      const size_t at = x8_of.size();
-      x8_of[key] = at;
-      if (m0->search_x8.size() <= at) m0->search_x8.resize(at + 1);
-      // rows past nt: the last product's bucket reads them (its columns
-      // there are not used); sized for the largest chunk of any machine
-      uint64_t pad = 0;
-      for (uint32_t j = 0; j < count; j++)
-        if (use_gemm[j])
-          pad = std::max<uint64_t>(pad, gemm_bucket(std::min<uint64_t>(gchunk[j], nt), gchunk[j]));
-      CK(m0->search_x8[at].ensure((nt + pad) * K));
-      CK(launch_expand_bits(m->x.as<uint32_t>(), nt, c0.Wp, c0.W, 0xFFFFFFFFu, gkind,
-                            m0->search_x8[at].as<uint8_t>(), st));
-    }
-    for (uint32_t i = 0; i < count; i++) {
-      if (!use_gemm[i]) continue;
-      tm_machine *m = ms[i];
-      const ClassDev &c0 = m->cls[0];
-      const void *src = sa->test_each && sa->test_each[i] ? (const void *)sa->test_each[i]
-                                                          : (const void *)sa->test_problems;
-      gx8[i] = m0->search_x8[x8_of[std::make_tuple(src, (uint64_t)m->features, c0.Wp, c0.W)]]
-                   .as<uint8_t>();
-      const uint64_t M = (uint64_t)m->classes * m->clauses, K = (uint64_t)c0.W * 32;
-      const uint64_t nc = gchunk[i];
-      for (uint64_t s0 = 0; s0 < nt && use_gemm[i]; s0 += nc) {
-        const uint64_t k = std::min<uint64_t>(nc, nt - s0);
-        const int g = gemm_clause_products(m0->device, gkind, m0->search_act8.as<uint8_t>(),
-                                           gx8[i] + s0 * K, m0->gemm_c.p, M, gemm_bucket(k, nc),
-                                           K, m0->gemm_ws.p, gws, st);
-        if (g < 0) use_gemm[i] = 0;
-        else if (g > 0) return fail(TM_ERR_CUDA, "search: cuBLASLt matmul failed (status %d)", g);
+      auto it = x4_of.find(key);
+      if (it == x4_of.end()) {
+        const size_t at = x4_of.size();
+        it = x4_of.emplace(key, at).first;
+        if (m0->search_x4.size() <= at) m0->search_x4.resize(at + 1);
+        CK(m0->search_x4[at].ensure(nt * K));
+        CK(launch_expand_fp4(m->x.as<uint32_t>(), nt, c0.Wp, c0.W, 0xFFFFFFFFu,
+                             m0->search_x4[at].as<uint8_t>(), st));
       }
+      vx4[i] = m0->search_x4[it->second].as<uint8_t>();
     }
-    CK(cudaStreamSynchronize(st));
+    if (amax) CK(m0->search_act4.ensure(amax));
   }
+  // machine i's vote sums of the holdout, added to its (cleared) sums unless
+  // *gate is 0
+  auto holdout_votes = [&](uint32_t i, const uint32_t *gate, uint32_t *err) -> cudaError_t {
+    tm_machine *m = ms[i];
+    const ClassDev &c0 = m->cls[0];
+    cudaError_t e = launch_expand_fp4(m->d_act + c0.act_off, (uint64_t)m->classes * m->clauses,
+                                      c0.Wp, c0.W, c0.emask, m0->search_act4.as<uint8_t>(), st);
+    if (e != cudaSuccess) return e;
+    return launch_votes(m0->device, m0->sms, m0->search_act4.as<uint8_t>(), vx4[i], m->classes,
+                        m->clauses, c0.W, m->tol, m->d_lits, (uint32_t)nt, m->sums.as<int32_t>(),
+                        gate, err, st);
+  };
   // ---- device tables ---------------------------------------------------------
   auto al = [](size_t v) { return (v + 255) & ~(size_t)255; };
   const size_t o_scores = al(count * sizeof(SearchState));
@@ -1593,7 +1570,7 @@ static int search_round(tm_machine *const *ms, const tm_train_args *args, uint32
   std::vector<LitsJob> lj(count), ljf(count);
   std::vector<ScoreJob> sj(count);
   std::vector<CopyJob> cj(count), rj(count);
-  uint32_t tiles = 0, tiles_f = 0;  // per-epoch predict (GEMM machines apart), final pass
+  uint32_t tiles = 0, tiles_f = 0;  // bitwise tiles: per-epoch predict, final pass
   for (uint32_t i = 0; i < count; i++) {
     tm_machine *m = ms[i];
     SearchState &S = hs[i];
@@ -1618,10 +1595,10 @@ static int search_round(tm_machine *const *ms, const tm_train_args *args, uint32
     P.classes = m->classes;
     const uint32_t jt = predict_job_tiles((uint32_t)nt, m->classes, m->clauses, &P.stiles, &P.tpc);
     P.tile0 = tiles;
-    if (!use_gemm[i]) tiles += jt;  // a GEMM machine's job has no tiles: never picked
+    if (!use_votes[i]) tiles += jt;  // a job without tiles is never picked
     pjf[i] = P;
     pjf[i].tile0 = tiles_f;
-    tiles_f += jt;
+    if (!use_votes[i]) tiles_f += jt;
     pjf[i].gate = &d_state[i].has_ckpt;
     lj[i] = LitsJob{m->d_act, m->d_cls, m->d_lits, &d_state[i].live, m->classes, m->clauses};
     ljf[i] = lj[i];
@@ -1648,7 +1625,6 @@ static int search_round(tm_machine *const *ms, const tm_train_args *args, uint32
   std::map<std::pair<uint64_t, uint64_t>, uint64_t> pidx;
   uint64_t pwords = 0;
   std::vector<uint64_t> joff(count);
-  uint32_t maxn = 1;
   for (uint32_t i = 0; i < count; i++) {
     auto key = std::make_pair(jobs[i].seed, (uint64_t)args[i].samples);
     auto it = pidx.find(key);
@@ -1659,10 +1635,8 @@ static int search_round(tm_machine *const *ms, const tm_train_args *args, uint32
     } else {
       joff[i] = it->second;
     }
-    maxn = std::max<uint32_t>(maxn, (uint32_t)args[i].samples);
   }
   CK(m0->perm.ensure(std::max<uint64_t>(pwords, 4) * 4));
-  CK(m0->perm_scratch.ensure(perm_scratch_bytes(maxn)));
   std::vector<TrainDev> td;
   std::vector<WorkItem> work;
   TrainShape sh{};
@@ -1670,10 +1644,12 @@ static int search_round(tm_machine *const *ms, const tm_train_args *args, uint32
   for (uint32_t i = 0; i < count; i++) td[i].gate = &d_state[i].live;
   // epoch 0's orders: the tuner's trial launches read them (the graph
   // rebuilds them for every epoch from the device epoch counter)
+  std::vector<OrderJob> orders;
   for (auto &kv : pidx)
-    CK(launch_perm(kv.first.first, 0, (uint32_t)kv.first.second,
-                   m0->perm.as<uint32_t>() + kv.second, m0->perm_scratch.p, m0->perm_scratch.cap,
-                   st, d_epoch));
+    orders.push_back(OrderJob{kv.first.first, m0->perm.as<uint32_t>() + kv.second, nullptr, nullptr,
+                              (uint32_t)kv.first.second, 0});
+  rc = queue_orders(m0, orders, d_epoch, nullptr);
+  if (rc) return rc;
   // Units of rows of at most 32 words train in a launch of their own, next
   // to the others' (two kernels of one graph at once): a launch's shared
   // memory slices are sized by its widest row, so narrow units in the same
@@ -1811,13 +1787,8 @@ static int search_round(tm_machine *const *ms, const tm_train_args *args, uint32
   uint64_t launches = 0;
   cudaError_t ce = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
   if (ce == cudaSuccess) {
-    for (auto &kv : pidx) {
-      if (ce != cudaSuccess) break;
-      ce = launch_perm(kv.first.first, 0, (uint32_t)kv.first.second,
-                       m0->perm.as<uint32_t>() + kv.second, m0->perm_scratch.p,
-                       m0->perm_scratch.cap, st, d_epoch);
-      launches += 1 + kSortKernels;
-    }
+    ce = launch_orders(orders.data(), orders.size(), m0->perm_scratch.p, m0->perm_scratch.cap, st,
+                       d_epoch, &launches);
     if (ce == cudaSuccess) ce = cudaMemsetAsync(counter, 0, 8, st);  // both work counters
     // external event records: real events inside the graph, so that the
     // train kernels' time can be read after each replay
@@ -1844,28 +1815,9 @@ static int search_round(tm_machine *const *ms, const tm_train_args *args, uint32
     if (ce == cudaSuccess && tiles)
       ce = launch_predict_multi((const PredictJob *)(base + o_pj), count, tiles, st);
     for (uint32_t i = 0; i < count && ce == cudaSuccess; i++) {
-      if (!use_gemm[i]) continue;
-      tm_machine *m = ms[i];
-      const ClassDev &c0 = m->cls[0];
-      const uint64_t M = (uint64_t)m->classes * m->clauses, K = (uint64_t)c0.W * 32;
-      const uint64_t nc = gchunk[i];
-      ce = launch_expand_bits(m->d_act + c0.act_off, M, c0.Wp, c0.W, c0.emask, gkind,
-                              m0->search_act8.as<uint8_t>(), st);
-      launches++;
-      for (uint64_t s0 = 0; s0 < nt && ce == cudaSuccess; s0 += nc) {
-        const uint64_t k = std::min<uint64_t>(nc, nt - s0);
-        const int g = gemm_clause_products(m0->device, gkind, m0->search_act8.as<uint8_t>(),
-                                           gx8[i] + s0 * K, m0->gemm_c.p, M,
-                                           gemm_bucket(k, nc), K, m0->gemm_ws.p, gws, st);
-        if (g != 0) {
-          ce = cudaErrorUnknown;
-          break;
-        }
-        ce = launch_gemm_votes(m0->gemm_c.p, gkind, m->d_lits, m->classes, m->clauses, m->tol,
-                               (uint32_t)k, m->sums.as<int32_t>() + s0 * m->classes, st,
-                               &d_state[i].live);
-        launches++;  // the epilogue (the GEMM is the library's)
-      }
+      if (!use_votes[i]) continue;
+      ce = holdout_votes(i, &d_state[i].live, d_err);
+      launches += 2;
     }
     if (ce == cudaSuccess)
       ce = launch_search_score((const ScoreJob *)(base + o_sj), d_state, d_scores, Es, count,
@@ -1950,6 +1902,11 @@ static int search_round(tm_machine *const *ms, const tm_train_args *args, uint32
     CK(launch_copy_multi((const CopyJob *)(base + o_rj), count, st));
     CK(launch_lits_multi((const LitsJob *)(base + o_ljf), count, maxC, st));
     CK(launch_predict_multi((const PredictJob *)(base + o_pjf), count, tiles_f, st));
+    for (uint32_t i = 0; i < count; i++)
+      if (use_votes[i]) {
+        CK(holdout_votes(i, &d_state[i].has_ckpt, d_err));
+        m0->stats.kernel_launches += 2;
+      }
     CK(launch_search_score((const ScoreJob *)(base + o_sj), d_state, d_scores, Es, count, maxC, 1,
                            st));
     m0->stats.kernel_launches += 4;
@@ -1960,6 +1917,7 @@ static int search_round(tm_machine *const *ms, const tm_train_args *args, uint32
   CK(cudaMemcpyAsync(hs.data(), d_state, count * sizeof(SearchState), cudaMemcpyDeviceToHost, st));
   CK(cudaMemcpyAsync(scores.data(), d_scores, scores.size() * 8, cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
+  if (hc[0]) return fail(TM_ERR_DEVICE, "search: a device wait ran out (status %u)", hc[0]);
   m0->stats.train_active_pairs += (uint64_t)hc[2] | ((uint64_t)hc[3] << 32);
   for (uint32_t i = 0; i < count; i++) {
     if (sa->final_scores) sa->final_scores[i] = hs[i].last;

@@ -99,10 +99,18 @@ cudaError_t launch_repack(const uint8_t *src, uint64_t n, uint64_t row_bytes, ui
 cudaError_t launch_labels(const int64_t *src, int32_t *dst, uint64_t n, cudaStream_t st);
 cudaError_t launch_setup(uint32_t *act, uint32_t *cnt, const ClassDev *cls, uint32_t classes,
                          uint32_t clauses, uint32_t B, uint64_t act_words, cudaStream_t st);
-cudaError_t launch_perm(uint64_t seed, uint32_t epoch, uint32_t n, uint32_t *out,
-                        void *scratch, size_t scratch_bytes, cudaStream_t st,
-                        const uint32_t *epoch_dev = nullptr);
-size_t perm_scratch_bytes(uint32_t n);
+// One epoch order: out[0 .. n) = samples by Philox key of (seed, epoch).
+struct OrderJob {
+  uint64_t seed;
+  uint32_t *out;
+  uint64_t *key;  // scratch of large orders (set by launch_orders)
+  uint32_t *cnt;
+  uint32_t n, epoch;
+};
+constexpr uint32_t TM_ORDER_BATCH = 64;  // orders per launch
+size_t order_scratch_bytes(uint32_t n);
+cudaError_t launch_orders(OrderJob *jobs, size_t count, void *scratch, size_t scratch_bytes,
+                          cudaStream_t st, const uint32_t *epoch_dev, uint64_t *launches);
 // k_train variants: automata in shared memory (one CTA per unit), in global
 // memory (one CTA per unit), or split over a 2-CTA cluster in shared memory.
 constexpr int TM_MODE_SMEM = 0;
