@@ -2339,41 +2339,69 @@ extern "C" int tm_predict_scores(tm_machine *m, const uint8_t *problems, const i
 // ---------------------------------------------------------------------------
 // state in the reference byte layout
 // ---------------------------------------------------------------------------
-static int copy_rows(tm_machine *m, bool to_host, uint8_t *host, bool counts) {
+// Classes [lo, hi) of the actions (counts = false) or count planes, in the
+// reference byte layout, to or from `buf` (host, or device memory of the
+// machine's device when on_device).  Class h's rows start where the classes
+// before it end, so the range is one contiguous byte slice of the full
+// layout.  Dense rows without padding are copied as they are; others are
+// packed or unpacked on the device, host buffers in blocks of classes of at
+// most TM_STATE_BLOCK bytes (or one class).
+constexpr uint64_t TM_STATE_BLOCK = 128ull << 20;
+
+static int copy_classes(tm_machine *m, uint32_t lo, uint32_t hi, bool to_buf, uint8_t *buf,
+                        bool counts, bool on_device) {
+  if (hi <= lo) return TM_OK;
   const uint32_t planes = counts ? m->B - 1 : 1;
-  uint64_t ho = 0;
-  for (uint32_t h = 0; h < m->classes; h++) {
-    const ClassDev &c = m->cls[h];
-    const uint64_t rows = (uint64_t)m->clauses * planes;
-    uint32_t *dev = (counts ? m->d_cnt + c.cnt_off : m->d_act + c.act_off);
-    const size_t width = m->n_chunks[h];
-    if (to_host)
-      CK(cudaMemcpy2DAsync(host + ho, width, dev, (size_t)c.Wp * 4, width, rows,
-                           cudaMemcpyDeviceToHost, m->st));
-    else
-      CK(cudaMemcpy2DAsync(dev, (size_t)c.Wp * 4, host + ho, width, width, rows,
-                           cudaMemcpyHostToDevice, m->st));
-    ho += rows * width;
+  uint32_t *words = counts ? m->d_cnt : m->d_act;
+  const uint64_t rows = (uint64_t)m->clauses * planes;
+  if (!m->individualized && m->n_chunks[0] == (uint64_t)m->cls[0].Wp * 4) {
+    const ClassDev &c = m->cls[lo];
+    uint32_t *dev = words + (counts ? c.cnt_off : c.act_off);
+    const uint64_t bytes = (uint64_t)(hi - lo) * rows * m->n_chunks[0];
+    const cudaMemcpyKind kind = on_device ? cudaMemcpyDeviceToDevice
+                                          : (to_buf ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice);
+    if (to_buf) CK(cudaMemcpyAsync(buf, dev, bytes, kind, m->st));
+    else CK(cudaMemcpyAsync(dev, buf, bytes, kind, m->st));
+    return TM_OK;
+  }
+  std::vector<uint64_t> offs(hi - lo);
+  uint64_t at = 0;
+  for (uint32_t h = lo; h < hi;) {
+    // a block of classes
+    uint64_t bytes = 0;
+    uint32_t h1 = h;
+    while (h1 < hi) {
+      const uint64_t b = rows * m->n_chunks[h1];
+      if (h1 > h && !on_device && bytes + b > TM_STATE_BLOCK) break;
+      offs[h1 - h] = bytes;
+      bytes += b;
+      h1++;
+    }
+    const uint64_t ob = ((uint64_t)(h1 - h) * 8 + 255) & ~255ull;
+    PoolBuf tmp;
+    CK(tmp.ensure(ob + (on_device ? 0 : bytes), m->st));
+    uint8_t *dbytes = on_device ? buf + at : tmp.as<uint8_t>() + ob;
+    // (offs is pageable: the copy has read it when the call returns)
+    cudaError_t e = cudaMemcpyAsync(tmp.p, offs.data(), (uint64_t)(h1 - h) * 8,
+                                    cudaMemcpyHostToDevice, m->st);
+    if (e == cudaSuccess && !on_device && !to_buf)
+      e = cudaMemcpyAsync(dbytes, buf + at, bytes, cudaMemcpyHostToDevice, m->st);
+    if (e == cudaSuccess)
+      e = launch_state_bytes(to_buf, words, m->d_cls, h, h1, m->clauses, planes, counts,
+                             tmp.as<uint64_t>(), dbytes, m->st);
+    if (e == cudaSuccess && !on_device && to_buf)
+      e = cudaMemcpyAsync(buf + at, dbytes, bytes, cudaMemcpyDeviceToHost, m->st);
+    tmp.release(m->st);
+    if (e != cudaSuccess) return fail(TM_ERR_CUDA, "state copy: %s", cudaGetErrorString(e));
+    note_launch(m, 1);
+    at += bytes;
+    h = h1;
   }
   return TM_OK;
 }
 
-// For dense machines the per-class loop above covers classes * clauses rows
-// in one copy: the class blocks are contiguous with the same stride.
 static int copy_all(tm_machine *m, bool to_host, uint8_t *host, bool counts) {
-  if (m->individualized) return copy_rows(m, to_host, host, counts);
-  const uint32_t planes = counts ? m->B - 1 : 1;
-  const ClassDev &c = m->cls[0];
-  const uint64_t rows = (uint64_t)m->classes * m->clauses * planes;
-  uint32_t *dev = counts ? m->d_cnt : m->d_act;
-  const size_t width = m->input_chunks;
-  if (to_host)
-    CK(cudaMemcpy2DAsync(host, width, dev, (size_t)c.Wp * 4, width, rows, cudaMemcpyDeviceToHost,
-                         m->st));
-  else
-    CK(cudaMemcpy2DAsync(dev, (size_t)c.Wp * 4, host, width, width, rows, cudaMemcpyHostToDevice,
-                         m->st));
-  return TM_OK;
+  return copy_classes(m, 0, m->classes, to_host, host, counts, false);
 }
 
 extern "C" int tm_export_state(tm_machine *m, uint8_t *actions, uint8_t *state) {
@@ -2406,34 +2434,6 @@ extern "C" int tm_import_state(tm_machine *m, const uint8_t *actions, const uint
     if (rc) return rc;
   }
   CK(cudaStreamSynchronize(m->st));
-  return TM_OK;
-}
-
-// Classes [lo, hi) of the actions (counts = false) or count planes, in the
-// reference byte layout, to or from `buf` (host, or device memory of the
-// machine's device when on_device).  Class h's rows start where the classes
-// before it end, so the range is one contiguous byte slice of the full
-// layout; for a dense machine it is also one strided device block.
-static int copy_classes(tm_machine *m, uint32_t lo, uint32_t hi, bool to_buf, uint8_t *buf,
-                        bool counts, bool on_device) {
-  const uint32_t planes = counts ? m->B - 1 : 1;
-  const cudaMemcpyKind kind = on_device ? cudaMemcpyDeviceToDevice
-                                        : (to_buf ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice);
-  uint64_t bo = 0;
-  for (uint32_t h = lo; h < hi;) {
-    // dense machines: every class from h on in one copy
-    const uint32_t h1 = m->individualized ? h + 1 : hi;
-    const ClassDev &c = m->cls[h];
-    const uint64_t rows = (uint64_t)(h1 - h) * m->clauses * planes;
-    uint32_t *dev = counts ? m->d_cnt + c.cnt_off : m->d_act + c.act_off;
-    const size_t width = m->n_chunks[h];
-    if (to_buf)
-      CK(cudaMemcpy2DAsync(buf + bo, width, dev, (size_t)c.Wp * 4, width, rows, kind, m->st));
-    else
-      CK(cudaMemcpy2DAsync(dev, (size_t)c.Wp * 4, buf + bo, width, width, rows, kind, m->st));
-    bo += rows * width;
-    h = h1;
-  }
   return TM_OK;
 }
 

@@ -96,6 +96,12 @@ constexpr uint32_t ST_PERM = 0xFFFFFFFFu;
 cudaError_t launch_repack(const uint8_t *src, uint64_t n, uint64_t row_bytes, uint64_t src_stride,
                           uint32_t *dst, uint32_t dst_words, cudaStream_t st,
                           uint32_t *zero = nullptr, uint64_t zero_words = 0);
+// Classes [lo, hi) between the device layout (`words`: actions, or count planes
+// with counts) and the reference's byte layout; offs (device): each class's
+// first byte in `bytes`.
+cudaError_t launch_state_bytes(bool pack, uint32_t *words, const ClassDev *cls, uint32_t lo,
+                               uint32_t hi, uint32_t clauses, uint32_t planes, bool counts,
+                               const uint64_t *offs, uint8_t *bytes, cudaStream_t st);
 cudaError_t launch_labels(const int64_t *src, int32_t *dst, uint64_t n, cudaStream_t st);
 cudaError_t launch_setup(uint32_t *act, uint32_t *cnt, const ClassDev *cls, uint32_t classes,
                          uint32_t clauses, uint32_t B, uint64_t act_words, cudaStream_t st);

@@ -52,6 +52,79 @@ cudaError_t launch_repack(const uint8_t *src, uint64_t n, uint64_t row_bytes, ui
   return cudaGetLastError();
 }
 
+// ---------------------------------------------------------------------------
+// State in the reference's byte layout: class h's rows (clauses x planes rows
+// of ceil(input_bits / 8) bytes) one after another, classes one after another.
+// One warp per row, grid.y = class; offs[y] is the block's first byte.  A
+// strided copy to the host of rows of 60 to 170 bytes moved 0.25 GB/s (7.5 ms
+// for an individualized machine's 1.9 MB); packed on the device first, one
+// contiguous copy moves them.  Bound by memory.
+// ---------------------------------------------------------------------------
+__global__ void k_pack_state(const uint32_t *__restrict__ words, const ClassDev *__restrict__ cls,
+                             uint32_t lo, uint32_t clauses, uint32_t planes, int counts,
+                             const uint64_t *__restrict__ offs, uint8_t *__restrict__ out) {
+  const ClassDev C = cls[lo + blockIdx.y];
+  const uint32_t nb = (C.input_bits + 7) >> 3, lane = threadIdx.x & 31;
+  const uint32_t *src = words + (counts ? C.cnt_off : C.act_off);
+  const uint64_t rows = (uint64_t)clauses * planes;
+  for (uint64_t r = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < rows;
+       r += ((uint64_t)gridDim.x * blockDim.x) >> 5) {
+    const uint32_t *row = src + r * C.Wp;
+    uint8_t *dst = out + offs[blockIdx.y] + r * nb;
+    uint32_t head = (uint32_t)(-(intptr_t)dst & 3);  // bytes before the first aligned word
+    if (head > nb) head = nb;
+    const uint32_t n4 = (nb - head) >> 2, tail = head + 4 * n4;
+    for (uint32_t w = lane; w < n4; w += 32) {
+      const uint32_t b = head + 4 * w, at = b >> 2;
+      // bytes b .. b + 3 lie within the row, so a second word exists if needed
+      const uint32_t hi = (b & 3) ? row[at + 1] : 0u;
+      *(uint32_t *)(dst + b) = __funnelshift_r(row[at], hi, 8 * (b & 3));
+    }
+    if (lane < head) dst[lane] = (uint8_t)(row[0] >> (8 * lane));
+    if (lane < nb - tail) {
+      const uint32_t b = tail + lane;
+      dst[b] = (uint8_t)(row[b >> 2] >> (8 * (b & 3)));
+    }
+  }
+}
+
+__global__ void k_unpack_state(uint32_t *__restrict__ words, const ClassDev *__restrict__ cls,
+                               uint32_t lo, uint32_t clauses, uint32_t planes, int counts,
+                               const uint64_t *__restrict__ offs, const uint8_t *__restrict__ in) {
+  const ClassDev C = cls[lo + blockIdx.y];
+  const uint32_t nb = (C.input_bits + 7) >> 3, lane = threadIdx.x & 31;
+  uint32_t *dst = words + (counts ? C.cnt_off : C.act_off);
+  const uint64_t rows = (uint64_t)clauses * planes;
+  for (uint64_t r = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < rows;
+       r += ((uint64_t)gridDim.x * blockDim.x) >> 5) {
+    const uint8_t *row = in + offs[blockIdx.y] + r * nb;
+    for (uint32_t w = lane; w < C.W; w += 32) {
+      uint32_t v = 0;
+#pragma unroll
+      for (uint32_t b = 0; b < 4; b++)
+        if (4 * w + b < nb) v |= (uint32_t)row[4 * w + b] << (8 * b);
+      dst[r * C.Wp + w] = v;
+    }
+  }
+}
+
+cudaError_t launch_state_bytes(bool pack, uint32_t *words, const ClassDev *cls, uint32_t lo,
+                               uint32_t hi, uint32_t clauses, uint32_t planes, bool counts,
+                               const uint64_t *offs, uint8_t *bytes, cudaStream_t st) {
+  if (hi <= lo) return cudaSuccess;
+  const uint64_t warps = (uint64_t)clauses * planes;
+  const uint32_t bx = (uint32_t)std::min<uint64_t>((warps + 7) / 8, 148ull * 8);
+  for (uint32_t h = lo; h < hi; h += 65535) {
+    const dim3 grid(bx, std::min<uint32_t>(hi - h, 65535));
+    if (pack)
+      k_pack_state<<<grid, 256, 0, st>>>(words, cls, h, clauses, planes, counts, offs + (h - lo), bytes);
+    else
+      k_unpack_state<<<grid, 256, 0, st>>>(words, cls, h, clauses, planes, counts, offs + (h - lo),
+                                           bytes);
+  }
+  return cudaGetLastError();
+}
+
 __global__ void k_labels(const int64_t *__restrict__ src, int32_t *__restrict__ dst, uint64_t n) {
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (uint64_t)gridDim.x * blockDim.x)
