@@ -11,10 +11,9 @@
 //     LOP3 per plane finds the bits that would overflow, then one LOP3 per
 //     plane applies the update to the others (count_step and its kin);
 //   - one body of update code serves all eight clauses, the planes addressed
-//     in shared memory: eight unrolled bodies (automata in registers) were 77 KB
-//     of code and half the warps waited for instructions (search rows: 127 ms
-//     against 69 ms); only rows above 64 words keep their lowest planes in
-//     registers, for room;
+//     in shared memory, or for rows above 64 words in global memory (L2): eight
+//     unrolled bodies (automata in registers) were 77 KB of code and half the
+//     warps waited for instructions (search rows: 127 ms against 69 ms);
 //   - a sample's row words go straight to the thread that owns them by 4- to
 //     16-byte asynchronous copies, three samples ahead: no mbarrier stands
 //     between a copy and its use;
@@ -28,9 +27,9 @@
 //     sample (a second one when the sample has Type Ib clauses), every warp
 //     taking the same decisions from it.
 // Measured (train calls, B200, before -> after): search rows of 49 words, 28.5M
-// active steps, 44.7 -> 25.7 ms (narrow rows 34.7 -> 17.4 ms); plain classifier
+// active steps, 44.7 -> 26 ms (narrow rows 34.7 -> 17.4 ms); plain classifier
 // 8,000 samples x 10 epochs, 320 units, 15.0 -> 2.8 ms; encoder rows of 256
-// words 190 -> 156 ms; sparse classifier rows of 1,024 words 127 -> 105 ms.
+// words 190 -> 113 ms; sparse classifier rows of 1,024 words 127 -> 90 ms.
 // The same rules and draws as k_train, so the same automata bit for bit.
 #include "tm_device.cuh"
 
@@ -249,16 +248,21 @@ __device__ __forceinline__ void draw_picks(uint32_t ibm, uint32_t sp, uint32_t e
     uint32_t *l0 = lev + slot * (2 * SW), *l1 = l0 + SW;
     uint32_t r[4], mk[4], old[4];
     draw4(sp, ee, g, ST_IB | (c << 20) | q, seed, r);
-    const uint32_t nv = npk - 4 * q;  // picks left: fewer than 4 in the last draw
 #pragma unroll
     for (uint32_t z = 0; z < 4; z++) {
       r[z] = __umulhi(r[z], input_bits);
-      mk[z] = z < nv ? 1u << (r[z] & 31) : 0u;
-      old[z] = atomicXor(&l0[r[z] >> 5], mk[z]);
+      mk[z] = 1u << (r[z] & 31);
     }
+    if (4 * q + 4 > npk) {  // the last draw may hold fewer than 4 picks
+#pragma unroll
+      for (uint32_t z = 1; z < 4; z++) mk[z] = 4 * q + z < npk ? mk[z] : 0u;
+    }
+#pragma unroll
+    for (uint32_t z = 0; z < 4; z++) old[z] = atomicXor(&l0[r[z] >> 5], mk[z]);
 #pragma unroll
     for (uint32_t z = 0; z < 4; z++) mk[z] &= old[z];
     if (mk[0] | mk[1] | mk[2] | mk[3]) {
+      // (all four again, without a branch per pick: most warps carry somewhere)
 #pragma unroll
       for (uint32_t z = 0; z < 4; z++) old[z] = atomicXor(&l1[r[z] >> 5], mk[z]);
 #pragma unroll
@@ -274,6 +278,9 @@ __device__ __forceinline__ void draw_picks(uint32_t ibm, uint32_t sp, uint32_t e
     }
   }
 }
+
+// samples whose vote thresholds are held at a time
+__host__ __device__ constexpr uint32_t wpt_group(uint32_t NT) { return NT < 64 ? NT : 64; }
 
 // Samples listed before a unit starts on them: enough that the threshold
 // pass (one sample per thread) and the row copies' start-up weigh little.
@@ -298,10 +305,10 @@ __host__ __device__ constexpr WptLayout wpt_layout(uint32_t NT, uint32_t SW, int
   L.planes = take((8 - RP) * 8 * SW * 4);
   L.ring = take(RING * SW * 4);
   L.list = take((wpt_fill(NT) + SC * NT) * 4);
-  L.thr = take(NT * 8 * 4);
-  L.acc = take(3 * 16 * 4);
+  L.thr = take(wpt_group(NT) * 8 * 4);
+  L.acc = take(NT == 32 ? 0 : 3 * 16 * 4);  // the one-warp form adds nothing up
   L.lev = take(IBS * 2 * SW * 4);
-  L.misc = take(64 * 4);
+  L.misc = take((NT == 32 ? 8 : 64) * 4);
   L.ovf = take(IBS * ovf_cap * 2);
   L.total = at;
   return L;
@@ -311,20 +318,24 @@ __host__ __device__ constexpr WptLayout wpt_layout(uint32_t NT, uint32_t SW, int
 
 // misc: [0] unit, [8..39] live counts of a scan, [48..55] overflow counts (2 parities x 4)
 // NT threads per unit (32: the one-warp form) of WPT words, SW words per
-// row slot (at most NT * WPT, at least the widest row), RP count planes in
-// registers, MINB CTAs per SM the registers are sized for.
-template <int NT, int WPT, int SW, int RP, int MINB>
+// row slot (at most NT * WPT, at least the widest row).  The first RP count
+// planes are held in registers, the last GP in global memory, the others and
+// the actions in shared memory; IBS Type Ib clauses are drawn at a time; MINB
+// CTAs per SM the registers are sized for.
+template <int NT, int WPT, int SW, int RP, int GP, int IBS, int MINB>
 __global__ void __launch_bounds__(NT, MINB)
     k_train_wpt(const TrainDev *__restrict__ machines, const WorkItem *__restrict__ work,
                 uint32_t nwork, uint32_t *__restrict__ counter, uint32_t e_begin, uint32_t e_end,
                 uint32_t ovf_cap, uint32_t *__restrict__ err) {
   constexpr bool ONE = NT == 32;
   constexpr uint32_t NW = NT / 32;
-  constexpr int IBS = 4;       // a sample has at most one Type I clause per pair
-  constexpr int SP = 8 - RP;   // planes in shared memory: count planes RP..6, then the actions
+  constexpr uint32_t TG = wpt_group(NT);
+  // planes in shared memory: count planes RP .. 6 - GP, then the actions
+  constexpr int SP = 8 - RP - GP;
+  constexpr int G0 = M7 - GP;  // first count plane that stays in global memory
   constexpr uint32_t FULL = 0xFFFFFFFFu;
   extern __shared__ __align__(128) uint8_t smem[];
-  const WptLayout o = wpt_layout(NT, SW, RP, IBS, ovf_cap);
+  const WptLayout o = wpt_layout(NT, SW, RP + GP, IBS, ovf_cap);
   const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t w0 = tid * WPT;  // this thread's first word
   // threads past the row slots own no words: they load word 0's (under masks
@@ -338,12 +349,13 @@ __global__ void __launch_bounds__(NT, MINB)
   uint32_t *lev = (uint32_t *)(smem + o.lev);
   uint16_t *ovf = (uint16_t *)(smem + o.ovf);
   uint32_t *misc = (uint32_t *)(smem + o.misc);
+  uint32_t *ocnt = misc + (ONE ? 0 : 48);  // overflow counts (2 parities x 4)
   auto sync = [] {
     if constexpr (ONE) __syncwarp();
     else __syncthreads();
   };
   for (uint32_t i = tid; i < IBS * 2 * SW; i += NT) lev[i] = 0;
-  if (tid < 8) misc[48 + tid] = 0;
+  if (tid < 8) ocnt[tid] = 0;
   // lane c of every warp decides clause c (lanes above 8 repeat them)
   const uint32_t cl = lane & 7;
   const int32_t sign = lane < 8 ? ((lane & 1) ? -1 : 1) : 0;
@@ -378,6 +390,10 @@ __global__ void __launch_bounds__(NT, MINB)
     const uint32_t g = wi.h * M.clause_chunks + wi.k;
     uint32_t *gact = M.act + C.act_off + (uint64_t)wi.k * 8 * Wp + w0;
     uint32_t *gcnt = M.cnt + C.cnt_off + (uint64_t)wi.k * 8 * M7 * Wp + w0;
+    // the count planes that stay in global memory are read and written in
+    // place; threads without words of their own read word 0's and store nothing
+    uint32_t *gpl = M.cnt + C.cnt_off + (uint64_t)wi.k * 8 * M7 * Wp + (w0 < Wp ? w0 : 0);
+    __builtin_assume(__isGlobal(gpl));
     // ---- the unit's automata onto the SM ------------------------------------
     uint32_t pl[8][RP > 0 ? RP : 1][WPT];
     const bool mine = w0 < Wp;  // Wp is a multiple of 4, so of WPT
@@ -385,13 +401,14 @@ __global__ void __launch_bounds__(NT, MINB)
     for (int c = 0; c < 8; c++)
 #pragma unroll
       for (int b = 0; b < 8; b++) {
+        if (b >= G0 && b < M7) continue;
         uint32_t t[WPT] = {};
         if (mine) WVec<WPT>::ld(b < M7 ? gcnt + (c * M7 + b) * Wp : gact + c * Wp, t);
         if (b < RP) {
 #pragma unroll
           for (int q = 0; q < WPT; q++) pl[c][b < RP ? b : 0][q] = t[q];
         } else if (w0 < SW) {
-          WVec<WPT>::st(splanes + (c * SP + b - RP) * SW, t);
+          WVec<WPT>::st(splanes + (c * SP + (b < M7 ? b - RP : SP - 1)) * SW, t);
         }
       }
     uint32_t vm[WPT], em[WPT], am[WPT];
@@ -409,10 +426,15 @@ __global__ void __launch_bounds__(NT, MINB)
 #define TM_CLAUSES(X) X(0) X(1) X(2) X(3) X(4) X(5) X(6) X(7)
     auto gather = [&](uint32_t c, uint32_t (&p)[M7][WPT], uint32_t (&a)[WPT]) {
       const uint32_t *base = splanes + c * (SP * SW);
+      const uint32_t *gbase = gpl + c * (M7 * Wp);
 #pragma unroll
       for (int b = RP; b < 8; b++) {
         uint32_t t[WPT];
-        WVec<WPT>::ld(base + (b - RP) * SW, t);
+        if (b >= G0 && b < M7) {
+          WVec<WPT>::ld(gbase + b * Wp, t);
+        } else {
+          WVec<WPT>::ld(base + (b < M7 ? b - RP : SP - 1) * SW, t);
+        }
 #pragma unroll
         for (int q = 0; q < WPT; q++) {
           if (b < M7) p[b < M7 ? b : 0][q] = t[q];
@@ -432,13 +454,15 @@ __global__ void __launch_bounds__(NT, MINB)
     };
     auto scatter = [&](uint32_t c, const uint32_t (&p)[M7][WPT], const uint32_t (&a)[WPT]) {
       uint32_t *base = splanes + c * (SP * SW);
+      uint32_t *gbase = gpl + c * (M7 * Wp);
       if (mine) {
 #pragma unroll
         for (int b = RP; b < 8; b++) {
           uint32_t t[WPT];
 #pragma unroll
           for (int q = 0; q < WPT; q++) t[q] = b < M7 ? p[b < M7 ? b : 0][q] : a[q];
-          WVec<WPT>::st(base + (b - RP) * SW, t);
+          if (b >= G0 && b < M7) WVec<WPT>::st(gbase + b * Wp, t);
+          else WVec<WPT>::st(base + (b < M7 ? b - RP : SP - 1) * SW, t);
         }
       }
       if constexpr (RP > 0) {
@@ -561,12 +585,12 @@ __global__ void __launch_bounds__(NT, MINB)
 #pragma unroll
           for (uint32_t a = 0; a < RING - 1; a++) fetch(a);
         }
-        for (uint32_t g0 = 0; g0 < cnt; g0 += NT) {
+        for (uint32_t g0 = 0; g0 < cnt; g0 += TG) {
           // ---- vote thresholds of a group of samples --------------------------
           if (g0) sync();
-          if (g0 + tid < cnt) vote_thresholds(list[g0 + tid], ee, g, M.T, seed, thr + tid * 8);
+          if (tid < TG && g0 + tid < cnt) vote_thresholds(list[g0 + tid], ee, g, M.T, seed, thr + tid * 8);
           sync();
-          const uint32_t ge = cnt - g0 < NT ? cnt - g0 : NT;
+          const uint32_t ge = cnt - g0 < TG ? cnt - g0 : TG;
           // ---- sequential per-sample steps ------------------------------------
           for (uint32_t a = 0; a < ge; a++) {
             fetch(g0 + a + RING - 1);
@@ -608,7 +632,7 @@ __global__ void __launch_bounds__(NT, MINB)
               const uint32_t nx2 = ab == 0 ? 2 : ab - 1;
               if (tid < 16) acc[nx2 * 16 + tid] = 0;
               // the previous step's overflow counts, for the next step
-              if (tid < IBS) misc[48 + (par ^ 1u) * IBS + tid] = 0;
+              if (tid < 4) ocnt[(par ^ 1u) * 4 + tid] = 0;
               ab = ab == 2 ? 0 : ab + 1;
             }
             const uint32_t F = (lane & 1) ? pr >> 16 : pr & 0xFFFFu;
@@ -625,83 +649,101 @@ __global__ void __launch_bounds__(NT, MINB)
             dirty = 0;
             if (!(ibm | fbm)) continue;
             const uint32_t sp = ent & 0x7FFFFFFFu;
-            uint32_t *oc = misc + 48 + par * IBS;
-            if (ibm) {
-              if (ONE) __syncwarp();
-              draw_picks<NT, SW>(ibm, sp, ee, g, seed, npk, nq, input_bits, lev, ovf, oc, ovf_cap);
-              sync();
-            }
+            uint32_t *oc = ocnt + par * 4;
+            // feedback, Type Ib clauses in rounds of at most IBS, the first with
+            // the Type Ia and II clauses
+            uint32_t rest = ibm, grp, todo = fbm;
+            do {
+              grp = 0;
+#pragma unroll
+              for (int k = 0; k < IBS; k++) {
+                grp |= rest & (0u - rest);
+                rest &= rest - 1u;
+              }
+              if constexpr (IBS == 4) rest = 0;  // a sample has at most one Type I clause per pair
+              todo |= grp;
+              if (grp) {
+                if (ONE) __syncwarp();
+                draw_picks<NT, SW>(grp, sp, ee, g, seed, npk, nq, input_bits, lev, ovf, oc, ovf_cap);
+                sync();
+              }
 #pragma unroll 1
-            for (uint32_t cm = ibm | fbm; cm; cm &= cm - 1) {
-              const uint32_t c = __ffs(cm) - 1;
-              uint32_t p[M7][WPT], ac[WPT];
-              gather(c, p, ac);
-              const bool is1 = (t1 >> c) & 1u;
-              bool changed = true;  // false: the action plane is as it was
-              if ((ibm >> c) & 1u) {
-                const uint32_t slot = __popc(ibm & ((1u << c) - 1u));
-                uint32_t *l0 = lev + slot * (2 * SW) + ws, *l1 = l0 + SW;
-                uint32_t m0[WPT], m1[WPT];
-                WVec<WPT>::ld(l0, m0);
-                WVec<WPT>::ld(l1, m1);
-                if (mine) {
-                  const uint32_t zero[WPT] = {};
-                  WVec<WPT>::st(l0, zero);
-                  WVec<WPT>::st(l1, zero);
+              for (uint32_t cm = todo; cm; cm &= cm - 1) {
+                const uint32_t c = __ffs(cm) - 1;
+                uint32_t p[M7][WPT], ac[WPT];
+                gather(c, p, ac);
+                const bool is1 = (t1 >> c) & 1u;
+                bool changed = true;  // false: the action plane is as it was
+                if ((grp >> c) & 1u) {
+                  const uint32_t slot = __popc(grp & ((1u << c) - 1u));
+                  uint32_t *l0 = lev + slot * (2 * SW) + ws, *l1 = l0 + SW;
+                  uint32_t m0[WPT], m1[WPT];
+                  WVec<WPT>::ld(l0, m0);
+                  WVec<WPT>::ld(l1, m1);
+                  if (mine) {
+                    const uint32_t zero[WPT] = {};
+                    WVec<WPT>::st(l0, zero);
+                    WVec<WPT>::st(l1, zero);
+                  } else {
+#pragma unroll
+                    for (int q = 0; q < WPT; q++) m0[q] = m1[q] = 0;
+                  }
+                  // an overflow entry is worth 4: twice a level-1 count
+                  const uint32_t no = 2 * min(oc[slot], ovf_cap);
+                  for (uint32_t t = 0;; t++) {
+                    count_sub(p, ac, m0, m1, am);
+                    if (t >= no) break;
+                    const uint32_t bit = ovf[slot * ovf_cap + (t >> 1)];
+#pragma unroll
+                    for (int q = 0; q < WPT; q++) {
+                      m0[q] = 0;
+                      m1[q] = (bit >> 5) == w0 + q ? 1u << (bit & 31) : 0u;
+                    }
+                  }
                 } else {
+                  // Type Ia (capi.c:177-180): inc where x = 1 (if L <= maximum),
+                  // dec where x = 0 and not included.  Type II (capi.c:192-196):
+                  // inc where x = 0 and not included.
+                  const bool incx = is1 && ((incM >> c) & 1u);
+                  uint32_t nx[WPT];
+                  if (ib == 1 && !incx) {
 #pragma unroll
-                  for (int q = 0; q < WPT; q++) m0[q] = m1[q] = 0;
-                }
-                // an overflow entry is worth 4: twice a level-1 count
-                const uint32_t no = 2 * min(oc[slot], ovf_cap);
-                for (uint32_t t = 0;; t++) {
-                  count_sub(p, ac, m0, m1, am);
-                  if (t >= no) break;
-                  const uint32_t bit = ovf[slot * ovf_cap + (t >> 1)];
+                    for (int q = 0; q < WPT; q++) nx[q] = ~(x[q] | ac[q]) & vm[q];
+                    if (is1) count_dec0(p, nx, am);
+                    else count_inc0(p, ac, nx, am);
+                    changed = !is1;
+                  } else {
+                    uint32_t c0[WPT], dm[WPT];
 #pragma unroll
-                  for (int q = 0; q < WPT; q++) {
-                    m0[q] = 0;
-                    m1[q] = (bit >> 5) == w0 + q ? 1u << (bit & 31) : 0u;
+                    for (int q = 0; q < WPT; q++) {
+                      nx[q] = ~(x[q] | included(p, ac[q], q, ib)) & vm[q];
+                      c0[q] = nx[q] | (incx ? x[q] & vm[q] : 0u);
+                      dm[q] = is1 ? nx[q] : 0u;
+                    }
+                    count_step(p, ac, c0, dm, am);
                   }
                 }
-              } else {
-                // Type Ia (capi.c:177-180): inc where x = 1 (if L <= maximum),
-                // dec where x = 0 and not included.  Type II (capi.c:192-196):
-                // inc where x = 0 and not included.
-                const bool incx = is1 && ((incM >> c) & 1u);
-                uint32_t nx[WPT];
-                if (ib == 1 && !incx) {
-#pragma unroll
-                  for (int q = 0; q < WPT; q++) nx[q] = ~(x[q] | ac[q]) & vm[q];
-                  if (is1) count_dec0(p, nx, am);
-                  else count_inc0(p, ac, nx, am);
-                  changed = !is1;
-                } else {
-                  uint32_t c0[WPT], dm[WPT];
-#pragma unroll
-                  for (int q = 0; q < WPT; q++) {
-                    nx[q] = ~(x[q] | included(p, ac[q], q, ib)) & vm[q];
-                    c0[q] = nx[q] | (incx ? x[q] & vm[q] : 0u);
-                    dm[q] = is1 ? nx[q] : 0u;
-                  }
-                  count_step(p, ac, c0, dm, am);
+                scatter(c, p, ac);
+                if (changed) {
+                  dirty |= 1u << c;
+                  const uint32_t l = lits_of(ac);
+                  if (ONE) L = cl == c ? l : L;
+                  else lval = lane == 4u + c ? l : lval;
                 }
               }
-              scatter(c, p, ac);
-              if (changed) {
-                dirty |= 1u << c;
-                const uint32_t l = lits_of(ac);
-                if (ONE) L = cl == c ? l : L;
-                else lval = lane == 4u + c ? l : lval;
-              }
-            }
-            if (ONE) {
-              if (ibm) {
+              if (ONE && grp) {
                 __syncwarp();
                 if (lane < IBS) oc[lane] = 0;
               }
-              if (dirty) settle();
-            }
+              if (rest) {
+                // the slots are used again: every thread has read its levels, and
+                // counts overflows apart
+                sync();
+                todo = 0;
+                if (!ONE) oc += IBS;
+              }
+            } while (rest);
+            if (ONE && dirty) settle();
           }
         }
         step += cnt;
@@ -718,12 +760,13 @@ __global__ void __launch_bounds__(NT, MINB)
       for (int c = 0; c < 8; c++)
 #pragma unroll
         for (int b = 0; b < 8; b++) {
+          if (b >= G0 && b < M7) continue;
           uint32_t t[WPT];
           if (b < RP) {
 #pragma unroll
             for (int q = 0; q < WPT; q++) t[q] = pl[c][b < RP ? b : 0][q];
           } else {
-            WVec<WPT>::ld(splanes + (c * SP + b - RP) * SW, t);
+            WVec<WPT>::ld(splanes + (c * SP + (b < M7 ? b - RP : SP - 1)) * SW, t);
           }
           WVec<WPT>::st(b < M7 ? gcnt + (c * M7 + b) * Wo : gact + c * Wo, t);
         }
@@ -1096,28 +1139,39 @@ __global__ void __launch_bounds__(SP_NT, MINB)
 
 // ---- configurations ----------------------------------------------------------
 // id (1-based).  k_train_wpt: W(threads per unit, words per thread, words
-// per row slot, register planes, CTAs per SM the registers are sized for);
-// k_train_spec: S(words per row slot, ring slots, CTAs per SM).
-#define TM_WPT_CONFIGS(W, S) \
-  W(1, 256, 4, 1024, 4, 1)   \
-  S(2, 256, 32, 1)           \
-  W(3, 128, 4, 512, 4, 2)    \
-  W(4, 128, 2, 256, 4, 4)    \
-  S(5, 64, 32, 3)            \
-  W(6, 32, 2, 64, 0, 16)     \
-  W(7, 32, 2, 56, 0, 16)     \
-  W(8, 32, 1, 32, 0, 20)     \
-  S(9, 128, 32, 2)           \
-  W(10, 64, 2, 128, 0, 8)    \
-  W(11, 256, 4, 1024, 3, 1)
+// per row slot, count planes in registers, count planes in global memory,
+// Type Ib slots, CTAs per SM the registers are sized for); k_train_spec:
+// S(words per row slot, ring slots, CTAs per SM).
+// Rows of up to 64 words keep every plane in shared memory (search rows: 26.2
+// ms; with three planes in L2 and 16 units per SM 30.7).  Wider rows leave
+// their count planes in L2, where the resident units' planes fit: the units
+// that shared memory then holds hide more latency than the planes cost
+// (256-word rows: 10 units of two warps 112 ms, 4 units of four warps with
+// four planes in registers 156 ms; 128 words 37 / 51 ms; 512 words 53 / 71 ms;
+// 1,024 words, two units with one plane in registers 90 ms, one unit with
+// three 105 ms).
+#define TM_WPT_CONFIGS(W, S)      \
+  W(1, 256, 4, 1024, 1, 6, 4, 2)  \
+  S(2, 256, 32, 1)                \
+  W(3, 128, 4, 512, 0, 7, 2, 5)   \
+  W(4, 64, 4, 256, 0, 7, 2, 10)   \
+  S(5, 64, 32, 3)                 \
+  W(6, 32, 2, 64, 0, 0, 4, 16)    \
+  W(7, 32, 2, 56, 0, 0, 4, 16)    \
+  W(8, 32, 1, 32, 0, 0, 4, 20)    \
+  S(9, 128, 32, 2)                \
+  W(10, 32, 4, 128, 0, 7, 2, 20)  \
+  W(11, 32, 2, 48, 0, 0, 4, 16)   \
+  W(12, 32, 1, 24, 0, 0, 4, 20)
 
 struct WptConfig {
   int ring;  // ring slots of k_train_spec, 0: k_train_wpt
-  int nt, sw, rp;
+  int nt, sw, off;  // off: count planes not in shared memory
+  int ibs;
 };
 static const WptConfig kWpt[] = {
-#define TM_W(ID, NT, WPT, SW, RP, MINB) {0, NT, SW, RP},
-#define TM_S(ID, SW, R, MINB) {R, (int)SP_NT, SW, 0},
+#define TM_W(ID, NT, WPT, SW, RP, GP, IBS, MINB) {0, NT, SW, RP + GP, IBS},
+#define TM_S(ID, SW, R, MINB) {R, (int)SP_NT, SW, 0, 4},
     TM_WPT_CONFIGS(TM_W, TM_S)
 #undef TM_W
 #undef TM_S
@@ -1129,7 +1183,7 @@ static uint32_t wpt_ovf_cap(uint32_t smax) { return smax / 4 > 0 ? smax / 4 : 1;
 static size_t wpt_bytes(const WptConfig &k, uint32_t smax) {
   const uint32_t oc = wpt_ovf_cap(smax);
   return k.ring ? spec_layout(k.sw, k.ring, oc).total
-                : wpt_layout(k.nt, k.sw, k.rp, 4, oc).total;
+                : wpt_layout(k.nt, k.sw, k.off, k.ibs, oc).total;
 }
 
 template <class F>
@@ -1149,8 +1203,8 @@ int train_wpt_occupancy(int id, uint32_t Wpmax, uint32_t smax, size_t *smem_byte
   const size_t bytes = wpt_bytes(k, smax);
   *smem_bytes = bytes;
   switch (id) {
-#define TM_W(ID, NT, WPT, SW, RP, MINB) \
-  case ID: return wpt_occ(k_train_wpt<NT, WPT, SW, RP, MINB>, NT, bytes);
+#define TM_W(ID, NT, WPT, SW, RP, GP, IBS, MINB) \
+  case ID: return wpt_occ(k_train_wpt<NT, WPT, SW, RP, GP, IBS, MINB>, NT, bytes);
 #define TM_S(ID, SW, R, MINB) \
   case ID: return wpt_occ(k_train_spec<SW, R, MINB>, SP_NT, bytes);
     TM_WPT_CONFIGS(TM_W, TM_S)
@@ -1163,10 +1217,8 @@ int train_wpt_occupancy(int id, uint32_t Wpmax, uint32_t smax, size_t *smem_byte
 // The configurations worth a launch of `units` units on `sms` SMs, rows of at
 // most Wpmax words (ids, best guess first; 0 to `max` of them).
 //   k_train_wpt with the smallest row slot that holds the rows: smaller slots
-//     hold more units per SM (search rows of 49 words: 25.7 ms in 56-word
-//     slots, 27.5 ms in 64-word ones).  For rows above 512 words three register
-//     planes when the shared memory allows it (105.1 against 110.1 ms on the
-//     large sparse classifier, 6,000 samples x 2), else four.
+//     hold more units per SM (rows of 49 words: 26.2 ms in 56-word slots,
+//     27.5 ms in 64-word ones).
 //   k_train_spec up to 6 units per SM and 256 words: with few units the chain
 //     of one unit's samples is what takes the time (plain classifier, 320
 //     units: 2.8 ms against 6.6 ms), with many the evaluations it throws away
@@ -1181,8 +1233,7 @@ int wpt_choices(uint32_t Wpmax, uint32_t smax, uint32_t units, int sms, int opti
       const WptConfig &k = kWpt[id - 1];
       if ((k.ring != 0) != (spec != 0) || Wpmax > (uint32_t)k.sw) continue;
       if (wpt_bytes(k, smax) > (size_t)optin) continue;
-      if (best && kWpt[best - 1].sw < k.sw) continue;
-      if (best && kWpt[best - 1].sw == k.sw && kWpt[best - 1].rp <= k.rp) continue;
+      if (best && kWpt[best - 1].sw <= k.sw) continue;
       best = id;
     }
     if (best && n < max) ids[n++] = best;
@@ -1198,9 +1249,9 @@ cudaError_t launch_train_wpt(int id, const TrainDev *machines, const WorkItem *w
   const size_t bytes = wpt_bytes(kWpt[id - 1], smax);
   const uint32_t oc = wpt_ovf_cap(smax);
   switch (id) {
-#define TM_W(ID, NT, WPT, SW, RP, MINB)                                          \
+#define TM_W(ID, NT, WPT, SW, RP, GP, IBS, MINB)                                 \
   case ID:                                                                       \
-    k_train_wpt<NT, WPT, SW, RP, MINB><<<grid, NT, bytes, st>>>(                 \
+    k_train_wpt<NT, WPT, SW, RP, GP, IBS, MINB><<<grid, NT, bytes, st>>>(        \
         machines, work, nwork, counter, e_begin, e_end, oc, err);                \
     break;
 #define TM_S(ID, SW, R, MINB)                                                    \

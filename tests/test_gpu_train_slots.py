@@ -85,9 +85,13 @@ def test_feedback_options(tm, features, pins, include_bits, maximum, specificity
 
 
 @pytest.mark.parametrize("features,classes,clauses", [
-    (1500, 10, 760),   # 950 units of 96-word rows: the two-warp kernel
+    (1500, 10, 760),   # 950 units of 94-word rows: 128-word slots
+    (2048, 10, 760),   # 128 words, the slot's last
+    (768, 10, 760),    # 48 words, the slot's last
+    (384, 10, 760),    # 24 words, the slot's last
+    (397, 10, 760),    # 25 words, one past it
     (1500, 2, 40),     # 10 units: timed against the speculative kernel
-    (16384, 3, 16),    # 1,024 words, three register planes
+    (16384, 3, 16),    # 1,024 words
 ])
 def test_choices_without_pin(tm, features, classes, clauses):
     rng = np.random.default_rng(classes)
