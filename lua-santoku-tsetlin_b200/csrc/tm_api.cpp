@@ -174,6 +174,9 @@ struct tm_machine {
   // the actions and a chunk of samples as 4-bit floats (k_votes)
   PoolBuf act4, x4;
   bool act4_valid = false;
+  // large predicts of clauses with few literals: their lists
+  PoolBuf lists, list_groups;
+  int list_state = 0;  // 0 not looked at, 1 lists made, 2 too many literals
   int act8_kind = 0;
   // (owner of a search round) the vote kernel's copy of the actions, shared
   // by the round's machines one after another, and the expanded holdout of
@@ -201,6 +204,7 @@ static void invalidate_derived(tm_machine *m) {
   m->lits_valid = false;
   m->act8_valid = false;
   m->act4_valid = false;
+  m->list_state = 0;
 }
 
 // ---- large-batch predict as a GEMM ------------------------------------------
@@ -481,6 +485,8 @@ extern "C" void tm_destroy(tm_machine *m) {
                     &m->search_act4, &m->tune_snap, &m->few})
     b->release();
   m->act4.release(m->st);
+  m->lists.release(m->st);
+  m->list_groups.release(m->st);
   m->x4.release(m->st);
   for (DevBuf &b : m->search_x4) b.release();
   if (m->ev0) cudaEventDestroy(m->ev0);
@@ -2131,9 +2137,50 @@ static bool votes_path(tm_machine *m, uint64_t n) {
   return m->tol <= TM_VOTES_TOL && W < (1u << 19) && M < (1ull << 31) && M * n * W >= (1ull << 25);
 }
 
-// The vote sums of n byte rows through k_votes (m->sums, cleared here); 1 when
-// its status word cannot be had (nothing was queued).
-static int predict_votes(tm_machine *m, const uint8_t *rows, uint64_t n, bool on_device) {
+// Whether a large predict of n samples reads literal lists (made here, once
+// per state of the automata): machines whose action words, 16 bytes each for
+// the tensor cores, exceed L2 (20 classes x 2,048 clauses of 32,768 literals,
+// 40 samples 189 -> 53 us), and from 2^32 tests on (2^31: 60 us either way).
+// A list costs by its literals, a product by the row: lists of at most one
+// literal in 32, 40 or 56 of the row, for tiles of 4, 2 or 1 words.  Equal
+// times were measured at 256 literals of 8,192 (12.4 ms; 49 literals 2.5 ms),
+// 576 of 20,000 (1.07 ms; 49 literals 0.2) and 624 of 32,768 (7.5 ms; 49
+// literals 0.88); lists count in blocks of 16 literals and the longest of 32.
+static int ensure_lists(tm_machine *m, uint64_t n, bool *use) {
+  const ClassDev &c0 = m->cls[0];
+  const uint64_t M = (uint64_t)m->classes * m->clauses;
+  const int tw = list_tile_words(c0.W);
+  *use = false;
+  if (!tw || (M * c0.W < (1ull << 23) && M * n * c0.W < (1ull << 32))) return TM_OK;
+  if (!m->list_state) {
+    const uint64_t ng = (uint64_t)m->classes * ((m->clauses + 31) / 32);
+    CK(m->list_groups.ensure(ng * 8 + 8, m->st));
+    uint8_t *gp = m->list_groups.as<uint8_t>();
+    uint32_t tot[2];
+    CK(cudaMemsetAsync(gp + ng * 8, 0, 8, m->st));
+    CK(launch_list_plan(m->d_lits, m->classes, m->clauses, m->tol, gp, (uint32_t *)(gp + ng * 8),
+                        m->st));
+    CK(cudaMemcpyAsync(tot, gp + ng * 8, 8, cudaMemcpyDeviceToHost, m->st));
+    CK(cudaStreamSynchronize(m->st));
+    note_launch(m, 1);
+    const uint64_t ratio = tw == 4 ? 32 : (tw == 2 ? 40 : 56);
+    m->list_state = 2;
+    if (tot[1] <= TM_LIST_NEED && tot[0] * 16ull * ratio <= ng * c0.W * 32) {
+      CK(m->lists.ensure((uint64_t)tot[0] * TM_LIST_BLOCK + 16, m->st));
+      CK(launch_list_fill(m->d_act, m->classes, m->clauses, c0, gp, m->lists.p, m->st));
+      note_launch(m, 1);
+      m->list_state = 1;
+    }
+  }
+  *use = m->list_state == 1;
+  return TM_OK;
+}
+
+// The vote sums of n byte rows through literal lists (*lists set) or k_votes
+// (m->sums, cleared here); 1 when its status word cannot be had (nothing was
+// queued).
+static int predict_votes(tm_machine *m, const uint8_t *rows, uint64_t n, bool on_device,
+                         bool *lists) {
   const ClassDev &c0 = m->cls[0];
   const uint64_t M = (uint64_t)m->classes * m->clauses, K = (uint64_t)c0.W * 16;
   const uint64_t nch = m->n_chunks[0];
@@ -2147,6 +2194,25 @@ static int predict_votes(tm_machine *m, const uint8_t *rows, uint64_t n, bool on
     if (pb) memcpy(pb, rows, n * nch);
     CK(cudaMemcpyAsync(m->raw.p, pb ? pb : rows, n * nch, cudaMemcpyHostToDevice, m->st));
     rows = m->raw.as<uint8_t>();
+  }
+  int rc = ensure_lists(m, n, lists);
+  if (rc) return rc;
+  if (*lists) {
+    ListVotes v{m->lists.p, m->list_groups.p, m->d_lits, m->classes, m->clauses, m->tol, c0.W,
+                nullptr, 0, (uint32_t)nch, nullptr, nullptr, m->device, m->sms};
+    // samples per launch: at most 512 MB of slices and 2^20 samples
+    const uint64_t nc = std::min<uint64_t>(
+        1 << 20, std::max<uint64_t>(128, (512ull << 20) / (c0.W * 4ull + 1) / 128 * 128));
+    CK(m->x4.ensure(list_slice_bytes(c0.W, std::min<uint64_t>(nc, n)), m->st));
+    v.slices = m->x4.as<uint32_t>();
+    for (uint64_t s0 = 0; s0 < n; s0 += nc) {
+      v.rows = rows + s0 * nch;
+      v.n = (uint32_t)std::min<uint64_t>(nc, n - s0);
+      v.sums = m->sums.as<int32_t>() + s0 * m->classes;
+      CK(launch_list_votes(v, m->st));
+      note_launch(m, 2);
+    }
+    return TM_OK;
   }
   if (!m->act4_valid) {
     CK(m->act4.ensure(M * K, m->st));
@@ -2188,8 +2254,8 @@ static int predict_common(tm_machine *m, const uint8_t *problems, const int64_t 
   int rc = ensure_lits(m);
   if (rc) return rc;
   if (m->timing) CK(cudaEventRecord(m->ev0, m->st));
-  bool votes = votes_path(m, n);
-  int gr = votes ? predict_votes(m, problems, n, on_device) : 1;
+  bool votes = votes_path(m, n), lists = false;
+  int gr = votes ? predict_votes(m, problems, n, on_device, &lists) : 1;
   if (gr < 0) return gr;
   votes = gr == 0;
   if (gr == 1) {
@@ -2207,7 +2273,7 @@ static int predict_common(tm_machine *m, const uint8_t *problems, const int64_t 
     gr = gemm_wanted(m, n) ? predict_gemm(m, n) : 1;
     if (gr < 0) return gr;
   }
-  m->stats.predict_gemm = gr ? 0 : (votes ? TM_GEMM_FP8 : m->act8_kind);
+  m->stats.predict_gemm = gr || lists ? 0 : (votes ? TM_GEMM_FP8 : m->act8_kind);
   if (gr == 1) {
     CK(launch_predict(m->d_act, m->d_lits, m->d_cls, nullptr, m->classes, m->clauses, m->tol,
                       m->x.as<uint32_t>(), (uint32_t)n, m->sums.as<int32_t>(), m->st));

@@ -184,6 +184,30 @@ cudaError_t launch_expand_fp4_bytes(const uint8_t *src, uint64_t rows, uint32_t 
 cudaError_t launch_votes(int dev, int sms, const uint8_t *act4, const uint8_t *x4, uint32_t classes,
                          uint32_t clauses, uint32_t W, uint32_t tol, const int32_t *lits, uint32_t n,
                          int32_t *sums, const uint32_t *gate, uint32_t *err, cudaStream_t st);
+// Large-batch predict over literal lists (tm_lists.cu), for machines whose
+// clauses hold few literals.  launch_list_plan fills `groups` (8 bytes per
+// group of 32 clauses of a class) and tot[0..1] (zero before): list blocks (of
+// TM_LIST_BLOCK bytes) and the largest literal count or vote, which must not
+// exceed TM_LIST_NEED for the others.  launch_list_votes writes the vote sums
+// of byte rows (`slices`: list_slice_bytes).
+constexpr uint32_t TM_LIST_NEED = 1023, TM_LIST_BLOCK = 1024;
+struct ListVotes {
+  const void *lists, *groups;
+  const int32_t *lits;
+  uint32_t classes, clauses, tol, W;
+  const uint8_t *rows;
+  uint32_t n, row_bytes;
+  uint32_t *slices;
+  int32_t *sums;
+  int device, sms;
+};
+int list_tile_words(uint32_t W);
+uint64_t list_slice_bytes(uint32_t W, uint64_t n);
+cudaError_t launch_list_plan(const int32_t *lits, uint32_t classes, uint32_t clauses, uint32_t tol,
+                             void *groups, uint32_t *tot, cudaStream_t st);
+cudaError_t launch_list_fill(const uint32_t *act, uint32_t classes, uint32_t clauses,
+                             const ClassDev &c, const void *groups, void *lists, cudaStream_t st);
+cudaError_t launch_list_votes(const ListVotes &v, cudaStream_t st);
 cudaError_t launch_lits(const uint32_t *act, const ClassDev *cls, uint32_t classes,
                         uint32_t clauses, int32_t *lits, cudaStream_t st);
 cudaError_t launch_predict(const uint32_t *act, const int32_t *lits, const ClassDev *cls,
