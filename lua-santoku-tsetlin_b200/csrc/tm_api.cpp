@@ -177,6 +177,7 @@ struct tm_machine {
   // large predicts of clauses with few literals: their lists
   PoolBuf lists, list_groups;
   int list_state = 0;  // 0 not looked at, 1 lists made, 2 too many literals
+  uint32_t few_calls = 0;  // small predicts in this state of the automata
   int act8_kind = 0;
   // (owner of a search round) the vote kernel's copy of the actions, shared
   // by the round's machines one after another, and the expanded holdout of
@@ -205,6 +206,7 @@ static void invalidate_derived(tm_machine *m) {
   m->act8_valid = false;
   m->act4_valid = false;
   m->list_state = 0;
+  m->few_calls = 0;
 }
 
 // ---- large-batch predict as a GEMM ------------------------------------------
@@ -2138,9 +2140,10 @@ static bool votes_path(tm_machine *m, uint64_t n) {
 }
 
 // Whether a large predict of n samples reads literal lists (made here, once
-// per state of the automata): machines whose action words, 16 bytes each for
-// the tensor cores, exceed L2 (20 classes x 2,048 clauses of 32,768 literals,
-// 40 samples 189 -> 53 us), and from 2^32 tests on (2^31: 60 us either way).
+// per state of the automata): where the action and sample words, 16 bytes each
+// for the tensor cores, exceed L2 (20 classes x 2,048 clauses of 32,768
+// literals, 40 samples 189 -> 53 us), and from 2^32 tests on (2^31: 60 us
+// either way).
 // A list costs by its literals, a product by the row: lists of at most one
 // literal in 32, 40 or 56 of the row, for tiles of 4, 2 or 1 words.  Equal
 // times were measured at 256 literals of 8,192 (12.4 ms; 49 literals 2.5 ms),
@@ -2151,7 +2154,7 @@ static int ensure_lists(tm_machine *m, uint64_t n, bool *use) {
   const uint64_t M = (uint64_t)m->classes * m->clauses;
   const int tw = list_tile_words(c0.W);
   *use = false;
-  if (!tw || (M * c0.W < (1ull << 23) && M * n * c0.W < (1ull << 32))) return TM_OK;
+  if (!tw || ((M + n) * c0.W < (1ull << 23) && M * n * c0.W < (1ull << 32))) return TM_OK;
   if (!m->list_state) {
     const uint64_t ng = (uint64_t)m->classes * ((m->clauses + 31) / 32);
     CK(m->list_groups.ensure(ng * 8 + 8, m->st));
@@ -2176,6 +2179,23 @@ static int ensure_lists(tm_machine *m, uint64_t n, bool *use) {
   return TM_OK;
 }
 
+// Whether a predict of few samples reads literal lists instead of every action
+// word: three samples or more (one or two 54-74 us against 55-84 us through
+// lists) on machines beyond L2 (64 MB of actions) that have lists, or are asked
+// a second time in one state: making the lists takes as long as two to four
+// such requests.  40,960 clauses of 32,768 literals, host rows, k_predict_few ->
+// lists: 3 samples 77 -> 61 us, 8 121 -> 50, 32 380 -> 58; 262,144 clauses of
+// 8,192 literals: 3 samples 110 -> 86 us, 32 638 -> 98.
+static int few_lists(tm_machine *m, uint64_t n, bool *use) {
+  *use = false;
+  if (m->individualized || !votes_wanted() || m->tol > TM_VOTES_TOL ||
+      (uint64_t)m->classes * m->clauses * m->cls[0].W < (1ull << 24))
+    return TM_OK;
+  if (!m->list_state && m->few_calls++ == 0) return TM_OK;
+  int rc = ensure_lits(m);
+  return rc ? rc : ensure_lists(m, n, use);
+}
+
 // The vote sums of n byte rows through literal lists (*lists set) or k_votes
 // (m->sums, cleared here); 1 when its status word cannot be had (nothing was
 // queued).
@@ -2184,10 +2204,10 @@ static int predict_votes(tm_machine *m, const uint8_t *rows, uint64_t n, bool on
   const ClassDev &c0 = m->cls[0];
   const uint64_t M = (uint64_t)m->classes * m->clauses, K = (uint64_t)c0.W * 16;
   const uint64_t nch = m->n_chunks[0];
-  if (!pin_stage(m, 0)) return 1;
   if (!m->sms) m->sms = num_sms(m->device);
-  uint32_t *status = (uint32_t *)(m->pin + TM_PIN_STAGE + TM_PIN_OUT);
-  *status = 0;
+  int rc = ensure_lists(m, n, lists);
+  if (rc) return rc;
+  if (!*lists && !pin_stage(m, 0)) return 1;
   if (!on_device) {
     CK(m->raw.ensure(n * nch));
     uint8_t *pb = pin_stage(m, n * nch);
@@ -2195,8 +2215,6 @@ static int predict_votes(tm_machine *m, const uint8_t *rows, uint64_t n, bool on
     CK(cudaMemcpyAsync(m->raw.p, pb ? pb : rows, n * nch, cudaMemcpyHostToDevice, m->st));
     rows = m->raw.as<uint8_t>();
   }
-  int rc = ensure_lists(m, n, lists);
-  if (rc) return rc;
   if (*lists) {
     ListVotes v{m->lists.p, m->list_groups.p, m->d_lits, m->classes, m->clauses, m->tol, c0.W,
                 nullptr, 0, (uint32_t)nch, nullptr, nullptr, m->device, m->sms};
@@ -2214,6 +2232,8 @@ static int predict_votes(tm_machine *m, const uint8_t *rows, uint64_t n, bool on
     }
     return TM_OK;
   }
+  uint32_t *status = (uint32_t *)(m->pin + TM_PIN_STAGE + TM_PIN_OUT);
+  *status = 0;
   if (!m->act4_valid) {
     CK(m->act4.ensure(M * K, m->st));
     // dense machines: the classes' clause rows follow each other
@@ -2246,15 +2266,21 @@ static int predict_common(tm_machine *m, const uint8_t *problems, const int64_t 
   if (n >= (1ull << 31)) return fail(TM_ERR_ARG, "predict: too many samples");
   if (n == 0) return TM_OK;
   DevGuard g(m->device);
-  if (n <= TM_SMALL_N_MAX && !m->individualized && predict_few_group(m->cls[0].Wp))
+  bool lists = false;
+  int rc = TM_OK;
+  if (n > 2 && n <= TM_SMALL_N_MAX) {
+    rc = few_lists(m, n, &lists);
+    if (rc) return rc;
+  }
+  if (n <= TM_SMALL_N_MAX && !lists && !m->individualized && predict_few_group(m->cls[0].Wp))
     return predict_few(m, problems, n, out_classes, out_codes, out_scores, on_device);
   std::vector<ClassDev> cls;
   const uint64_t sb = n * m->classes * 4;
   CK(m->sums.ensure(sb));
-  int rc = ensure_lits(m);
+  rc = ensure_lits(m);
   if (rc) return rc;
   if (m->timing) CK(cudaEventRecord(m->ev0, m->st));
-  bool votes = votes_path(m, n), lists = false;
+  bool votes = lists || votes_path(m, n);
   int gr = votes ? predict_votes(m, problems, n, on_device, &lists) : 1;
   if (gr < 0) return gr;
   votes = gr == 0;
@@ -2316,7 +2342,7 @@ static int predict_common(tm_machine *m, const uint8_t *problems, const int64_t 
     if (out_scores) CK(back(out_scores, dsc, scb));
   }
   CK(cudaStreamSynchronize(m->st));
-  if (votes && *(volatile uint32_t *)(m->pin + TM_PIN_STAGE + TM_PIN_OUT))
+  if (votes && !lists && *(volatile uint32_t *)(m->pin + TM_PIN_STAGE + TM_PIN_OUT))
     return fail(TM_ERR_DEVICE, "predict: a wait of the vote kernel ran out");
   if (po) {
     const uint8_t *q = po;

@@ -1699,7 +1699,8 @@ __global__ void __launch_bounds__(256, NS <= 2 ? 3 : 2)
 // on small machines.  Whole calls from host memory, before (repack, the
 // row-per-warp kernel reading rows through L1, finalize, two copies) -> now:
 // plain classifier, one sample 36.3 -> 24.0 us; large sparse classifier, five
-// samples 133 -> 81 us.
+// samples 133 -> 81 us (repeated requests of three samples or more read lists
+// there instead).
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t maj3(uint32_t a, uint32_t b, uint32_t c) {
   uint32_t d;

@@ -89,4 +89,39 @@ def test_lists(tm, classes, features, clauses, tol, counts, sizes, lists):
             assert torch.equal(torch.as_tensor(got).cuda().reshape(-1).long(), cls), n
             sc = t.predict_scores(x.cpu().numpy().reshape(-1), n)
             assert np.array_equal(np.asarray(sc).reshape(n, classes), want.cpu().numpy()), n
+        # few samples: every action word for the first request, lists after it
+        for n in (3, 32, 1):
+            x = torch.randint(0, 256, (n, row), generator=g, device="cuda", dtype=torch.uint8)
+            want = _want(acts, x, classes, clauses, n, bits, tol).cpu().numpy()
+            for _ in range(2):
+                sc = t.predict_scores(x.cpu().numpy().reshape(-1), n)
+                assert np.array_equal(np.asarray(sc).reshape(n, classes), want), n
+    t.destroy()
+
+
+def test_few_samples_then_lists(tm):
+    """64 MB of actions: the second small request of a state makes the lists, a
+    new state starts over."""
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(3)
+    classes, features, clauses, tol = 8, 8192, 4096, 24
+    row = features // 4
+    t = tm.create("encoder", dict(hidden=classes, visible=features, clauses=clauses,
+                                  clause_tolerance=tol, clause_maximum=64, specificity=9.0,
+                                  reusable=False))
+    t.stats_enable(True)
+    ab, sb = t.class_bytes(0, classes)
+    for again in range(2):
+        buf = torch.zeros(ab + sb, dtype=torch.uint8, device="cuda")
+        hit = torch.randint(0, ab, (classes * clauses * 40,), generator=g, device="cuda")
+        buf[hit] = 1 << (again + 2)
+        torch.cuda.synchronize()
+        t.import_classes(0, classes, buf)
+        for n in (5, 5, 32, 3):
+            x = torch.randint(0, 256, (n, row), generator=g, device="cuda", dtype=torch.uint8)
+            want = _want(buf[:ab], x, classes, clauses, n, 2 * features, tol).cpu().numpy()
+            torch.cuda.synchronize()
+            sc = t.predict_scores(x.cpu().numpy().reshape(-1), n)
+            assert np.array_equal(np.asarray(sc).reshape(n, classes), want), n
     t.destroy()
