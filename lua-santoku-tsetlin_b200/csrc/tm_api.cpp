@@ -2148,7 +2148,7 @@ static bool votes_path(tm_machine *m, uint64_t n) {
 // literal in 32, 40 or 56 of the row, for tiles of 4, 2 or 1 words.  Equal
 // times were measured at 256 literals of 8,192 (12.4 ms; 49 literals 2.5 ms),
 // 576 of 20,000 (1.07 ms; 49 literals 0.2) and 624 of 32,768 (7.5 ms; 49
-// literals 0.88); lists count in blocks of 16 literals and the longest of 32.
+// literals 0.7); lists count in blocks of 16 literals and the longest of 32.
 static int ensure_lists(tm_machine *m, uint64_t n, bool *use) {
   const ClassDev &c0 = m->cls[0];
   const uint64_t M = (uint64_t)m->classes * m->clauses;
@@ -2169,7 +2169,7 @@ static int ensure_lists(tm_machine *m, uint64_t n, bool *use) {
     const uint64_t ratio = tw == 4 ? 32 : (tw == 2 ? 40 : 56);
     m->list_state = 2;
     if (tot[1] <= TM_LIST_NEED && tot[0] * 16ull * ratio <= ng * c0.W * 32) {
-      CK(m->lists.ensure((uint64_t)tot[0] * TM_LIST_BLOCK + 16, m->st));
+      CK(m->lists.ensure(((uint64_t)tot[0] + 1) * TM_LIST_BLOCK, m->st));
       CK(launch_list_fill(m->d_act, m->classes, m->clauses, c0, gp, m->lists.p, m->st));
       note_launch(m, 1);
       m->list_state = 1;

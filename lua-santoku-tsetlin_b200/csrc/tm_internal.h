@@ -188,7 +188,8 @@ cudaError_t launch_votes(int dev, int sms, const uint8_t *act4, const uint8_t *x
 // clauses hold few literals.  launch_list_plan fills `groups` (8 bytes per
 // group of 32 clauses of a class) and tot[0..1] (zero before): list blocks (of
 // TM_LIST_BLOCK bytes) and the largest literal count or vote, which must not
-// exceed TM_LIST_NEED for the others.  launch_list_votes writes the vote sums
+// exceed TM_LIST_NEED for the others; `lists` has room for one more block.
+// launch_list_votes writes the vote sums
 // of byte rows (`slices`: list_slice_bytes).
 constexpr uint32_t TM_LIST_NEED = 1023, TM_LIST_BLOCK = 1024;
 struct ListVotes {

@@ -21,8 +21,9 @@
 // wide as shared memory allows: a wide read spends fewer clocks and fewer
 // address instructions per byte.  Predicts of 20,000 samples, tensor-core
 // kernel -> lists: 256 x 1,024 clauses of 8,192 literals, 32 of them included
-// 12.4 -> 2.5 ms, 110 included 12.4 -> 6.6 ms; 20 x 2,048 clauses of 32,768
-// literals, 32 included 7.5 -> 0.88 ms, 110 included 7.5 -> 1.9 ms.
+// 12.4 -> 2.5 ms (2-word tiles 2.8), 110 included 12.4 -> 6.6 ms; 20 x 2,048
+// clauses of 32,768 literals, 32 included 7.5 -> 0.70 ms, 110 included 7.5 ->
+// 1.66 ms.
 #include <algorithm>
 #include <atomic>
 
@@ -41,7 +42,9 @@ __device__ __forceinline__ void copies_done() {
 }
 
 constexpr int SL_ACC = 12;     // planes of the vote sums kept between flushes
-constexpr int SL_NT = 384;     // threads of k_list_votes
+// threads of k_list_votes: as many warps as its registers (166, 114 and 80 a
+// thread) leave room for (one-word tiles with 384 threads 0.86 ms, 768 0.70)
+__host__ __device__ constexpr int list_threads(int tw) { return tw == 4 ? 384 : (tw == 2 ? 512 : 768); }
 constexpr uint32_t SL_SMEM = 224 * 1024;
 
 __device__ __forceinline__ uint32_t x3(uint32_t a, uint32_t b, uint32_t c) { return a ^ b ^ c; }
@@ -49,18 +52,14 @@ __device__ __forceinline__ uint32_t m3(uint32_t a, uint32_t b, uint32_t c) {
   return (a & b) | (c & (a | b));
 }
 
-// a lane's clause of group g: its literal count and the most it votes
-struct ListClause {
-  uint32_t L, cap;
-};
-__device__ __forceinline__ ListClause list_clause(const int32_t *lits, uint32_t h, uint32_t c,
-                                                  uint32_t clauses, uint32_t tol) {
-  ListClause r{0, 0};
-  if (c < clauses) {
-    r.L = (uint32_t)lits[(uint64_t)h * clauses + c];
-    r.cap = r.L == 0 || r.L > tol ? tol : r.L;
-  }
-  return r;
+// a lane's clause c of class h: its literal count, and the most it votes
+__device__ __forceinline__ uint32_t list_count(const int32_t *lits, uint32_t h, uint32_t c,
+                                               uint32_t clauses) {
+  return c < clauses ? (uint32_t)lits[(uint64_t)h * clauses + c] : 0;
+}
+__device__ __forceinline__ uint32_t list_cap(uint32_t L, uint32_t c, uint32_t clauses,
+                                             uint32_t tol) {
+  return c < clauses ? (L == 0 || L > tol ? tol : L) : 0;
 }
 
 // A warp per group: groups[g] = {first block of 16 literals, blocks | need <<
@@ -74,9 +73,9 @@ __global__ void k_list_plan(const int32_t *__restrict__ lits, uint32_t classes, 
   for (uint64_t g = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; g < ng;
        g += ((uint64_t)gridDim.x * blockDim.x) >> 5) {
     const uint32_t h = (uint32_t)(g / gpc), j = (uint32_t)(g - (uint64_t)h * gpc);
-    const ListClause k = list_clause(lits, h, j * 32 + lane, clauses, tol);
-    const uint32_t mx = __reduce_max_sync(0xFFFFFFFFu, k.L);
-    const uint32_t mc = __reduce_max_sync(0xFFFFFFFFu, k.cap);
+    const uint32_t L = list_count(lits, h, j * 32 + lane, clauses);
+    const uint32_t mx = __reduce_max_sync(0xFFFFFFFFu, L);
+    const uint32_t mc = __reduce_max_sync(0xFFFFFFFFu, list_cap(L, j * 32 + lane, clauses, tol));
     if (lane == 0) {
       const uint32_t blocks = (mx + 15) / 16, need = mx > mc ? mx : mc;
       const uint32_t off = atomicAdd(&tot[0], blocks);
@@ -228,10 +227,12 @@ __device__ __forceinline__ Words<TW> full_add(Words<TW> &a, const Words<TW> &b,
 }
 
 // The votes of one clause per lane, added to acc: P counter planes (literal
-// counts and votes below 2^P).
+// counts and votes below 2^P).  n0, n1: the first block of the group's lists
+// at lp, on return the one at `next`.
 template <int TW, int P>
-__device__ __forceinline__ void list_group(const uint32_t *xs, const uint4 *lp, uint32_t blocks,
-                                           uint32_t cap, Words<TW> (&acc)[SL_ACC]) {
+__device__ __forceinline__ void list_group(const uint32_t *xs, const uint4 *lp, const uint4 *next,
+                                           uint4 &n0, uint4 &n1, uint32_t blocks, uint32_t cap,
+                                           Words<TW> (&acc)[SL_ACC]) {
   Words<TW> f[P];
 #pragma unroll
   for (int b = 0; b < P; b++)
@@ -252,19 +253,12 @@ __device__ __forceinline__ void list_group(const uint32_t *xs, const uint4 *lp, 
     const Words<TW> b4 = full_add(f[1], c2, d2);
     return full_add(f[2], a4, b4);
   };
-  uint4 n0 = make_uint4(0, 0, 0, 0), n1 = n0;
-  if (blocks) {
-    n0 = __ldg(lp);
-    n1 = __ldg(lp + 32);
-  }
 #pragma unroll 1
   for (uint32_t b = 0; b < blocks; b++) {
     const uint4 q0 = n0, q1 = n1;
-    lp += 64;
-    if (b + 1 < blocks) {
-      n0 = __ldg(lp);
-      n1 = __ldg(lp + 32);
-    }
+    lp = b + 1 < blocks ? lp + 64 : next;
+    n0 = __ldg(lp);
+    n1 = __ldg(lp + 32);
     const Words<TW> a8 = eight(q0), b8 = eight(q1);
     Words<TW> c = full_add(f[3], a8, b8);
 #pragma unroll
@@ -275,6 +269,10 @@ __device__ __forceinline__ void list_group(const uint32_t *xs, const uint4 *lp, 
         f[p].w[t] ^= c.w[t];
         c.w[t] = k;
       }
+  }
+  if (!blocks) {
+    n0 = __ldg(next);
+    n1 = __ldg(next + 32);
   }
   // votes (capi.c:110-118): cap - failed, zero where that is negative
   uint32_t m[P];
@@ -300,22 +298,23 @@ __device__ __forceinline__ void list_group(const uint32_t *xs, const uint4 *lp, 
 
 // Grid: tiles x parts, the parts of one tile's groups `tiles` blocks apart.
 template <int TW>
-__global__ void __launch_bounds__(SL_NT, 1)
+__global__ void __launch_bounds__(list_threads(TW), 1)
     k_list_votes(const uint4 *__restrict__ lists, const uint2 *__restrict__ groups,
                  const int32_t *__restrict__ lits, uint32_t classes, uint32_t clauses, uint32_t gpc,
                  uint32_t tol, uint32_t tiles, uint32_t parts, const uint32_t *__restrict__ slices,
                  uint32_t Kp, uint32_t n, int32_t *__restrict__ sums) {
   extern __shared__ __align__(16) uint32_t xs[];
+  constexpr int NT = list_threads(TW);
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t tile = blockIdx.x % tiles, part = blockIdx.x / tiles;
   {
     const uint4 *src = (const uint4 *)(slices + (uint64_t)tile * Kp * TW);
     const uint32_t q = Kp * TW / 4;
-    for (uint32_t i = threadIdx.x; i < q; i += SL_NT) copy16((uint4 *)xs + i, src + i);
+    for (uint32_t i = threadIdx.x; i < q; i += NT) copy16((uint4 *)xs + i, src + i);
   }
   // this warp's groups
-  const uint64_t ng = (uint64_t)classes * gpc, shares = (uint64_t)parts * (SL_NT / 32);
-  const uint64_t me = (uint64_t)part * (SL_NT / 32) + warp;
+  const uint64_t ng = (uint64_t)classes * gpc, shares = (uint64_t)parts * (NT / 32);
+  const uint64_t me = (uint64_t)part * (NT / 32) + warp;
   uint64_t g = ng * me / shares;
   const uint64_t ge = ng * (me + 1) / shares;
   copies_done();
@@ -326,18 +325,31 @@ __global__ void __launch_bounds__(SL_NT, 1)
 #pragma unroll
     for (int t = 0; t < TW; t++) acc[b].w[t] = 0;
   uint32_t h = (uint32_t)(g / gpc), j = (uint32_t)(g - (uint64_t)h * gpc), used = 0;
-  uint2 gn = g < ge ? __ldg(&groups[g]) : make_uint2(0, 0);
+  // the next group's place, literal counts and first block are read while one
+  // is counted (a group with no literals names a readable block all the same)
+  uint2 gn = make_uint2(0, 0);
+  uint32_t Ln = 0;
+  if (g < ge) {
+    gn = __ldg(&groups[g]);
+    Ln = list_count(lits, h, j * 32 + lane, clauses);
+  }
+  uint4 n0 = __ldg(lists + (uint64_t)gn.x * 64 + lane);
+  uint4 n1 = __ldg(lists + (uint64_t)gn.x * 64 + lane + 32);
   while (g < ge) {
     const uint2 gi = gn;
-    if (g + 1 < ge) gn = __ldg(&groups[g + 1]);
     const uint32_t need = gi.y >> 16, blocks = gi.y & 0xFFFFu;
-    const ListClause k = list_clause(lits, h, j * 32 + lane, clauses, tol);
+    const uint32_t cap = list_cap(Ln, j * 32 + lane, clauses, tol);
+    const bool ends = ++j == gpc;
+    if (g + 1 < ge) {
+      gn = __ldg(&groups[g + 1]);
+      Ln = list_count(lits, h + ends, (ends ? 0 : j * 32) + lane, clauses);
+    }
     const uint4 *lp = lists + (uint64_t)gi.x * 64 + lane;
-    if (need < 128) list_group<TW, 7>(xs, lp, blocks, k.cap, acc);
-    else list_group<TW, 10>(xs, lp, blocks, k.cap, acc);
+    const uint4 *next = lists + (uint64_t)gn.x * 64 + lane;
+    if (need < 128) list_group<TW, 7>(xs, lp, next, n0, n1, blocks, cap, acc);
+    else list_group<TW, 10>(xs, lp, next, n0, n1, blocks, cap, acc);
     used += need < tol ? need : tol;
     g++;
-    const bool ends = ++j == gpc;
     const uint32_t after = gn.y >> 16;
     if (g < ge && !ends && used + (after < tol ? after : tol) < 1u << SL_ACC) continue;
     // the sums of the lanes of one parity (a class's clauses vote for it and
@@ -397,11 +409,11 @@ cudaError_t run_tw(const ListVotes &v, cudaStream_t st) {
   // eight waves of CTAs level out the last one, if a warp's share of a tile
   // stays eight groups or more; few tiles are split until every SM has a CTA
   const uint32_t gpc = (v.clauses + 31) / 32;
-  const uint64_t ng = (uint64_t)v.classes * gpc, warps = SL_NT / 32;
+  const uint64_t ng = (uint64_t)v.classes * gpc, warps = list_threads(TW) / 32;
   uint64_t parts = std::min<uint64_t>(((uint64_t)v.sms * 8 + tiles - 1) / tiles, ng / (warps * 8));
   const uint64_t fill = ((uint64_t)v.sms + tiles - 1) / tiles;
   parts = std::max(parts, std::min<uint64_t>(fill, (ng + warps - 1) / warps));
-  k_list_votes<TW><<<(unsigned)(tiles * parts), SL_NT, (size_t)Kp * TW * 4, st>>>(
+  k_list_votes<TW><<<(unsigned)(tiles * parts), list_threads(TW), (size_t)Kp * TW * 4, st>>>(
       (const uint4 *)v.lists, (const uint2 *)v.groups, v.lits, v.classes, v.clauses, gpc, v.tol,
       tiles, (uint32_t)parts, v.slices, Kp, v.n, v.sums);
   return cudaGetLastError();
