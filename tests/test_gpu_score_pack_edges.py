@@ -28,13 +28,37 @@ def test_pack_widths(tm, features, flip, n):
     assert np.array_equal(got.cpu().numpy(), want)
 
 
+@pytest.mark.parametrize("features", [128, 256, 384, 1152, 127, 129])
+@pytest.mark.parametrize("flip", [True, False])
+def test_pack_aligned_rows(tm, features, flip):
+    """Whole 16-byte rows, through fewer and more quads than a CTA; an output
+    that is not 16-byte aligned."""
+    import torch
+    rng = np.random.default_rng(features)
+    for n in (1, 3, 301):
+        s, f = np.nonzero(rng.random((n, features)) < 0.1)
+        idx = (s * features + f).astype(np.int64)
+        want = R.bits_to_cvec(idx, n, features, flip)
+        assert np.array_equal(tm.bits_to_cvec(idx, n, features, flip), want)
+        dev = torch.tensor(idx, device="cuda")
+        assert np.array_equal(tm.bits_to_cvec(dev, n, features, flip).cpu().numpy(), want)
+        buf = torch.zeros(want.size + 16, dtype=torch.uint8, device="cuda")
+        torch.cuda.synchronize()
+        out = buf[4:4 + want.size]
+        tm._check(tm.lib().tm_bits_to_cvec(dev.data_ptr(), dev.numel(), n, features, int(flip), 1, 0,
+                                           out.data_ptr()))
+        assert np.array_equal(out.cpu().numpy(), want.ravel())
+        assert not buf[:4].any() and not buf[4 + want.size:].any()
+
+
 def test_pack_no_set_bits(tm):
     for flip in (True, False):
         want = R.bits_to_cvec(np.zeros(0, np.int64), 5, 45, flip)
         assert np.array_equal(tm.bits_to_cvec(np.zeros(0, np.int64), 5, 45, flip), want)
 
 
-@pytest.mark.parametrize("n,hidden", [(2, 7), (3, 8), (5, 9), (70000, 3), (40, 12000), (3, 90001)])
+@pytest.mark.parametrize("n,hidden", [(2, 7), (3, 8), (5, 9), (70000, 3), (40, 12000), (3, 90001),
+                                      (50, 255), (50, 256), (50, 257), (50, 1)])
 def test_code_scores(tm, n, hidden):
     import torch
     rng = np.random.default_rng(n + hidden)
