@@ -16,8 +16,8 @@ evaluator.class_accuracy).  One step is one epoch of the round: all 64
 machines train one epoch over the 60,000 samples, then predict and score
 the 15,000 holdout samples -- `tm_train_batch_search`, one CUDA graph
 replay per epoch (the train kernels of the two row widths on two streams,
-the holdout predict of the large machines as 8-bit GEMM nodes).  `value` counts machine-samples (train + holdout) per
-second over K consecutive epochs; rounds restart after 10 epochs and their
+the holdout predict of the large machines on the tensor cores).  `value`
+counts machine-samples (train + holdout) per second over K consecutive epochs; rounds restart after 10 epochs and their
 set-up (machine creation, staging, graph capture) is inside the timed
 region.  `plain` is the same round run the reference's way: one machine at
 a time, one launch per epoch, the metric on the host between epochs.
@@ -26,7 +26,7 @@ a time, one launch per epoch, the metric on the host between epochs.
 
 Other workloads (--workload): c1 / c0 / c2 -- one machine, one step = one
 training epoch from the initial state + predict of the test set (large
-predicts as the 8-bit GEMM); serve -- resident machines under Poisson
+predicts over literal lists or on the tensor cores); serve -- resident machines under Poisson
 requests.
 
 Arms:
@@ -244,17 +244,20 @@ def balanced_chunks(classes, threads, at_most):
 #       python bench.py --profile-launch c1_small
 INSTR_PER_PAIR = {
     # batched search rows (784 / 392 features, 40 % flipped bits), 64
-    # machines, one epoch over 6,000 samples: 87.03e9, 87.91e9 and 90.86e9
+    # machines, one epoch over 6,000 samples: 87.03e9, 87.91e9 and 53.40e9
     # / 105.91e6
     ("search", 3, 1): 821.7,     # one warp per unit, four units per CTA
     ("search", 3, 2): 830.0,     # one warp per unit, one unit per CTA
-    ("search", 4, 7): 857.9,     # one warp per unit, 2 words per lane in registers
+    ("search", 4, 7): 504.2,     # word-per-thread, row slots of 56 and 32 words
     # large sparse classifier rows (16,384 features), c1_small (1.091e6 active
-    # steps): 13.54e9 global planes; 11.66e9 word-per-thread (512 x 2 words)
+    # steps): 13.54e9 global planes; 7.92e9 word-per-thread
     ("c1", 1, 1): 12410.0,
     ("c1_small", 1, 1): 12410.0,
-    ("c1", 4, 1): 10681.0,
-    ("c1_small", 4, 1): 10681.0,
+    ("c1", 4, 1): 7259.0,
+    ("c1_small", 4, 1): 7259.0,
+    # encoder rows (4,096 features), c2_small (65.54e6 active steps): 117.16e9
+    ("c2", 4, 4): 1788.0,
+    ("c2_small", 4, 4): 1788.0,
 }
 
 
@@ -440,7 +443,8 @@ def run_ours(args, w):
     key = (args.workload, st["train_mode"], st["train_cpw"])
     roof = issue_roofline(key, st["train_active_pairs"] / max(1, st["train_launches"]), avg_ms,
                           sm_mhz, extra={
-                              "kernel": "k_train_warp" if st["train_mode"] == 3 else "k_train",
+                              "kernel": {3: "k_train_warp", 4: "k_train_wpt"}.get(
+                                  st["train_mode"], "k_train"),
                               "hbm": {"algorithmic_bytes_per_launch": alg,
                                       "achieved_gbs": alg / (avg_ms / 1e3) / 1e9,
                                       "peak_gbs": peaks["hbm_gbs"], "peak_source": peak_kind,
@@ -472,24 +476,27 @@ def run_ours(args, w):
         },
     }
     if rank == 0 and st["predict_gemm"]:
-        # the predict ran as an 8-bit GEMM: clauses x samples x literal
-        # bytes (32 per row word), two operations per product
+        # the predict ran on the tensor cores: clauses x samples x literals (32
+        # per row word), two operations per product
         words = (((2 * w["features"] + 7) // 8 + 3) // 4)
         ops = 2.0 * w["classes"] * w["clauses"] * (hi_s - lo_s) * 32 * words
         t_s = st["predict_kernel_ms"] / max(1, st["predict_launches"]) / 1e3 + 1e-12
+        peak = 4.5e15 if st["predict_gemm"] == 1 else 9e15
         out["kernels"].update({
             "predict_path": "int8 GEMM" if st["predict_gemm"] == 1 else "e2m1 vote kernel",
             "predict_tensor_ops_per_s": ops / t_s,
-            "predict_tensor_peak_ops_per_s": 4.5e15,
-            "predict_tensor_peak_source": "nominal dense 8-bit rate of a B200 (no measured "
-                                          "8-bit peak here); the predict time includes the "
-                                          "byte expansions and the vote epilogue",
-            "predict_frac_of_tensor_peak": ops / t_s / 4.5e15})
+            "predict_tensor_peak_ops_per_s": peak,
+            "predict_tensor_peak_source": "nominal dense rate of a B200 at the operands' width "
+                                          "(not measured here); the predict time includes the "
+                                          "expansions and the vote epilogue",
+            "predict_frac_of_tensor_peak": ops / t_s / peak})
     elif rank == 0:
         pk = tm.int_peaks(dev.index if dev.index is not None else 0)
         wops = out["kernels"]["predict_literal_evals_per_s"] / 32
         bound = min(32 * pk["lop3"] / 62, 32 * pk["popc"] / 17)
-        out["kernels"].update({"predict_path": "bitwise", "int_peaks_ops_per_s": pk,
+        # beyond what testing every word allows: literal lists
+        path = "literal lists" if wops > bound else "bitwise"
+        out["kernels"].update({"predict_path": path, "int_peaks_ops_per_s": pk,
                                "predict_word_ops_per_s": wops,
                                "predict_int_bound_word_ops_per_s": bound,
                                "predict_frac_of_int_bound": wops / bound})

@@ -183,11 +183,13 @@ int tm_train_batch_search(tm_machine *const *machines, const tm_train_args *args
 /* machine:predict(problems, n) / (problems, dim_offsets, n): capi.c:1088-1110.
  * Classifier: out_classes[n] (int64, argmax, ties to the lowest class).
  * Encoder: out_codes[n * ceil(hidden/8)].
- * Up to 32 samples run a kernel that reads every clause row once; large
- * predicts of dense machines run as an 8-bit tensor-core GEMM of action and
- * literal bytes (exact integer accumulation: the same results), which keeps
- * a byte copy of the actions on the device (classes x clauses x 32 row
- * words bytes) until the automata change. */
+ * Up to 32 samples of a dense machine run as one kernel that reads every
+ * clause row once; large predicts of dense machines run over literal lists
+ * where clauses hold few literals (the lists, at most half the size of the
+ * actions, stay on the device until the automata change; machines with more
+ * than 64 MB of actions use them from the second small predict in a state
+ * too), else as tensor-core products of 4-bit floats (exact sums; 16 bytes
+ * per row word of the actions stay on the device as long). */
 int tm_predict(tm_machine *m, const uint8_t *problems, const int64_t *dim_offsets, uint64_t n,
                int64_t *out_classes, uint8_t *out_codes, int32_t on_device);
 
@@ -343,12 +345,12 @@ typedef struct tm_stats {
   int32_t train_mode;         /* last train kernel variant: 0 automata in shared memory,
                                  1 count planes in global memory, 2 split over a 2-CTA
                                  cluster, 3 one warp per unit (rows of at most 64 words),
-                                 4 words owned by threads (automata in registers and
-                                 shared memory) */
+                                 4 words owned by threads (actions in shared memory,
+                                 count planes there or in global memory) */
   int32_t train_autotuned;    /* 1 if the autotuner chose that variant */
   int32_t train_cpw;          /* modes 0-2: clauses per warp; mode 3: 1 = four units per
-                                 CTA, 2 = one; mode 4: the configuration (1-7) */
-  int32_t predict_gemm;       /* last predict: 0 bitwise kernels, 1 int8 GEMM, 2 GEMM of
+                                 CTA, 2 = one; mode 4: the configuration (1-12) */
+  int32_t predict_gemm;       /* last predict: 0 bitwise kernels or lists, 1 int8 GEMM, 2 GEMM of
                                  small floats (the e2m1 vote kernel, or e4m3) */
   uint64_t train_active_pairs; /* (unit, sample) steps trained after negative sampling */
   double search_epoch_ms;     /* device-resident search rounds: summed epoch graph time */
@@ -399,8 +401,8 @@ int tm_reset_stats(tm_machine *m);
  * machines, in arrival order -- into shared device launches as launch slots
  * and its device-memory budget allow; each request completes with exactly
  * the result tm_predict gives for it alone.  Large requests of dense
- * machines run as the 8-bit GEMM tm_predict uses: the server holds each
- * dense machine's action bytes (outside hbm_budget_bytes) while open, and
+ * machines run as a GEMM of 8-bit operands: the server holds each dense
+ * machine's action bytes (outside hbm_budget_bytes) while open, and
  * the machines must not train meanwhile. */
 typedef struct tm_server tm_server;
 
