@@ -827,6 +827,12 @@ __global__ void __launch_bounds__(SP_NT, MINB)
                  uint32_t nwork, uint32_t *__restrict__ counter, uint32_t e_begin, uint32_t e_end,
                  uint32_t ovf_cap, uint32_t *__restrict__ err) {
   constexpr int NK = SW / 64;       // word pairs per lane
+  // Rows above 128 words: while every first sample moves an action, one sample
+  // at a time, each warp evaluating its own clause, without a barrier after the
+  // update (80 units of 219-word rows 2.24 -> 1.87 ms, 76 encoder units of 191
+  // words 4.86 -> 4.14 ms).  In narrower rows eight evaluations cost less than
+  // the second exchange (333 units of 44 words 6.7 ms, 7.3 ms this way).
+  constexpr bool ALONE = NK >= 4;
   constexpr uint32_t FULL = 0xFFFFFFFFu;
   // rows a round may need were issued two rounds before it (R = 32) or one
   constexpr int AHEAD = R >= 32 ? 1 : 0;
@@ -892,6 +898,7 @@ __global__ void __launch_bounds__(SP_NT, MINB)
       }
       l = __reduce_add_sync(FULL, l);
       if (lane == 0) lits[warp] = l;
+      if (ALONE) __syncwarp();
     };
 #pragma unroll
     for (int k = 0; k < NK; k++) {
@@ -960,11 +967,12 @@ __global__ void __launch_bounds__(SP_NT, MINB)
         nsteps += cnt;
         // rows [from, to) of the list into their ring slots, by all threads
         auto fetch = [&](uint32_t from, uint32_t to) {
+          constexpr uint32_t TR = NK >= 4 ? 32 : 16;  // threads per row
           const uint32_t q4 = Wp >> 2;
-          for (uint32_t a = from + (tid >> 4); a < to; a += SP_NT / 16) {
+          for (uint32_t a = from + tid / TR; a < to; a += SP_NT / TR) {
             const uint32_t *src = xbase + (uint64_t)(list[a] & 0x7FFFFFFFu) * Wp;
             uint32_t *dst = ring + (a % R) * SW;
-            for (uint32_t q = tid & 15; q < q4; q += 16) cp_async_words<16>(dst + 4 * q, src + 4 * q);
+            for (uint32_t q = tid % TR; q < q4; q += TR) cp_async_words<16>(dst + 4 * q, src + 4 * q);
           }
           cp_commit();
         };
@@ -978,58 +986,93 @@ __global__ void __launch_bounds__(SP_NT, MINB)
           const uint32_t ge = cnt - g0 < SP_NT ? cnt : g0 + SP_NT;
           for (uint32_t b = g0; b < ge;) {
             const uint32_t be = b + win < ge ? b + win : ge;  // the round's end
-            // ---- this warp's sample of the round -------------------------------
-            const uint32_t a = b + warp;
-            uint32_t r = 0;
-            if (a < be) {
+            // what sample a does (lane c holds clause c's vote, `few` if its
+            // literals may grow): Type Ib clauses (capi.c:181-190), Type Ia and
+            // II << 8, Type Ia increments << 16
+            auto decide = [&](uint32_t a, int32_t vote, bool few) -> uint32_t {
               const bool pa = list[a] >> 31;
               const int32_t tc = thr[(a - g0) * 8 + cl];
-              const uint32_t L = lits[cl];
-              const uint32_t *xs = ring + (a % R) * SW + 2 * lane;
-              uint32_t f[8] = {};
-#pragma unroll
-              for (int k = 0; k < NK; k++) {
-                uint2 x = *(const uint2 *)(xs + 64 * k);
-                x.x |= ~em[k][0];
-                x.y |= ~em[k][1];
-#pragma unroll
-                for (int c = 0; c < 8; c++) {
-                  const uint2 t = *(const uint2 *)(planes + (c * 8 + M7) * SW + 2 * lane + 64 * k);
-                  f[c] += __popc(t.x & ~x.x) + __popc(t.y & ~x.y);
-                }
-              }
-              uint32_t pk[4];
-#pragma unroll
-              for (int c = 0; c < 4; c++)
-                pk[c] = __reduce_add_sync(FULL, f[2 * c] + (f[2 * c + 1] << 16));
-              const uint32_t pr =
-                  (lane & 4) ? ((lane & 2) ? pk[3] : pk[2]) : ((lane & 2) ? pk[1] : pk[0]);
-              const uint32_t F = (lane & 1) ? pr >> 16 : pr & 0xFFFFu;
-              // votes (capi.c:110-118), signed by clause parity (:148-161)
-              int32_t vote = (int32_t)(L == 0 || L > tol ? tol : L) - (int32_t)F;
-              vote = vote < 0 ? 0 : vote;
               const int32_t v = (int32_t)__reduce_add_sync(FULL, (uint32_t)(vote * sign));
               const uint32_t fm = __ballot_sync(FULL, (pa ? v : -v) < tc) & 0xFFu;
-              if (fm) {
-                const uint32_t vt = __ballot_sync(FULL, vote > 0);
-                const uint32_t inc = __ballot_sync(FULL, L <= maxlit);
-                const uint32_t t1 = pa ? 0x55u : 0xAAu;  // Type I clauses
-                // Type Ib (capi.c:181-190), Type Ia and II, Type Ia increments
-                r = (fm & t1 & ~vt) | (fm & vt) << 8 | (fm & vt & t1 & inc & 0xFFu) << 16;
+              if (!fm) return 0;
+              const uint32_t vt = __ballot_sync(FULL, vote > 0);
+              const uint32_t inc = __ballot_sync(FULL, few);
+              const uint32_t t1 = pa ? 0x55u : 0xAAu;  // Type I clauses
+              return (fm & t1 & ~vt) | (fm & vt) << 8 | (fm & vt & t1 & inc & 0xFFu) << 16;
+            };
+            // votes (capi.c:110-118), signed by clause parity (:148-161)
+            auto votes = [&](uint32_t L, uint32_t F) {
+              const int32_t vote = (int32_t)(L == 0 || L > tol ? tol : L) - (int32_t)F;
+              return vote < 0 ? 0 : vote;
+            };
+            uint32_t rs;  // lane w: what the round's sample w does
+            const bool alone = ALONE && win == 1;
+            if (alone) {
+              // ---- one sample, each warp its own clause ---------------------------
+              const uint32_t *xs = ring + (b % R) * SW + 2 * lane;
+              uint32_t f = 0;
+#pragma unroll
+              for (int k = 0; k < NK; k++) {
+                const uint2 x = *(const uint2 *)(xs + 64 * k);
+                const uint2 t = *(const uint2 *)(own + M7 * SW + 64 * k);
+                f += __popc(t.x & em[k][0] & ~x.x) + __popc(t.y & em[k][1] & ~x.y);
               }
+              f = __reduce_add_sync(FULL, f);
+              const uint32_t L = lits[warp];
+              if (lane == 0)
+                res[par * SPW + warp] = (uint32_t)votes(L, f) | (L <= maxlit ? 0x80000000u : 0u);
+              cp_wait<AHEAD>();
+              __syncthreads();
+              const uint32_t rv = res[par * SPW + cl];
+              const uint32_t r = decide(b, (int32_t)(rv & 0x7FFFFFFFu), rv >> 31);
+              rs = cl == 0 ? r : 0;
+            } else {
+              // ---- this warp's sample of the round --------------------------------
+              const uint32_t a = b + warp;
+              uint32_t r = 0;
+              if (a < be) {
+                const uint32_t L = lits[cl];
+                const uint32_t *xs = ring + (a % R) * SW + 2 * lane;
+                uint32_t f[8] = {};
+#pragma unroll
+                for (int k = 0; k < NK; k++) {
+                  uint2 x = *(const uint2 *)(xs + 64 * k);
+                  x.x |= ~em[k][0];
+                  x.y |= ~em[k][1];
+#pragma unroll
+                  for (int c = 0; c < 8; c++) {
+                    const uint2 t =
+                        *(const uint2 *)(planes + (c * 8 + M7) * SW + 2 * lane + 64 * k);
+                    f[c] += __popc(t.x & ~x.x) + __popc(t.y & ~x.y);
+                  }
+                }
+                uint32_t pk[4];
+#pragma unroll
+                for (int c = 0; c < 4; c++)
+                  pk[c] = __reduce_add_sync(FULL, f[2 * c] + (f[2 * c + 1] << 16));
+                const uint32_t pr =
+                    (lane & 4) ? ((lane & 2) ? pk[3] : pk[2]) : ((lane & 2) ? pk[1] : pk[0]);
+                r = decide(a, votes(L, (lane & 1) ? pr >> 16 : pr & 0xFFFFu), L <= maxlit);
+              }
+              if (lane == 0) res[par * SPW + warp] = r;
+              cp_wait<AHEAD>();
+              __syncthreads();
+              rs = res[par * SPW + cl];
             }
-            if (lane == 0) res[par * SPW + warp] = r;
-            cp_wait<AHEAD>();
-            __syncthreads();
-            // rows behind this round are done with: refill their slots
-            {
+            // rows behind this round are done with: refill their slots, eight at
+            // a time while the rounds are single samples (a round that grows from
+            // one sample reaches at most 15 rows within the two rounds that its
+            // copies may take; a ring of 16 is refilled at once)
+            if (!alone || AHEAD == 0 || b + R - fetched >= 8) {
               const uint32_t to = cnt - b < (uint32_t)R ? cnt : b + R;
               fetch(fetched, to);
               fetched = to;
+            } else {
+              cp_commit();
             }
             // ---- feedback of the round's samples, in order -----------------------
-            const uint32_t rs = res[par * SPW + cl];
             par ^= 1u;
+            bool moved = false;
             uint32_t next = be;
             for (uint32_t pend = __ballot_sync(FULL, rs != 0) & 0xFFu; pend; pend &= pend - 1) {
               const uint32_t w = __ffs(pend) - 1;
@@ -1108,14 +1151,18 @@ __global__ void __launch_bounds__(SP_NT, MINB)
                 // an action may have moved: the later results no longer hold
                 if ((ibm | fbm) & jbit) recount();
                 next = b + w + 1;
-                __syncthreads();
+                moved = true;
+                if (!alone) __syncthreads();  // alone, a warp reads its own clause only
                 break;
               }
             }
             // a round that ended early is followed by one that little longer
-            // (evaluations thrown away take issue slots from other units), a
-            // full one by one of twice its length
-            const uint32_t grown = next < be ? next - b + 1 : 2 * win;
+            // (evaluations thrown away take issue slots from other units), in
+            // the ALONE form by one sample if its first one ended it; a full
+            // one by one of twice its length
+            const uint32_t done = next - b;
+            const uint32_t grown = ALONE && moved && done == 1 ? 1
+                                   : (next < be ? done + 1 : 2 * win);
             win = grown < SPW ? grown : SPW;
             b = next;
           }
@@ -1165,18 +1212,24 @@ __global__ void __launch_bounds__(SP_NT, MINB)
   W(12, 32, 1, 24, 0, 0, 4, 20)
 
 struct WptConfig {
-  int ring;  // ring slots of k_train_spec, 0: k_train_wpt
+  int id, ring;  // ring slots of k_train_spec, 0: k_train_wpt
   int nt, sw, off;  // off: count planes not in shared memory
   int ibs;
 };
-static const WptConfig kWpt[] = {
-#define TM_W(ID, NT, WPT, SW, RP, GP, IBS, MINB) {0, NT, SW, RP + GP, IBS},
-#define TM_S(ID, SW, R, MINB) {R, (int)SP_NT, SW, 0, 4},
+static constexpr WptConfig kWpt[] = {
+#define TM_W(ID, NT, WPT, SW, RP, GP, IBS, MINB) {ID, 0, NT, SW, RP + GP, IBS},
+#define TM_S(ID, SW, R, MINB) {ID, R, (int)SP_NT, SW, 0, 4},
     TM_WPT_CONFIGS(TM_W, TM_S)
 #undef TM_W
 #undef TM_S
 };
 constexpr int kWptCount = (int)(sizeof(kWpt) / sizeof(kWpt[0]));
+constexpr bool wpt_in_order() {
+  for (int i = 0; i < kWptCount; i++)
+    if (kWpt[i].id != i + 1) return false;
+  return true;
+}
+static_assert(wpt_in_order(), "a configuration's place is its id");
 
 static uint32_t wpt_ovf_cap(uint32_t smax) { return smax / 4 > 0 ? smax / 4 : 1; }
 
