@@ -243,7 +243,7 @@ static bool votes_wanted() {
 
 constexpr uint64_t TM_PIN_STAGE = 256 << 10;
 // the output half ends with the status word of k_votes (a larger block would
-// leave the 512 KB that the driver serves from one chunk: 1.3 ms instead of 6 us)
+// leave the 512 KB that CUDA serves from one chunk: 1.3 ms instead of 6 us)
 constexpr uint64_t TM_PIN_OUT = TM_PIN_STAGE - 64;
 
 // The input half of the machine's pinned staging buffer, ready to be
