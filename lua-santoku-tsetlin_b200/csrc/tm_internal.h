@@ -117,6 +117,7 @@ constexpr uint32_t TM_ORDER_BATCH = 64;  // orders per launch
 size_t order_scratch_bytes(uint32_t n);
 cudaError_t launch_orders(OrderJob *jobs, size_t count, void *scratch, size_t scratch_bytes,
                           cudaStream_t st, const uint32_t *epoch_dev, uint64_t *launches);
+void raise_smem(const void *kernel);
 // k_train variants: automata in shared memory (one CTA per unit), in global
 // memory (one CTA per unit), or split over a 2-CTA cluster in shared memory.
 constexpr int TM_MODE_SMEM = 0;

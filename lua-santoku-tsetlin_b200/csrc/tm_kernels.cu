@@ -1124,6 +1124,22 @@ __global__ void __launch_bounds__(WPC * 32)
   }
 }
 
+// Lets `kernel` take all the dynamic shared memory a block can opt into on the
+// current device.  Always that much, never a launch's own size: a limit that
+// followed the launch being planned would be too low for another one of the
+// same kernel -- a search round plans two train launches before it runs them,
+// and host threads plan theirs at any time.
+void raise_smem(const void *kernel) {
+  int dev = 0, optin = 0;
+  cudaFuncAttributes a;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
+      cudaFuncGetAttributes(&a, kernel) != cudaSuccess)
+    return;
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       optin - (int)a.sharedSizeBytes);
+}
+
 // shared memory per warp of k_train_warp, in words (a multiple of 32)
 static uint32_t warp_slice_words(uint32_t Wpmax, uint32_t Bmax, uint32_t ib_words,
                                  uint32_t ovf_cap) {
@@ -1132,10 +1148,8 @@ static uint32_t warp_slice_words(uint32_t Wpmax, uint32_t Bmax, uint32_t ib_word
 
 template <int WPC>
 static int warp_occ(bool exact, size_t bytes) {
-  cudaFuncSetAttribute(k_train_warp<7, false, WPC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)bytes);
-  cudaFuncSetAttribute(k_train_warp<7, true, WPC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)bytes);
+  raise_smem((const void *)k_train_warp<7, false, WPC>);
+  raise_smem((const void *)k_train_warp<7, true, WPC>);
   int nb = 0;
   if (exact)
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_train_warp<7, true, WPC>, WPC * 32, bytes);
@@ -1187,8 +1201,7 @@ cudaError_t launch_train_warp(const TrainDev *machines, const WorkItem *work, ui
 
 template <bool S, bool P, int BM, bool EX = false, int CPW = 1>
 static int occ_of(const TrainSmem &lay) {
-  cudaFuncSetAttribute(k_train<S, P, BM, EX, CPW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       lay.total);
+  raise_smem((const void *)k_train<S, P, BM, EX, CPW>);
   if (!P) {
     int nb = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_train<S, P, BM, EX, CPW>,

@@ -1241,7 +1241,7 @@ static size_t wpt_bytes(const WptConfig &k, uint32_t smax) {
 
 template <class F>
 static int wpt_occ(F kernel, int threads, size_t bytes) {
-  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  raise_smem((const void *)kernel);
   int nb = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, threads, bytes);
   return nb;
