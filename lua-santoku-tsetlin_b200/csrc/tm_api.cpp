@@ -848,6 +848,21 @@ static bool lookup_tuned(const TrainShape &sh, const tm_machine *m0, TrainPlan &
   return plan_mode(v.first, sh, out, v.second);
 }
 
+// The plans of the kernels of tm_train_wpt.cu that are worth this launch, best
+// guess first: 8-bit units of rows up to 1,024 words, where they beat every
+// other variant at each width measured (4 to 1,024 words, 40 to 93,000 units).
+static std::vector<TrainPlan> wpt_plans(const TrainShape &sh) {
+  std::vector<TrainPlan> plans;
+  if (sh.Bmin != 8 || sh.Bmax != 8) return plans;
+  int ids[4];
+  const int k = wpt_choices(sh.Wpmax, sh.smax, sh.units, sh.sms, sh.optin, ids, 4);
+  for (int i = 0; i < k; i++) {
+    TrainPlan p;
+    if (plan_mode(TM_MODE_WPT, sh, p, ids[i])) plans.push_back(p);
+  }
+  return plans;
+}
+
 // Times every feasible variant on the first samples of epoch 0 of a
 // sample of the launch's units, keeps the fastest, and resets the automata
 // of every job to their initial state.
@@ -855,6 +870,12 @@ static int autotune_plan(std::vector<TrainJob> &jobs, const std::vector<TrainDev
                          const std::vector<WorkItem> &work, const TrainShape &sh,
                          tm_machine *m0, TrainPlan &out, bool &tuned) {
   tuned = false;
+  std::vector<TrainPlan> cand = wpt_plans(sh);
+  if (cand.size() == 1) {  // nothing to time
+    out = cand[0];
+    tuned = true;
+    return TM_OK;
+  }
   if (m0->autotune == 1 && lookup_tuned(sh, m0, out)) {
     tuned = true;
     return TM_OK;
@@ -862,20 +883,6 @@ static int autotune_plan(std::vector<TrainJob> &jobs, const std::vector<TrainDev
   if (!m0->ev0) {
     CK(cudaEventCreate(&m0->ev0));
     CK(cudaEventCreate(&m0->ev1));
-  }
-  std::vector<TrainPlan> cand;
-  // 8-bit units of rows up to 1,024 words: the kernels of tm_train_wpt.cu beat
-  // every other variant at each width measured (28 to 1,024 words, 40 to
-  // 93,000 units), so only their choices are tried; the others serve what
-  // these cannot hold (other state widths, wider rows, overflow lists of a
-  // very low specificity that do not fit the shared memory).
-  if (sh.Bmin == 8 && sh.Bmax == 8) {
-    int ids[4];
-    const int k = wpt_choices(sh.Wpmax, sh.smax, sh.units, sh.sms, sh.optin, ids, 4);
-    for (int i = 0; i < k; i++) {
-      TrainPlan p;
-      if (plan_mode(TM_MODE_WPT, sh, p, ids[i])) cand.push_back(p);
-    }
   }
   if (cand.empty())
     for (int mode : {TM_MODE_WARP, TM_MODE_SMEM, TM_MODE_GLOBAL, TM_MODE_PAIR}) {
@@ -885,11 +892,6 @@ static int autotune_plan(std::vector<TrainJob> &jobs, const std::vector<TrainDev
         if (plan_mode(mode, sh, p, cpw)) cand.push_back(p);
       }
     }
-  if (cand.size() == 1 && cand[0].mode == TM_MODE_WPT) {  // nothing to time
-    out = cand[0];
-    tuned = true;
-    return TM_OK;
-  }
   if (cand.size() < 2) return TM_OK;  // nothing to choose: the heuristic plan
   // Two trials, each on automata reset to the initial state (capi.c:1136-
   // 1146; a trial on automata that earlier trials trained would see another
@@ -1110,8 +1112,10 @@ static void build_tables(std::vector<TrainJob> &jobs, uint32_t e0, uint32_t e1, 
                   num_sms(dev)};
 }
 
-// The train-kernel variant of a launch: pinned, tuned (trials at epoch 0,
-// on the freshly reset automata) or by the heuristic.
+// The train-kernel variant of a launch: pinned, tuned (trials at epoch 0, on
+// the freshly reset automata; later launches of the call take what they found,
+// or where none ran -- one choice only, or machines of the call that stopped
+// left another shape -- the best guess) or, untuned, by the heuristic.
 static int choose_plan(std::vector<TrainJob> &jobs, const std::vector<TrainDev> &td,
                        const std::vector<WorkItem> &work, const TrainShape &sh, uint32_t e0,
                        tm_machine *m0, TrainPlan &plan, bool &tuned) {
@@ -1126,14 +1130,19 @@ static int choose_plan(std::vector<TrainJob> &jobs, const std::vector<TrainDev> 
     int rc = autotune_plan(jobs, td, work, sh, m0, plan, tuned);
     if (rc) return rc;
   }
-  if (!tuned && m0->force_mode < 0) {
-    if (m0->autotune && lookup_tuned(sh, m0, plan)) {
+  if (!tuned && m0->force_mode < 0 && m0->autotune) {
+    const std::vector<TrainPlan> plans = wpt_plans(sh);
+    if (plans.size() == 1) {
+      plan = plans[0];
       tuned = true;
-    } else {
-      int rc = heuristic_plan(sh, m0, plan);
-      if (rc) return rc;
+    } else if (lookup_tuned(sh, m0, plan)) {
+      tuned = true;
+    } else if (!plans.empty()) {
+      plan = plans[0];
+      tuned = true;
     }
   }
+  if (!tuned && m0->force_mode < 0) return heuristic_plan(sh, m0, plan);
   return TM_OK;
 }
 

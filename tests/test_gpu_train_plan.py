@@ -1,0 +1,74 @@
+"""Which train kernel runs: a call that launches once per epoch (an `each`
+callback, a batch with one, machines of a batch that end early) keeps the
+word-per-thread kernels (train_mode 4) after its first epoch, whether the tuner
+timed two of them or had one choice, and ends in the state of a call that runs
+all epochs at once."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [
+    (10, 784, 760),    # 950 units: one choice
+    (3, 16384, 16),    # rows above 256 words: one choice
+    (10, 784, 64),     # 80 units: two choices, timed
+]
+IDS = ["units950", "words1024", "units80"]
+
+
+def _table(classes, features, clauses, seed=1):
+    return dict(classes=classes, features=features, clauses=clauses, clause_tolerance=16,
+                clause_maximum=50, specificity=11.0, target=20, reusable=True, seed=seed)
+
+
+def _inputs(classes, features, n=120):
+    rng = np.random.default_rng(classes * features)
+    b = rng.random((n, features)) < 0.1
+    x = np.packbits(np.concatenate([b, ~b], axis=1), axis=1, bitorder="little").ravel()
+    return dict(samples=n, problems=x, solutions=rng.integers(0, classes, size=n).astype(np.int64),
+                iterations=3)
+
+
+@pytest.mark.parametrize("autotune", [1, 2])
+@pytest.mark.parametrize("shape", SHAPES, ids=IDS)
+def test_each_epoch_keeps_the_kernel(tm, shape, autotune):
+    inp = _inputs(shape[0], shape[1])
+    t = tm.create("classifier", _table(*shape))
+    t.set_autotune(autotune)
+    t.stats_enable(True)
+    seen = []
+
+    def each(epoch):
+        st = t.stats()
+        seen.append((st["train_mode"], st["train_cpw"], st["train_autotuned"]))
+        return True
+
+    t.train(dict(inp, each=each))
+    assert len(seen) == 3 and seen[0][0] == 4 and set(seen) == {seen[0]}, seen
+    assert seen[0][2] == 1
+    once = tm.create("classifier", _table(*shape))
+    once.set_autotune(0)
+    once.train(inp)
+    for a, b in zip(t.export_state(), once.export_state()):
+        assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("shape", SHAPES, ids=IDS)
+def test_batch_epochs_keep_the_kernel(tm, shape):
+    inp = _inputs(shape[0], shape[1])
+    ms = [tm.create("classifier", _table(*shape, seed=i)) for i in range(3)]
+    ms[0].stats_enable(True)
+    seen = []
+
+    def each(epoch):
+        seen.append(ms[0].stats()["train_mode"])
+
+    # machine i trains i + 1 epochs: each launch has fewer units than the one before
+    tm.train_batch(ms, [dict(inp, iterations=i + 1) for i in range(3)], each=each)
+    assert seen == [4, 4, 4]
+    for i, m in enumerate(ms):
+        once = tm.create("classifier", _table(*shape, seed=i))
+        once.set_autotune(0)
+        once.train(dict(inp, iterations=i + 1))
+        for a, b in zip(m.export_state(), once.export_state()):
+            assert np.array_equal(a, b)
