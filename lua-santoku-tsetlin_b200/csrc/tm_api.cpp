@@ -692,6 +692,7 @@ static int validate_train(tm_machine *m, const tm_train_args *a) {
 struct TrainShape {
   uint32_t Wpmax, Bmin, Bmax, smax, units;
   int optin, sms;
+  bool many_ovf;  // Type Ib clauses meet overflow entries often (WPT_OVF)
 };
 
 struct TrainPlan {
@@ -715,7 +716,7 @@ static bool plan_mode(int mode, const TrainShape &sh, TrainPlan &p, int cpw = 1)
     // cpw is the configuration id; the automata of 8-bit units only
     if (sh.Bmin != 8 || sh.Bmax != 8) return false;
     size_t bytes = 0;
-    const int occ = train_wpt_occupancy(cpw, sh.Wpmax, sh.smax, &bytes);
+    const int occ = train_wpt_occupancy(cpw, sh.Wpmax, sh.smax, sh.many_ovf, &bytes);
     if (occ <= 0 || (int)bytes > sh.optin) return false;
     p.grid = (int)std::min<uint64_t>(sh.units, (uint64_t)sh.sms * occ);
     return true;
@@ -806,8 +807,8 @@ static int launch_plan(const TrainPlan &p, const TrainShape &sh, const std::vect
                          (unsigned long long *)(err + 2)));
   else if (p.mode == TM_MODE_WPT)
     CK(launch_train_wpt(p.cpw, (const TrainDev *)base, (const WorkItem *)(base + off_w),
-                        (uint32_t)work.size(), counter, e0, e1, sh.Wpmax, sh.smax, p.grid, err,
-                        st));
+                        (uint32_t)work.size(), counter, e0, e1, sh.Wpmax, sh.smax, sh.many_ovf,
+                        p.grid, err, st));
   else
     CK(launch_train((const TrainDev *)base, (const WorkItem *)(base + off_w),
                     (uint32_t)work.size(), counter, e0, e1, lay, p.mode, sh.Bmin, sh.Bmax,
@@ -832,8 +833,8 @@ static std::string tune_key(const TrainShape &sh, const tm_machine *m0) {
   // units bucketed by powers of two: the wave count matters, not the exact count
   uint32_t ub = 0;
   while ((1u << ub) < sh.units && ub < 31) ub++;
-  snprintf(k, sizeof k, "%d:%u:%u:%u:%u:%u:%d:%d", m0->device, sh.Wpmax, sh.Bmin, sh.Bmax, sh.smax,
-           ub, m0->no_warp ? 1 : 0, m0->pair ? 1 : 0);
+  snprintf(k, sizeof k, "%d:%u:%u:%u:%u:%u:%d:%d:%d", m0->device, sh.Wpmax, sh.Bmin, sh.Bmax, sh.smax,
+           ub, m0->no_warp ? 1 : 0, m0->pair ? 1 : 0, sh.many_ovf ? 1 : 0);
   return k;
 }
 
@@ -1063,6 +1064,7 @@ static void build_tables(std::vector<TrainJob> &jobs, uint32_t e0, uint32_t e1, 
   td.assign(jobs.size(), TrainDev{});
   work.clear();
   uint32_t Wpmax = 4, Bmin = 32, Bmax = 2, smax = 0;
+  double ovf = 0.0;
   for (size_t i = 0; i < jobs.size(); i++) {
     TrainJob &J = jobs[i];
     tm_machine *m = J.m;
@@ -1095,6 +1097,7 @@ static void build_tables(std::vector<TrainJob> &jobs, uint32_t e0, uint32_t e1, 
       const ClassDev &c = J.cls[h];
       Wpmax = std::max(Wpmax, c.Wp);
       smax = std::max(smax, c.s_picks);
+      ovf += wpt_overflow(c.input_bits, c.s_picks) * m->clause_chunks;
       const double frac =
           m->type == TM_CLASSIFIER ? std::min(1.0, 1.0 / m->classes + m->negative) : 1.0;
       const double cost = (double)t.n * (t.epochs - e0) * frac * c.Wp * m->B *
@@ -1109,7 +1112,7 @@ static void build_tables(std::vector<TrainJob> &jobs, uint32_t e0, uint32_t e1, 
                    [](const WorkItem &a, const WorkItem &b) { return a.cost > b.cost; });
   const int dev = m0->device;
   sh = TrainShape{Wpmax, Bmin, Bmax, smax, (uint32_t)work.size(), max_smem_optin(dev),
-                  num_sms(dev)};
+                  num_sms(dev), ovf >= WPT_OVF * work.size()};
 }
 
 // The train-kernel variant of a launch: pinned, tuned (trials at epoch 0, on
@@ -1684,15 +1687,18 @@ static int search_round(tm_machine *const *ms, const tm_train_args *args, uint32
         out.Bmin = 32;
         out.Bmax = 2;
         out.smax = 0;
+        double ovf = 0.0;
         for (const WorkItem &wi : w) {
           const ClassDev &c = jobs[wi.m].cls[wi.h];
           const uint32_t B = jobs[wi.m].m->B;
           out.Wpmax = std::max(out.Wpmax, c.Wp);
           out.smax = std::max(out.smax, c.s_picks);
+          ovf += wpt_overflow(c.input_bits, c.s_picks);
           out.Bmin = std::min(out.Bmin, B);
           out.Bmax = std::max(out.Bmax, B);
         }
         out.units = (uint32_t)w.size();
+        out.many_ovf = ovf >= WPT_OVF * w.size();
       };
       shape_of(work_n, sh_n);
       shape_of(wide, sh);
@@ -1759,7 +1765,7 @@ static int search_round(tm_machine *const *ms, const tm_train_args *args, uint32
                                (unsigned long long *)(d_err + 2));
     if (pl.mode == TM_MODE_WPT)
       return launch_train_wpt(pl.cpw, (const TrainDev *)tbase, wk, nw, ctr, 0, 1, shp.Wpmax,
-                              shp.smax, pl.grid, d_err, s_);
+                              shp.smax, shp.many_ovf, pl.grid, d_err, s_);
     return launch_train((const TrainDev *)tbase, wk, nw, ctr, 0, 1, ly, pl.mode, shp.Bmin,
                         shp.Bmax, pl.cpw, pl.grid, d_err, s_);
   };

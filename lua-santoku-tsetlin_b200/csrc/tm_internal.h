@@ -166,10 +166,17 @@ constexpr int TM_WPT_PINNED = 8;
 constexpr int TM_MODE_WPT = 4;
 int wpt_choices(uint32_t Wpmax, uint32_t smax, uint32_t units, int sms, int optin, int *ids,
                 int max);
-int train_wpt_occupancy(int id, uint32_t Wpmax, uint32_t smax, size_t *smem_bytes);
+// Overflow entries that a Type Ib clause of `bits` literals expects: bits picked
+// four times and more.  Launches whose units average WPT_OVF or more (many_ovf)
+// run the kernels' form for many entries.  Times without it over times with it:
+// 0.91 to 1.05 below one entry, 1.00 to 1.06 at 1.4, 0.95 to 1.05 at 1.6, 0.96 to
+// 1.15 at 2.4, 1.1 to 1.5 at 9, 3.3 to 7.2 at 125.
+constexpr double WPT_OVF = 1.5;
+double wpt_overflow(uint32_t bits, uint32_t picks);
+int train_wpt_occupancy(int id, uint32_t Wpmax, uint32_t smax, bool many_ovf, size_t *smem_bytes);
 cudaError_t launch_train_wpt(int id, const TrainDev *machines, const WorkItem *work,
                              uint32_t nwork, uint32_t *counter, uint32_t e_begin, uint32_t e_end,
-                             uint32_t Wpmax, uint32_t smax, int grid, uint32_t *err,
+                             uint32_t Wpmax, uint32_t smax, bool many_ovf, int grid, uint32_t *err,
                              cudaStream_t st);
 // Large-batch predict in one tensor-core kernel (tm_votes.cu): bit rows as
 // 4-bit floats (16 bytes per word), and the vote sums of n samples x classes

@@ -31,6 +31,8 @@
 // 8,000 samples x 10 epochs, 320 units, 15.0 -> 2.8 ms; encoder rows of 256
 // words 190 -> 113 ms; sparse classifier rows of 1,024 words 127 -> 90 ms.
 // The same rules and draws as k_train, so the same automata bit for bit.
+#include <math.h>
+
 #include "tm_device.cuh"
 
 namespace tmb {
@@ -279,6 +281,24 @@ __device__ __forceinline__ void draw_picks(uint32_t ibm, uint32_t sp, uint32_t e
   }
 }
 
+// Overflow entries (each worth 4) of one clause that lie in words [first, first
+// + words), those of the calling warp: their bits into the level-1 words `l1`,
+// which the warp's lanes have read and cleared.  A lane takes every 32nd entry
+// from `at` on and stops at a bit that is set already: it waits until the
+// caller has subtracted and cleared what there is.  (Rows of 24,000 literals at
+// specificity 1.2, 250 entries per clause, 800 units: 121.8 ms with every entry
+// subtracted from every word, 16.3 ms this way.)
+__device__ __forceinline__ void take_overflow(const uint16_t *entries, uint32_t n, uint32_t &at,
+                                              uint32_t first, uint32_t words, uint32_t *l1) {
+  __syncwarp();
+  while (at < n) {
+    const uint32_t e = entries[at], w = e >> 5, bit = 1u << (e & 31);
+    if (w - first < words && (atomicOr(&l1[w], bit) & bit)) break;
+    at += 32;
+  }
+  __syncwarp();
+}
+
 // samples whose vote thresholds are held at a time
 __host__ __device__ constexpr uint32_t wpt_group(uint32_t NT) { return NT < 64 ? NT : 64; }
 
@@ -321,8 +341,11 @@ __host__ __device__ constexpr WptLayout wpt_layout(uint32_t NT, uint32_t SW, int
 // row slot (at most NT * WPT, at least the widest row).  The first RP count
 // planes are held in registers, the last GP in global memory, the others and
 // the actions in shared memory; IBS Type Ib clauses are drawn at a time; MINB
-// CTAs per SM the registers are sized for.
-template <int NT, int WPT, int SW, int RP, int GP, int IBS, int MINB>
+// CTAs per SM the registers are sized for; OV for launches whose Type Ib
+// clauses meet overflow entries at all often (WPT_OVF): a warp hands them to
+// the lanes they concern, where the other form, cheaper without entries,
+// subtracts each from every word.
+template <int NT, int WPT, int SW, int RP, int GP, int IBS, int MINB, bool OV>
 __global__ void __launch_bounds__(NT, MINB)
     k_train_wpt(const TrainDev *__restrict__ machines, const WorkItem *__restrict__ work,
                 uint32_t nwork, uint32_t *__restrict__ counter, uint32_t e_begin, uint32_t e_end,
@@ -689,15 +712,37 @@ __global__ void __launch_bounds__(NT, MINB)
                     for (int q = 0; q < WPT; q++) m0[q] = m1[q] = 0;
                   }
                   // an overflow entry is worth 4: twice a level-1 count
-                  const uint32_t no = 2 * min(oc[slot], ovf_cap);
-                  for (uint32_t t = 0;; t++) {
-                    count_sub(p, ac, m0, m1, am);
-                    if (t >= no) break;
-                    const uint32_t bit = ovf[slot * ovf_cap + (t >> 1)];
+                  if constexpr (OV) {
+                    const uint32_t no = min(oc[slot], ovf_cap);
+                    uint32_t next = lane;  // this lane's next entry
+                    for (uint32_t t = 0;; t++) {
+                      count_sub(p, ac, m0, m1, am);
+                      if (t & 1u) continue;
+                      if (!__any_sync(FULL, next < no)) break;
+                      take_overflow(ovf + slot * ovf_cap, no, next, warp * 32 * WPT, 32 * WPT,
+                                    lev + slot * (2 * SW) + SW);
+                      WVec<WPT>::ld(l1, m1);
+                      if (mine) {
+                        const uint32_t zero[WPT] = {};
+                        WVec<WPT>::st(l1, zero);
+                      }
 #pragma unroll
-                    for (int q = 0; q < WPT; q++) {
-                      m0[q] = 0;
-                      m1[q] = (bit >> 5) == w0 + q ? 1u << (bit & 31) : 0u;
+                      for (int q = 0; q < WPT; q++) {
+                        m0[q] = 0;
+                        m1[q] = mine ? m1[q] : 0;
+                      }
+                    }
+                  } else {
+                    const uint32_t no = 2 * min(oc[slot], ovf_cap);
+                    for (uint32_t t = 0;; t++) {
+                      count_sub(p, ac, m0, m1, am);
+                      if (t >= no) break;
+                      const uint32_t bit = ovf[slot * ovf_cap + (t >> 1)];
+#pragma unroll
+                      for (int q = 0; q < WPT; q++) {
+                        m0[q] = 0;
+                        m1[q] = (bit >> 5) == w0 + q ? 1u << (bit & 31) : 0u;
+                      }
                     }
                   }
                 } else {
@@ -821,7 +866,7 @@ __host__ __device__ constexpr SpecLayout spec_layout(uint32_t SW, uint32_t R, ui
 
 // misc: [0] unit, [8..39] live counts of a scan, [48..55] overflow counts
 // (2 parities x 4), [56..63] literal counts, [64..79] results (2 x 8)
-template <int SW, int R, int MINB>
+template <int SW, int R, int MINB, bool OV>
 __global__ void __launch_bounds__(SP_NT, MINB)
     k_train_spec(const TrainDev *__restrict__ machines, const WorkItem *__restrict__ work,
                  uint32_t nwork, uint32_t *__restrict__ counter, uint32_t e_begin, uint32_t e_end,
@@ -1118,15 +1163,30 @@ __global__ void __launch_bounds__(SP_NT, MINB)
                     WVec<2>::st(l0, zero);
                     WVec<2>::st(l1, zero);
                     // an overflow entry is worth 4: twice a level-1 count
-                    const uint32_t no = 2 * min(oc[slot], ovf_cap);
-                    for (uint32_t t = 0;; t++) {
-                      count_sub(p, ac, m0, m1, ma);
-                      if (t >= no) break;
-                      const uint32_t bit = ovf[slot * ovf_cap + (t >> 1)];
+                    if constexpr (OV) {
+                      const uint32_t no = min(oc[slot], ovf_cap);
+                      uint32_t next = lane;  // this lane's next entry
+                      for (uint32_t t = 0;; t++) {
+                        count_sub(p, ac, m0, m1, ma);
+                        if (t & 1u) continue;
+                        if (!__any_sync(FULL, next < no)) break;
+                        take_overflow(ovf + slot * ovf_cap, no, next, 64 * k, 64,
+                                      lev + slot * (2 * SW) + SW);
+                        WVec<2>::ld(l1, m1);
+                        WVec<2>::st(l1, zero);
+                        m0[0] = m0[1] = 0;
+                      }
+                    } else {
+                      const uint32_t no = 2 * min(oc[slot], ovf_cap);
+                      for (uint32_t t = 0;; t++) {
+                        count_sub(p, ac, m0, m1, ma);
+                        if (t >= no) break;
+                        const uint32_t bit = ovf[slot * ovf_cap + (t >> 1)];
 #pragma unroll
-                      for (int q = 0; q < 2; q++) {
-                        m0[q] = 0;
-                        m1[q] = (bit >> 5) == 64 * k + 2 * lane + q ? 1u << (bit & 31) : 0u;
+                        for (int q = 0; q < 2; q++) {
+                          m0[q] = 0;
+                          m1[q] = (bit >> 5) == 64 * k + 2 * lane + q ? 1u << (bit & 31) : 0u;
+                        }
                       }
                     }
                   } else {
@@ -1233,6 +1293,12 @@ static_assert(wpt_in_order(), "a configuration's place is its id");
 
 static uint32_t wpt_ovf_cap(uint32_t smax) { return smax / 4 > 0 ? smax / 4 : 1; }
 
+double wpt_overflow(uint32_t bits, uint32_t picks) {
+  if (!bits) return 0.0;
+  const double l = (double)picks / bits;
+  return bits * (1.0 - exp(-l) * (1.0 + l + l * l / 2 + l * l * l / 6));
+}
+
 static size_t wpt_bytes(const WptConfig &k, uint32_t smax) {
   const uint32_t oc = wpt_ovf_cap(smax);
   return k.ring ? spec_layout(k.sw, k.ring, oc).total
@@ -1247,24 +1313,29 @@ static int wpt_occ(F kernel, int threads, size_t bytes) {
   return nb;
 }
 
-// Resident CTAs (units) per SM of configuration `id` for rows of at most
-// Wpmax words (0 when it cannot hold them), and its shared memory.
-int train_wpt_occupancy(int id, uint32_t Wpmax, uint32_t smax, size_t *smem_bytes) {
-  if (id < 1 || id > kWptCount) return 0;
-  const WptConfig &k = kWpt[id - 1];
-  if (Wpmax > (uint32_t)k.sw) return 0;
-  const size_t bytes = wpt_bytes(k, smax);
-  *smem_bytes = bytes;
+template <bool OV>
+static int config_occ(int id, size_t bytes) {
   switch (id) {
 #define TM_W(ID, NT, WPT, SW, RP, GP, IBS, MINB) \
-  case ID: return wpt_occ(k_train_wpt<NT, WPT, SW, RP, GP, IBS, MINB>, NT, bytes);
+  case ID: return wpt_occ(k_train_wpt<NT, WPT, SW, RP, GP, IBS, MINB, OV>, NT, bytes);
 #define TM_S(ID, SW, R, MINB) \
-  case ID: return wpt_occ(k_train_spec<SW, R, MINB>, SP_NT, bytes);
+  case ID: return wpt_occ(k_train_spec<SW, R, MINB, OV>, SP_NT, bytes);
     TM_WPT_CONFIGS(TM_W, TM_S)
 #undef TM_W
 #undef TM_S
   }
   return 0;
+}
+
+// Resident CTAs (units) per SM of configuration `id` for rows of at most
+// Wpmax words (0 when it cannot hold them), and its shared memory.
+int train_wpt_occupancy(int id, uint32_t Wpmax, uint32_t smax, bool many_ovf, size_t *smem_bytes) {
+  if (id < 1 || id > kWptCount) return 0;
+  const WptConfig &k = kWpt[id - 1];
+  if (Wpmax > (uint32_t)k.sw) return 0;
+  const size_t bytes = wpt_bytes(k, smax);
+  *smem_bytes = bytes;
+  return many_ovf ? config_occ<true>(id, bytes) : config_occ<false>(id, bytes);
 }
 
 // The configurations worth a launch of `units` units on `sms` SMs, rows of at
@@ -1294,28 +1365,37 @@ int wpt_choices(uint32_t Wpmax, uint32_t smax, uint32_t units, int sms, int opti
   return n;
 }
 
-cudaError_t launch_train_wpt(int id, const TrainDev *machines, const WorkItem *work,
-                             uint32_t nwork, uint32_t *counter, uint32_t e_begin, uint32_t e_end,
-                             uint32_t Wpmax, uint32_t smax, int grid, uint32_t *err,
-                             cudaStream_t st) {
-  if (id < 1 || id > kWptCount || Wpmax > (uint32_t)kWpt[id - 1].sw) return cudaErrorInvalidValue;
-  const size_t bytes = wpt_bytes(kWpt[id - 1], smax);
-  const uint32_t oc = wpt_ovf_cap(smax);
+template <bool OV>
+static void config_launch(int id, int grid, size_t bytes, cudaStream_t st,
+                          const TrainDev *machines, const WorkItem *work, uint32_t nwork,
+                          uint32_t *counter, uint32_t e_begin, uint32_t e_end, uint32_t ovf_cap,
+                          uint32_t *err) {
   switch (id) {
 #define TM_W(ID, NT, WPT, SW, RP, GP, IBS, MINB)                                 \
   case ID:                                                                       \
-    k_train_wpt<NT, WPT, SW, RP, GP, IBS, MINB><<<grid, NT, bytes, st>>>(        \
-        machines, work, nwork, counter, e_begin, e_end, oc, err);                \
+    k_train_wpt<NT, WPT, SW, RP, GP, IBS, MINB, OV><<<grid, NT, bytes, st>>>(    \
+        machines, work, nwork, counter, e_begin, e_end, ovf_cap, err);           \
     break;
 #define TM_S(ID, SW, R, MINB)                                                    \
   case ID:                                                                       \
-    k_train_spec<SW, R, MINB><<<grid, SP_NT, bytes, st>>>(                       \
-        machines, work, nwork, counter, e_begin, e_end, oc, err);                \
+    k_train_spec<SW, R, MINB, OV><<<grid, SP_NT, bytes, st>>>(                   \
+        machines, work, nwork, counter, e_begin, e_end, ovf_cap, err);           \
     break;
     TM_WPT_CONFIGS(TM_W, TM_S)
 #undef TM_W
 #undef TM_S
   }
+}
+
+cudaError_t launch_train_wpt(int id, const TrainDev *machines, const WorkItem *work,
+                             uint32_t nwork, uint32_t *counter, uint32_t e_begin, uint32_t e_end,
+                             uint32_t Wpmax, uint32_t smax, bool many_ovf, int grid, uint32_t *err,
+                             cudaStream_t st) {
+  if (id < 1 || id > kWptCount || Wpmax > (uint32_t)kWpt[id - 1].sw) return cudaErrorInvalidValue;
+  const size_t bytes = wpt_bytes(kWpt[id - 1], smax);
+  (many_ovf ? config_launch<true> : config_launch<false>)(id, grid, bytes, st, machines, work, nwork,
+                                                          counter, e_begin, e_end,
+                                                          wpt_ovf_cap(smax), err);
   return cudaGetLastError();
 }
 
