@@ -849,9 +849,14 @@ static bool lookup_tuned(const TrainShape &sh, const tm_machine *m0, TrainPlan &
   return plan_mode(v.first, sh, out, v.second);
 }
 
-// The plans of the kernels of tm_train_wpt.cu that are worth this launch, best
-// guess first: 8-bit units of rows up to 1,024 words, where they beat every
-// other variant at each width measured (4 to 1,024 words, 40 to 93,000 units).
+// The plans that are worth a launch of 8-bit units with rows up to 1,024 words,
+// best guess first (none for other launches): those of tm_train_wpt.cu, and for
+// rows above 256 words with two SMs for every unit the 2-CTA cluster, which
+// shares a unit's words between them (20 units of 500 words at specificity 4:
+// 2.07 ms against 2.33).  The best of them is as fast as the best of all variants
+// that the tuner used to try, or faster, on rows of 4 to 1,024 words, 20 to
+// 93,000 units and specificities 1.2 to 25, but for 188-word rows at specificity
+// 2 and two units per SM (36.3 against 34.9 ms).
 static std::vector<TrainPlan> wpt_plans(const TrainShape &sh) {
   std::vector<TrainPlan> plans;
   if (sh.Bmin != 8 || sh.Bmax != 8) return plans;
@@ -861,6 +866,10 @@ static std::vector<TrainPlan> wpt_plans(const TrainShape &sh) {
     TrainPlan p;
     if (plan_mode(TM_MODE_WPT, sh, p, ids[i])) plans.push_back(p);
   }
+  TrainPlan p;
+  if (!plans.empty() && sh.Wpmax > 256 && 2 * sh.units <= (uint32_t)sh.sms &&
+      plan_mode(TM_MODE_PAIR, sh, p))
+    plans.push_back(p);
   return plans;
 }
 

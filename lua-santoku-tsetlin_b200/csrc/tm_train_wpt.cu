@@ -1343,25 +1343,37 @@ int train_wpt_occupancy(int id, uint32_t Wpmax, uint32_t smax, bool many_ovf, si
 //   k_train_wpt with the smallest row slot that holds the rows: smaller slots
 //     hold more units per SM (rows of 49 words: 26.2 ms in 56-word slots,
 //     27.5 ms in 64-word ones).
-//   k_train_spec up to 6 units per SM and 256 words: with few units the chain
-//     of one unit's samples is what takes the time (plain classifier, 320
-//     units: 2.8 ms against 6.6 ms), with many the evaluations it throws away
-//     (search rows, 15,000 units: 67.8 against 25.7 ms).
+//   Up to 6 units per SM also:
+//   k_train_spec for rows up to 256 words: with few units the chain of one
+//     unit's samples is what takes the time (plain classifier, 320 units: 2.8 ms
+//     against 6.6 ms), with many the evaluations it throws away (search rows,
+//     15,000 units: 67.8 against 25.7 ms).
+//   k_train_wpt with the next larger slot, whose units have twice the threads to
+//     scan and to draw with (four words per thread, so for rows above 64 words:
+//     encoder rows of 94 words, specificity 4, 800 units 35.3 ms with the two
+//     choices above, 26.4 ms in 256-word slots; 4,800 units 18.2 against 24.5 ms
+//     at specificity 5).
 int wpt_choices(uint32_t Wpmax, uint32_t smax, uint32_t units, int sms, int optin, int *ids,
                 int max) {
-  int n = 0;
-  for (int spec = 0; spec < 2; spec++) {
-    if (spec && units > 6u * (uint32_t)sms) break;
+  auto smallest = [&](bool spec, int threads) {
     int best = 0;
     for (int id = 1; id <= kWptCount; id++) {
       const WptConfig &k = kWpt[id - 1];
-      if ((k.ring != 0) != (spec != 0) || Wpmax > (uint32_t)k.sw) continue;
+      if ((k.ring != 0) != spec || k.nt < threads || Wpmax > (uint32_t)k.sw) continue;
       if (wpt_bytes(k, smax) > (size_t)optin) continue;
       if (best && kWpt[best - 1].sw <= k.sw) continue;
       best = id;
     }
-    if (best && n < max) ids[n++] = best;
+    return best;
+  };
+  const int first = smallest(false, 0);
+  int pick[3] = {first, 0, 0}, n = 0;
+  if (units <= 6u * (uint32_t)sms) {
+    pick[1] = smallest(true, 0);
+    if (first && Wpmax > 64) pick[2] = smallest(false, kWpt[first - 1].nt + 1);
   }
+  for (int id : pick)
+    if (id && n < max) ids[n++] = id;
   return n;
 }
 

@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 
 SHAPES = [
     (10, 784, 760),    # 950 units: one choice
-    (3, 16384, 16),    # rows above 256 words: one choice
+    (10, 16384, 64),   # 1,024 words: one choice
     (10, 784, 64),     # 80 units: two choices, timed
 ]
 IDS = ["units950", "words1024", "units80"]
@@ -72,3 +72,21 @@ def test_batch_epochs_keep_the_kernel(tm, shape):
         once.train(dict(inp, iterations=i + 1))
         for a, b in zip(m.export_state(), once.export_state()):
             assert np.array_equal(a, b)
+
+
+def test_few_units_get_more_threads_where_that_is_faster(tm):
+    """800 units of 94-word rows, 5.4 per SM: two warps per unit (configuration 4)
+    take 0.75 of the time of one (10) or of eight samples at once (9)."""
+    rng = np.random.default_rng(2)
+    n, hidden, visible = 2000, 10, 1500
+    b = rng.random((n, visible)) < 0.2
+    x = np.packbits(np.concatenate([b, ~b], axis=1), axis=1, bitorder="little").ravel()
+    t = tm.create("encoder", dict(hidden=hidden, visible=visible, clauses=640, clause_tolerance=64,
+                                  clause_maximum=64, specificity=4.0, target=30, reusable=True,
+                                  seed=3))
+    t.set_autotune(2)
+    t.stats_enable(True)
+    t.train(dict(samples=n, sentences=x, codes=rng.integers(0, 256, size=2 * n).astype(np.uint8),
+                 iterations=1))
+    st = t.stats()
+    assert (st["train_mode"], st["train_cpw"], st["train_autotuned"]) == (4, 4, 1)
