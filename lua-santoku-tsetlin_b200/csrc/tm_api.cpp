@@ -45,6 +45,14 @@ static int fail(int code, const char *fmt, ...) {
                   "%s failed: %s", #call, cudaGetErrorString(e_));                    \
   } while (0)
 
+// Whether an allocation of memory that the caller can do without failed for want
+// of it (the error is cleared then).
+static bool no_memory(cudaError_t e) {
+  if (e != cudaErrorMemoryAllocation) return false;
+  cudaGetLastError();
+  return true;
+}
+
 // Every device allocation of the library goes through here.  A failure
 // injected by tm_debug_fail_alloc makes the chosen allocation report
 // cudaErrorMemoryAllocation without calling cudaMalloc, so the error paths
@@ -2455,8 +2463,25 @@ extern "C" int tm_predict_scores(tm_machine *m, const uint8_t *problems, const i
 // before it end, so the range is one contiguous byte slice of the full
 // layout.  Dense rows without padding are copied as they are; others are
 // packed or unpacked on the device, host buffers in blocks of classes of at
-// most TM_STATE_BLOCK bytes (or one class).
+// most TM_STATE_BLOCK bytes (or one class), or without the memory for that
+// copied row by row.
 constexpr uint64_t TM_STATE_BLOCK = 128ull << 20;
+
+static int copy_strided(tm_machine *m, uint32_t lo, uint32_t hi, bool to_buf, uint8_t *buf,
+                        bool counts, bool on_device) {
+  const cudaMemcpyKind kind = on_device ? cudaMemcpyDeviceToDevice
+                                        : (to_buf ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice);
+  const uint64_t rows = (uint64_t)m->clauses * (counts ? m->B - 1 : 1);
+  for (uint32_t h = lo; h < hi; h++) {
+    const ClassDev &c = m->cls[h];
+    uint32_t *dev = counts ? m->d_cnt + c.cnt_off : m->d_act + c.act_off;
+    const size_t width = m->n_chunks[h], pitch = (size_t)c.Wp * 4;
+    if (to_buf) CK(cudaMemcpy2DAsync(buf, width, dev, pitch, width, rows, kind, m->st));
+    else CK(cudaMemcpy2DAsync(dev, pitch, buf, width, width, rows, kind, m->st));
+    buf += rows * width;
+  }
+  return TM_OK;
+}
 
 static int copy_classes(tm_machine *m, uint32_t lo, uint32_t hi, bool to_buf, uint8_t *buf,
                         bool counts, bool on_device) {
@@ -2489,7 +2514,15 @@ static int copy_classes(tm_machine *m, uint32_t lo, uint32_t hi, bool to_buf, ui
     }
     const uint64_t ob = ((uint64_t)(h1 - h) * 8 + 255) & ~255ull;
     PoolBuf tmp;
-    CK(tmp.ensure(ob + (on_device ? 0 : bytes), m->st));
+    const cudaError_t te = tmp.ensure(ob + (on_device ? 0 : bytes), m->st);
+    if (no_memory(te)) {
+      int rc = copy_strided(m, h, h1, to_buf, buf + at, counts, on_device);
+      if (rc) return rc;
+      at += bytes;
+      h = h1;
+      continue;
+    }
+    CK(te);
     uint8_t *dbytes = on_device ? buf + at : tmp.as<uint8_t>() + ob;
     // (offs is pageable: the copy has read it when the call returns)
     cudaError_t e = cudaMemcpyAsync(tmp.p, offs.data(), (uint64_t)(h1 - h) * 8,
