@@ -2166,7 +2166,8 @@ static bool votes_path(tm_machine *m, uint64_t n) {
 }
 
 // Whether a large predict of n samples reads literal lists (made here, once
-// per state of the automata): where the action and sample words, 16 bytes each
+// per state of the automata; without the memory for them, not in this state):
+// where the action and sample words, 16 bytes each
 // for the tensor cores, exceed L2 (20 classes x 2,048 clauses of 32,768
 // literals, 40 samples 189 -> 53 us), and from 2^32 tests on (2^31: 60 us
 // either way).
@@ -2183,7 +2184,12 @@ static int ensure_lists(tm_machine *m, uint64_t n, bool *use) {
   if (!tw || ((M + n) * c0.W < (1ull << 23) && M * n * c0.W < (1ull << 32))) return TM_OK;
   if (!m->list_state) {
     const uint64_t ng = (uint64_t)m->classes * ((m->clauses + 31) / 32);
-    CK(m->list_groups.ensure(ng * 8 + 8, m->st));
+    cudaError_t e = m->list_groups.ensure(ng * 8 + 8, m->st);
+    if (no_memory(e)) {
+      m->list_state = 2;
+      return TM_OK;
+    }
+    CK(e);
     uint8_t *gp = m->list_groups.as<uint8_t>();
     uint32_t tot[2];
     CK(cudaMemsetAsync(gp + ng * 8, 0, 8, m->st));
@@ -2195,7 +2201,9 @@ static int ensure_lists(tm_machine *m, uint64_t n, bool *use) {
     const uint64_t ratio = tw == 4 ? 32 : (tw == 2 ? 40 : 56);
     m->list_state = 2;
     if (tot[1] <= TM_LIST_NEED && tot[0] * 16ull * ratio <= ng * c0.W * 32) {
-      CK(m->lists.ensure(((uint64_t)tot[0] + 1) * TM_LIST_BLOCK, m->st));
+      e = m->lists.ensure(((uint64_t)tot[0] + 1) * TM_LIST_BLOCK, m->st);
+      if (no_memory(e)) return TM_OK;
+      CK(e);
       CK(launch_list_fill(m->d_act, m->classes, m->clauses, c0, gp, m->lists.p, m->st));
       note_launch(m, 1);
       m->list_state = 1;
@@ -2203,6 +2211,11 @@ static int ensure_lists(tm_machine *m, uint64_t n, bool *use) {
   }
   *use = m->list_state == 1;
   return TM_OK;
+}
+
+// device room for the classes, codes and scores of n samples
+static uint64_t predict_out_bytes(const tm_machine *m, uint64_t n) {
+  return n * 8 + n * m->class_chunks + n * m->classes * 8 + 64;
 }
 
 // Whether a predict of few samples reads literal lists instead of every action
@@ -2219,12 +2232,21 @@ static int few_lists(tm_machine *m, uint64_t n, bool *use) {
     return TM_OK;
   if (!m->list_state && m->few_calls++ == 0) return TM_OK;
   int rc = ensure_lits(m);
-  return rc ? rc : ensure_lists(m, n, use);
+  if (!rc) rc = ensure_lists(m, n, use);
+  if (rc || !*use) return rc;
+  // all that the lists need beyond k_predict_few, which serves the call without it
+  cudaError_t e = m->x4.ensure(list_slice_bytes(m->cls[0].W, n), m->st);
+  if (e == cudaSuccess) e = m->sums.ensure(n * m->classes * 4);
+  if (e == cudaSuccess) e = m->raw.ensure(n * m->n_chunks[0]);
+  if (e == cudaSuccess) e = m->outc.ensure(predict_out_bytes(m, n));
+  *use = !no_memory(e);
+  if (*use) CK(e);
+  return TM_OK;
 }
 
 // The vote sums of n byte rows through literal lists (*lists set) or k_votes
-// (m->sums, cleared here); 1 when its status word cannot be had (nothing was
-// queued).
+// (m->sums, cleared here).  Without sums queued: 1 when the status word of
+// k_votes cannot be had, 2 when the memory of either cannot (*lists not set).
 static int predict_votes(tm_machine *m, const uint8_t *rows, uint64_t n, bool on_device,
                          bool *lists) {
   const ClassDev &c0 = m->cls[0];
@@ -2247,7 +2269,12 @@ static int predict_votes(tm_machine *m, const uint8_t *rows, uint64_t n, bool on
     // samples per launch: at most 512 MB of slices and 2^20 samples
     const uint64_t nc = std::min<uint64_t>(
         1 << 20, std::max<uint64_t>(128, (512ull << 20) / (c0.W * 4ull + 1) / 128 * 128));
-    CK(m->x4.ensure(list_slice_bytes(c0.W, std::min<uint64_t>(nc, n)), m->st));
+    const cudaError_t e = m->x4.ensure(list_slice_bytes(c0.W, std::min<uint64_t>(nc, n)), m->st);
+    if (no_memory(e)) {
+      *lists = false;
+      return 2;
+    }
+    CK(e);
     v.slices = m->x4.as<uint32_t>();
     for (uint64_t s0 = 0; s0 < n; s0 += nc) {
       v.rows = rows + s0 * nch;
@@ -2260,17 +2287,22 @@ static int predict_votes(tm_machine *m, const uint8_t *rows, uint64_t n, bool on
   }
   uint32_t *status = (uint32_t *)(m->pin + TM_PIN_STAGE + TM_PIN_OUT);
   *status = 0;
+  // samples per launch: at most 512 MB of operand, whole tiles of 256
+  const uint64_t nc = std::max<uint64_t>(256, ((512ull << 20) / K) / 256 * 256);
+  cudaError_t e = m->act4_valid ? cudaSuccess : m->act4.ensure(M * K, m->st);
+  if (e == cudaSuccess) e = m->x4.ensure(std::min<uint64_t>(nc, n) * K, m->st);
+  if (no_memory(e)) {
+    if (!m->act4_valid) m->act4.release(m->st);
+    return 2;
+  }
+  CK(e);
   if (!m->act4_valid) {
-    CK(m->act4.ensure(M * K, m->st));
     // dense machines: the classes' clause rows follow each other
     CK(launch_expand_fp4(m->d_act + c0.act_off, M, c0.Wp, c0.W, c0.emask, m->act4.as<uint8_t>(),
                          m->st));
     note_launch(m, 1);
     m->act4_valid = true;
   }
-  // samples per launch: at most 512 MB of operand, whole tiles of 256
-  const uint64_t nc = std::max<uint64_t>(256, ((512ull << 20) / K) / 256 * 256);
-  CK(m->x4.ensure(std::min<uint64_t>(nc, n) * K, m->st));
   for (uint64_t s0 = 0; s0 < n; s0 += nc) {
     const uint64_t k = std::min<uint64_t>(nc, n - s0);
     int32_t *sums = m->sums.as<int32_t>() + s0 * m->classes;
@@ -2309,8 +2341,9 @@ static int predict_common(tm_machine *m, const uint8_t *problems, const int64_t 
   bool votes = lists || votes_path(m, n);
   int gr = votes ? predict_votes(m, problems, n, on_device, &lists) : 1;
   if (gr < 0) return gr;
+  const bool refused = gr == 2;  // for want of memory: the bitwise tiles, which need little
   votes = gr == 0;
-  if (gr == 1) {
+  if (gr >= 1) {
     // the repack launch also clears the vote sums
     rc = stage_rows(m, m->x, problems, dim_offsets, n, on_device, cls, m->sums.as<uint32_t>(),
                     sb / 4);
@@ -2322,7 +2355,7 @@ static int predict_common(tm_machine *m, const uint8_t *problems, const int64_t 
       if (rc) return rc;
     }
     if (m->timing) CK(cudaEventRecord(m->ev0, m->st));  // the evaluation alone
-    gr = gemm_wanted(m, n) ? predict_gemm(m, n) : 1;
+    gr = !refused && gemm_wanted(m, n) ? predict_gemm(m, n) : 1;
     if (gr < 0) return gr;
   }
   m->stats.predict_gemm = gr || lists ? 0 : (votes ? TM_GEMM_FP8 : m->act8_kind);
@@ -2342,7 +2375,7 @@ static int predict_common(tm_machine *m, const uint8_t *problems, const int64_t 
     dcod = out_codes;
     dsc = out_scores;
   } else {
-    CK(m->outc.ensure(clsb + codb + scb + 64));
+    CK(m->outc.ensure(predict_out_bytes(m, n)));
     uint8_t *p = m->outc.as<uint8_t>();
     if (out_classes) dcls = (int64_t *)p;
     if (out_codes) dcod = p + clsb;

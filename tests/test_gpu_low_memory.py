@@ -56,3 +56,64 @@ def test_state_copies_without_staging(tm, ind):
         assert ind or torch.equal(mine, part)
         assert all(np.array_equal(a, c) for a, c in zip(u.export_state(), want))
         u.destroy()
+
+
+def _clauses_of(tm, classes, features, clauses, literals, seed):
+    """A machine whose clauses include `literals` literals each, and byte rows."""
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(seed)
+    t = tm.create("classifier", dict(classes=classes, features=features, clauses=clauses,
+                                     clause_tolerance=20, clause_maximum=64, specificity=9.0,
+                                     reusable=False))
+    t.stats_enable(True)
+    ab, sb = t.class_bytes(0, classes)
+    acts = torch.zeros(classes * clauses, ab // (classes * clauses) * 8, dtype=torch.bool,
+                       device="cuda")
+    at = torch.randint(0, 2 * features, (classes * clauses, literals), generator=g, device="cuda")
+    acts.scatter_(1, at, True)
+    w = 1 << torch.arange(8, device="cuda", dtype=torch.int32)
+    buf = torch.zeros(ab + sb, dtype=torch.uint8, device="cuda")
+    buf[:ab] = (acts.view(classes * clauses, -1, 8).int() * w).sum(2).to(torch.uint8).reshape(-1)
+    x = torch.randint(0, 256, (400, features // 4), generator=g, device="cuda", dtype=torch.uint8)
+    x |= torch.randint(0, 256, x.shape, generator=g, device="cuda", dtype=torch.uint8)
+    torch.cuda.synchronize()
+
+    def fresh():  # a new state of the same automata: nothing derived is left
+        t.import_classes(0, classes, buf)
+    return t, x.cpu().numpy(), fresh
+
+
+@pytest.mark.parametrize("n,literals", [(8, 20), (400, 20), (400, 700)],
+                         ids=["few", "lists", "tensor"])
+def test_predict_without_its_copies_of_the_actions(tm, n, literals):
+    """Literal lists, the samples' slices, the 4-bit copies of actions and samples:
+    a predict that cannot have them returns the same sums another way, and the
+    next state uses them again."""
+    t, x, fresh = _clauses_of(tm, 8, 8192, 4096, literals, n + literals)
+    x = x[:n].ravel()
+    fresh()
+    want = t.predict_scores(x, n)
+    want = t.predict_scores(x, n)  # (small requests: lists from the second on)
+    t.destroy()
+    refused = 0
+    for k in range(12):
+        t, _, fresh = _clauses_of(tm, 8, 8192, 4096, literals, n + literals)
+        fresh()
+        if n <= 32:
+            assert np.array_equal(t.predict_scores(x, n), want)
+        _fails_at(tm, k)
+        try:
+            got = t.predict_scores(x, n)
+        except tm.TsetlinError as e:
+            # host rows, vote sums and outputs: nothing else may be needed
+            assert n > 32 and "memory" in str(e).lower()
+            assert any(w in str(e) for w in ("sums", "raw", "outc", "m->x")), str(e)
+            refused += 1
+        else:
+            assert np.array_equal(got, want), k
+        finally:
+            _fails_at(tm, -1)
+        assert np.array_equal(t.predict_scores(x, n), want), k
+        t.destroy()
+    assert refused <= 4
