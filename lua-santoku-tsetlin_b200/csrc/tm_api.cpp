@@ -1539,7 +1539,8 @@ static int search_round(tm_machine *const *ms, const tm_train_args *args, uint32
   // ---- the holdout predict of large dense machines as k_votes ---------------
   // Their holdout rows are expanded to 4-bit floats once; in every epoch the
   // graph expands the trained actions and runs the vote kernel (gated by the
-  // machine's live flag, like the bitwise predict).
+  // machine's live flag, like the bitwise predict).  A machine whose copies
+  // find no memory keeps the bitwise predict.
   std::vector<char> use_votes(count, 0);
   std::vector<const uint8_t *> vx4(count, nullptr);
   if (!m0->sms) m0->sms = num_sms(m0->device);
@@ -1555,23 +1556,27 @@ static int search_round(tm_machine *const *ms, const tm_train_args *args, uint32
       // beside the launch of all small machines' tiles, a machine's own two
       // launches pay from more work on than in a predict of its own
       if (!votes_path(m, nt) || M * nt * c0.W < (1ull << 27) || nt * K > (2ull << 30)) continue;
-      use_votes[i] = 1;
-      amax = std::max<uint64_t>(amax, M * K);
       const void *src = sa->test_each && sa->test_each[i] ? (const void *)sa->test_each[i]
                                                           : (const void *)sa->test_problems;
       const auto key = std::make_tuple(src, (uint64_t)m->features, c0.Wp, c0.W);
       auto it = x4_of.find(key);
       if (it == x4_of.end()) {
         const size_t at = x4_of.size();
-        it = x4_of.emplace(key, at).first;
         if (m0->search_x4.size() <= at) m0->search_x4.resize(at + 1);
-        CK(m0->search_x4[at].ensure(nt * K));
+        const cudaError_t e = m0->search_x4[at].ensure(nt * K);
+        if (no_memory(e)) continue;
+        CK(e);
+        it = x4_of.emplace(key, at).first;
         CK(launch_expand_fp4(m->x.as<uint32_t>(), nt, c0.Wp, c0.W, 0xFFFFFFFFu,
                              m0->search_x4[at].as<uint8_t>(), st));
       }
       vx4[i] = m0->search_x4[it->second].as<uint8_t>();
+      use_votes[i] = 1;
+      amax = std::max<uint64_t>(amax, M * K);
     }
-    if (amax) CK(m0->search_act4.ensure(amax));
+    const cudaError_t e = amax ? m0->search_act4.ensure(amax) : cudaSuccess;
+    if (no_memory(e)) use_votes.assign(count, 0);
+    else CK(e);
   }
   // machine i's vote sums of the holdout, added to its (cleared) sums unless
   // *gate is 0

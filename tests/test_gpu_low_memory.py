@@ -117,3 +117,44 @@ def test_predict_without_its_copies_of_the_actions(tm, n, literals):
         assert np.array_equal(t.predict_scores(x, n), want), k
         t.destroy()
     assert refused <= 4
+
+
+def test_search_round_without_its_holdout_copies(tm):
+    """The holdout of a large machine as 4-bit floats, and its actions: without them
+    the round scores it with the bitwise kernel, to the same scores."""
+    rng = np.random.default_rng(3)
+    n, nt, classes, features = 200, 1200, 8, 2000
+    b = rng.random((n + nt, features)) < 0.1
+    y = (b[:, 0].astype(np.int64) + 2 * b[:, 7] + 4 * b[:, 11]) % classes
+    x = np.packbits(np.concatenate([b, ~b], axis=1), axis=1, bitorder="little")
+    tbl = dict(classes=classes, features=features, clauses=256, clause_tolerance=20,
+               clause_maximum=40, specificity=9.0, target=30, reusable=True, seed=4)
+
+    def run(k):
+        t = tm.create("classifier", tbl)  # 2.5e8 tests of the holdout
+        t.stats_enable(True)
+        _fails_at(tm, k)
+        try:
+            r = tm.train_batch_search(
+                [t], [dict(samples=n, problems=x[:n].ravel(), solutions=y[:n], iterations=2)],
+                dict(samples=nt, problems=x[n:].ravel(), solutions=y[n:]))
+        except tm.TsetlinError as e:
+            assert "memory" in str(e).lower()
+            return str(e)
+        finally:
+            _fails_at(tm, -1)
+        launches = t.stats()["kernel_launches"]
+        t.destroy()
+        return [np.asarray(r["scores"]), np.asarray(r["best"])], launches
+
+    run(-1)  # the tuner times its choices once
+    want, usual = run(-1)
+    fewer = 0
+    for k in range(24):
+        got = run(k)
+        if isinstance(got, str):
+            assert "search_x4" not in got and "search_act4" not in got, got
+            continue
+        assert all(np.array_equal(a, c) for a, c in zip(got[0], want)), k
+        fewer += got[1] < usual
+    assert fewer == 2  # the bitwise kernel is one launch an epoch, not two
