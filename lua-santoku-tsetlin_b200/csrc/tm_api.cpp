@@ -1167,7 +1167,7 @@ static int choose_plan(std::vector<TrainJob> &jobs, const std::vector<TrainDev> 
 }
 
 // Queues epoch orders on the owner's stream, with scratch for the large ones:
-// as many at a time as fit 256 MB.
+// as many at a time as fit 256 MB, or without that much memory one.
 static int queue_orders(tm_machine *m0, std::vector<OrderJob> &orders, const uint32_t *epoch_dev,
                         uint64_t *launches) {
   size_t one = 0, all = 0;
@@ -1177,7 +1177,9 @@ static int queue_orders(tm_machine *m0, std::vector<OrderJob> &orders, const uin
     all += b;
   }
   const size_t want = std::max(one, std::min<size_t>(all, 256u << 20));
-  if (want) CK(m0->perm_scratch.ensure(want));
+  cudaError_t e = want ? m0->perm_scratch.ensure(want) : cudaSuccess;
+  if (want > one && no_memory(e)) e = one ? m0->perm_scratch.ensure(one) : cudaSuccess;
+  CK(e);
   CK(launch_orders(orders.data(), orders.size(), m0->perm_scratch.p, m0->perm_scratch.cap, m0->st,
                    epoch_dev, launches));
   return TM_OK;

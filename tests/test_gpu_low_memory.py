@@ -158,3 +158,31 @@ def test_search_round_without_its_holdout_copies(tm):
         assert all(np.array_equal(a, c) for a, c in zip(got[0], want)), k
         fewer += got[1] < usual
     assert fewer == 2  # the bitwise kernel is one launch an epoch, not two
+
+
+def test_orders_one_after_another(tm):
+    """Scratch for several large epoch orders at once (20,000 samples, three epochs):
+    with room for one they run in turn."""
+    rng = np.random.default_rng(6)
+    n = 20000
+    b = rng.random((n, 20)) < 0.4
+    x = np.packbits(np.concatenate([b, ~b], axis=1), axis=1, bitorder="little").ravel()
+    tbl = dict(classes=2, features=20, clauses=8, clause_tolerance=6, clause_maximum=9,
+               specificity=4.0, target=7, reusable=True, seed=1)
+    inp = dict(samples=n, problems=x, solutions=(b[:, 0] ^ b[:, 3]).astype(np.int64), iterations=3)
+    t = tm.create("classifier", tbl)
+    t.train(inp)
+    want = t.export_state()
+    t.destroy()
+    for k in range(12):
+        t = tm.create("classifier", tbl)
+        _fails_at(tm, k)
+        try:
+            t.train(inp)
+        except tm.TsetlinError as e:
+            assert "memory" in str(e).lower() and "perm_scratch" not in str(e), str(e)
+        else:
+            assert all(np.array_equal(a, c) for a, c in zip(t.export_state(), want)), k
+        finally:
+            _fails_at(tm, -1)
+        t.destroy()
