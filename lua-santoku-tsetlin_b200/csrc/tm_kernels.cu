@@ -170,7 +170,7 @@ cudaError_t launch_setup(uint32_t *act, uint32_t *cnt, const ClassDev *cls, uint
 // about n / 4 buckets leaves a handful of samples per bucket, which one thread
 // sorts by (key, index).  All orders of a call -- epochs of one machine,
 // machines of a search round -- go into the same launches: one for orders of
-// up to ORDER_SMALL samples (a CTA per order, all in shared memory), four for
+// up to ORDER_SMALL samples (a CTA per order, all in shared memory), five for
 // larger ones.  Bound by launch latency and Philox.  Ten epochs of 8,000
 // samples: 110 launches (a library radix sort per order) -> one; sixteen
 // orders of 6,000 samples in a search epoch: 1.4 ms -> 0.02 ms.
@@ -186,11 +186,16 @@ __device__ __forceinline__ uint64_t order_key(const OrderJob &J, uint32_t epoch,
   philox(i, epoch, 0u, ST_PERM, J.seed, o);
   return ((uint64_t)o[0] << 32) | o[1];
 }
-// buckets: a power of two near n / 4 (at least 32, at most 2^24)
+// buckets: a power of two near n / 4 (at least 32)
 __host__ __device__ __forceinline__ uint32_t order_bits(uint32_t n) {
   uint32_t b = 5;
-  while (b < 24 && (4ull << b) < n) b++;
+  while ((4ull << b) < n) b++;
   return b;
+}
+// buckets of one CTA in the scan of a large order: at most ORDER_CHUNKS parts
+constexpr uint32_t ORDER_CHUNKS = 1024;
+__host__ __device__ __forceinline__ uint32_t order_chunk(uint32_t nb) {
+  return nb / ORDER_CHUNKS > 4096 ? nb / ORDER_CHUNKS : 4096;
 }
 
 // keys / idx [lo, hi) of one bucket, sorted by (key, index): insertion for
@@ -267,39 +272,106 @@ __global__ void __launch_bounds__(1024) k_order_small(const __grid_constant__ Or
 }
 
 // Orders above ORDER_SMALL (grid.y = order): counts, their scan, placement and
-// the buckets' sort, in global scratch (keys, then counters; indices in place)
+// the buckets' sort, in global scratch (entries, then counters)
 __global__ void k_order_count(const __grid_constant__ OrderBatch B, const uint32_t *epoch_dev) {
   const OrderJob &J = B.job[blockIdx.y];
   const uint32_t shift = 64 - order_bits(J.n), epoch = J.epoch + (epoch_dev ? *epoch_dev : 0u);
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < J.n; i += gridDim.x * blockDim.x)
     atomicAdd(&J.cnt[order_key(J, epoch, i) >> shift], 1u);
 }
-__global__ void __launch_bounds__(1024) k_order_scan(const __grid_constant__ OrderBatch B) {
-  const OrderJob &J = B.job[blockIdx.x];
-  scan_buckets(J.cnt, 1u << order_bits(J.n));
+// sum of `v` over a CTA of 1,024 threads, and before this thread
+__device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t &before) {
+  __shared__ uint32_t part[32];
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t inc = v;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, inc, d);
+    if (lane >= (uint32_t)d) inc += t;
+  }
+  if (lane == 31) part[warp] = inc;
+  __syncthreads();
+  const uint32_t p = part[lane];
+  before = __reduce_add_sync(0xFFFFFFFFu, lane < warp ? p : 0u) + inc - v;
+  const uint32_t all = __reduce_add_sync(0xFFFFFFFFu, p);
+  __syncthreads();
+  return all;
 }
-__global__ void k_order_place(const __grid_constant__ OrderBatch B, const uint32_t *epoch_dev) {
+// The exclusive scan of the counters, a CTA per chunk of them: each chunk's sum
+// (behind the counters), then every CTA adds up the sums before its own and
+// scans its chunk, 16 bytes per thread at a time.  Bound by memory.  (Orders of
+// 2^20, 2^23 and 2^25 samples: 0.33, 2.7 and 19 ms with one CTA over all counters,
+// 0.27, 1.1 and 3.7 ms by a library radix sort, now 0.10, 0.53 and 2.5 ms.)
+__global__ void __launch_bounds__(1024) k_order_sums(const __grid_constant__ OrderBatch B) {
   const OrderJob &J = B.job[blockIdx.y];
-  const uint32_t shift = 64 - order_bits(J.n), epoch = J.epoch + (epoch_dev ? *epoch_dev : 0u);
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < J.n; i += gridDim.x * blockDim.x) {
-    const uint64_t k = order_key(J, epoch, i);
-    const uint32_t at = atomicAdd(&J.cnt[k >> shift], 1u);
-    J.key[at] = k;
-    J.out[at] = i;
+  const uint32_t nb = 1u << order_bits(J.n), c = order_chunk(nb);
+  if (blockIdx.x >= nb / c) return;
+  const uint4 *q = (const uint4 *)(J.cnt + (size_t)blockIdx.x * c);
+  uint32_t sum = 0, before;
+  for (uint32_t i = threadIdx.x; i < c / 4; i += 1024) {
+    const uint4 v = q[i];
+    sum += v.x + v.y + v.z + v.w;
+  }
+  const uint32_t all = block_scan(sum, before);
+  if (threadIdx.x == 0) J.cnt[nb + blockIdx.x] = all;
+}
+__global__ void __launch_bounds__(1024) k_order_scan(const __grid_constant__ OrderBatch B) {
+  const OrderJob &J = B.job[blockIdx.y];
+  const uint32_t nb = 1u << order_bits(J.n), c = order_chunk(nb);
+  if (blockIdx.x >= nb / c) return;
+  uint4 *q = (uint4 *)(J.cnt + (size_t)blockIdx.x * c);
+  uint32_t before;
+  uint32_t base = block_scan(threadIdx.x < blockIdx.x ? J.cnt[nb + threadIdx.x] : 0u, before);
+  for (uint32_t i = threadIdx.x; i < c / 4; i += 1024) {
+    uint4 v = q[i];
+    const uint32_t all = block_scan(v.x + v.y + v.z + v.w, before);
+    uint32_t at = base + before;
+    const uint4 o = make_uint4(at, at + v.x, at + v.x + v.y, at + v.x + v.y + v.z);
+    q[i] = o;
+    base += all;
   }
 }
-__global__ void k_order_sort(const __grid_constant__ OrderBatch B) {
+// An entry of a bucket: the 32 key bits below those that name the bucket, then
+// the sample, so that placing a sample is one 8-byte write: bound by memory, each
+// write a sector of its own (an order of 2^25 samples 2.5 ms, with whole keys and
+// samples in two places 4.9 ms).
+__global__ void k_order_place(const __grid_constant__ OrderBatch B, const uint32_t *epoch_dev) {
   const OrderJob &J = B.job[blockIdx.y];
-  const uint32_t nb = 1u << order_bits(J.n);
-  for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x)
-    sort_bucket(J.key, J.out, b ? J.cnt[b - 1] : 0, J.cnt[b]);
+  const uint32_t bits = order_bits(J.n), epoch = J.epoch + (epoch_dev ? *epoch_dev : 0u);
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < J.n; i += gridDim.x * blockDim.x) {
+    const uint64_t k = order_key(J, epoch, i);
+    const uint32_t at = atomicAdd(&J.cnt[k >> (64 - bits)], 1u);
+    J.key[at] = (k << bits >> 32) << 32 | i;
+  }
+}
+// Entries by (key, sample), the samples alone to `out`.  Two entries of equal 32
+// bits (one pair in sixteen orders of 2^27) are compared by their whole keys.
+__global__ void k_order_sort(const __grid_constant__ OrderBatch B, const uint32_t *epoch_dev) {
+  const OrderJob &J = B.job[blockIdx.y];
+  const uint32_t nb = 1u << order_bits(J.n), epoch = J.epoch + (epoch_dev ? *epoch_dev : 0u);
+  auto above = [&](uint64_t a, uint64_t b) {
+    if ((a ^ b) >> 32) return a > b;
+    const uint64_t ka = order_key(J, epoch, (uint32_t)a), kb = order_key(J, epoch, (uint32_t)b);
+    return ka != kb ? ka > kb : a > b;
+  };
+  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < nb; k += gridDim.x * blockDim.x) {
+    const uint32_t lo = k ? J.cnt[k - 1] : 0, hi = J.cnt[k];
+    for (uint32_t a = lo + 1; a < hi; a++) {
+      const uint64_t v = J.key[a];
+      uint32_t q = a;
+      for (; q > lo && above(J.key[q - 1], v); q--) J.key[q] = J.key[q - 1];
+      J.key[q] = v;
+    }
+    for (uint32_t a = lo; a < hi; a++) J.out[a] = (uint32_t)J.key[a];
+  }
 }
 
 static size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 
 // scratch of one order (none for small ones)
 size_t order_scratch_bytes(uint32_t n) {
-  return n <= ORDER_SMALL ? 0 : align256((size_t)n * 8) + align256((size_t)4 << order_bits(n));
+  return n <= ORDER_SMALL ? 0 : align256((size_t)n * 8) +
+                                 align256(((size_t)4 << order_bits(n)) + 4 * ORDER_CHUNKS);
 }
 
 // Queues the orders of `jobs` (out, seed, epoch and n set).  scratch holds at
@@ -355,10 +427,13 @@ cudaError_t launch_orders(OrderJob *jobs, size_t count, void *scratch, size_t sc
       const uint32_t bx = (nmax + 255) / 256 < 148 * 4 ? (nmax + 255) / 256 : 148 * 4;
       const dim3 grid(bx, k);
       k_order_count<<<grid, 256, 0, st>>>(B, epoch_dev);
-      k_order_scan<<<k, 1024, 0, st>>>(B);
+      const uint32_t nb = 1u << order_bits(nmax);
+      const dim3 chunks(std::min(nb / order_chunk(nb), ORDER_CHUNKS), k);
+      k_order_sums<<<chunks, 1024, 0, st>>>(B);
+      k_order_scan<<<chunks, 1024, 0, st>>>(B);
       k_order_place<<<grid, 256, 0, st>>>(B, epoch_dev);
-      k_order_sort<<<dim3((bx + 3) / 4, k), 256, 0, st>>>(B);
-      if (launches) *launches += 4;
+      k_order_sort<<<grid, 256, 0, st>>>(B, epoch_dev);
+      if (launches) *launches += 5;
     }
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
