@@ -475,15 +475,17 @@ def run_ours(args, w):
                                             / 1e3 + 1e-12),
         },
     }
-    if rank == 0 and st["predict_gemm"]:
+    path = t.predict_path() if rank == 0 else None
+    if path in ("fp4", "int8", "fp8"):
         # the predict ran on the tensor cores: clauses x samples x literals (32
         # per row word), two operations per product
         words = (((2 * w["features"] + 7) // 8 + 3) // 4)
         ops = 2.0 * w["classes"] * w["clauses"] * (hi_s - lo_s) * 32 * words
         t_s = st["predict_kernel_ms"] / max(1, st["predict_launches"]) / 1e3 + 1e-12
-        peak = 4.5e15 if st["predict_gemm"] == 1 else 9e15
+        peak = 9e15 if path == "fp4" else 4.5e15
         out["kernels"].update({
-            "predict_path": "int8 GEMM" if st["predict_gemm"] == 1 else "e2m1 vote kernel",
+            "predict_path": {"fp4": "e2m1 vote kernel", "int8": "int8 GEMM",
+                             "fp8": "e4m3 GEMM"}[path],
             "predict_tensor_ops_per_s": ops / t_s,
             "predict_tensor_peak_ops_per_s": peak,
             "predict_tensor_peak_source": "nominal dense rate of a B200 at the operands' width "
@@ -494,9 +496,9 @@ def run_ours(args, w):
         pk = tm.int_peaks(dev.index if dev.index is not None else 0)
         wops = out["kernels"]["predict_literal_evals_per_s"] / 32
         bound = min(32 * pk["lop3"] / 62, 32 * pk["popc"] / 17)
-        # beyond what testing every word allows: literal lists
-        path = "literal lists" if wops > bound else "bitwise"
-        out["kernels"].update({"predict_path": path, "int_peaks_ops_per_s": pk,
+        # (lists leave words out: beyond what testing every word allows)
+        out["kernels"].update({"predict_path": "literal lists" if path == "lists" else path,
+                               "int_peaks_ops_per_s": pk,
                                "predict_word_ops_per_s": wops,
                                "predict_int_bound_word_ops_per_s": bound,
                                "predict_frac_of_int_bound": wops / bound})

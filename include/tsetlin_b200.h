@@ -351,7 +351,8 @@ typedef struct tm_stats {
   int32_t train_cpw;          /* modes 0-2: clauses per warp; mode 3: 1 = four units per
                                  CTA, 2 = one; mode 4: the configuration (1-12) */
   int32_t predict_gemm;       /* last predict: 0 bitwise kernels or lists, 1 int8 GEMM, 2 GEMM of
-                                 small floats (the e2m1 vote kernel, or e4m3) */
+                                 small floats (the e2m1 vote kernel, or e4m3);
+                                 tm_predict_path tells all of them apart */
   uint64_t train_active_pairs; /* (unit, sample) steps trained after negative sampling */
   double search_epoch_ms;     /* device-resident search rounds: summed epoch graph time */
   uint64_t search_epochs;     /* epoch graph replays */
@@ -392,6 +393,15 @@ int tm_debug_fail_alloc(int64_t after);
 /* on != 0 starts timing (events around every train / predict kernel). */
 int tm_stats_enable(tm_machine *m, int32_t on);
 int tm_get_stats(const tm_machine *m, tm_stats *out);
+/* What evaluated the machine's last predict: TM_PATH_*. */
+#define TM_PATH_NONE 0    /* no predict yet */
+#define TM_PATH_FEW 1     /* the one-launch kernel of up to 32 samples */
+#define TM_PATH_BITS 2    /* bitwise tiles */
+#define TM_PATH_LISTS 3   /* literal lists */
+#define TM_PATH_FP4 4     /* tensor cores, 4-bit floats */
+#define TM_PATH_INT8 5    /* cuBLASLt products of 8-bit integers */
+#define TM_PATH_FP8 6     /* cuBLASLt products of 8-bit floats */
+int tm_predict_path(const tm_machine *m);
 int tm_reset_stats(tm_machine *m);
 
 /* ---- serving: resident machines, continuous batching ------------------- */

@@ -186,6 +186,7 @@ struct tm_machine {
   PoolBuf lists, list_groups;
   int list_state = 0;  // 0 not looked at, 1 lists made, 2 too many literals
   uint32_t few_calls = 0;  // small predicts in this state of the automata
+  int predict_path = TM_PATH_NONE;  // of the last predict
   int act8_kind = 0;
   // (owner of a search round) the vote kernel's copy of the actions, shared
   // by the round's machines one after another, and the expanded holdout of
@@ -541,8 +542,13 @@ extern "C" int tm_get_stats(const tm_machine *m, tm_stats *out) {
   return TM_OK;
 }
 
+extern "C" int tm_predict_path(const tm_machine *m) {
+  return m ? m->predict_path : fail(TM_ERR_ARG, "null machine");
+}
+
 extern "C" int tm_reset_stats(tm_machine *m) {
   if (!m) return fail(TM_ERR_ARG, "null machine");
+  m->predict_path = TM_PATH_NONE;
   m->stats = tm_stats{};
   return TM_OK;
 }
@@ -2143,6 +2149,7 @@ static int predict_few(tm_machine *m, const uint8_t *problems, uint64_t n, int64
   if (m->timing) CK(cudaEventRecord(m->ev1, m->st));
   m->stats.predict_launches++;
   m->stats.predict_gemm = 0;
+  m->predict_path = TM_PATH_FEW;
   if (!on_device && !po) {
     if (out_classes) CK(cudaMemcpyAsync(out_classes, f.out_classes, clsb, cudaMemcpyDeviceToHost, m->st));
     if (out_codes) CK(cudaMemcpyAsync(out_codes, f.out_codes, codb, cudaMemcpyDeviceToHost, m->st));
@@ -2367,6 +2374,10 @@ static int predict_common(tm_machine *m, const uint8_t *problems, const int64_t 
     if (gr < 0) return gr;
   }
   m->stats.predict_gemm = gr || lists ? 0 : (votes ? TM_GEMM_FP8 : m->act8_kind);
+  m->predict_path = gr      ? TM_PATH_BITS
+                    : lists ? TM_PATH_LISTS
+                    : votes ? TM_PATH_FP4
+                    : m->act8_kind == TM_GEMM_FP8 ? TM_PATH_FP8 : TM_PATH_INT8;
   if (gr == 1) {
     CK(launch_predict(m->d_act, m->d_lits, m->d_cls, nullptr, m->classes, m->clauses, m->tol,
                       m->x.as<uint32_t>(), (uint32_t)n, m->sums.as<int32_t>(), m->st));

@@ -159,6 +159,9 @@ class _ServerConfig(ctypes.Structure):
     ]
 
 
+# by the numbers of tm_predict_path
+PREDICT_PATHS = ("none", "few", "bitwise", "lists", "fp4", "int8", "fp8")
+
 _lib = None
 EXPORTS = (
     "tm_params_init", "tm_create", "tm_train", "tm_train_batch", "tm_train_batch_each",
@@ -169,7 +172,7 @@ EXPORTS = (
     "tm_checkpoint", "tm_restore", "tm_reconfigure", "tm_restrict", "tm_type",
     "tm_destroy", "tm_last_error", "tm_align", "tm_get_info", "tm_export_state",
     "tm_import_state", "tm_export_classes", "tm_import_classes", "tm_class_accuracy", "tm_encoding_accuracy", "tm_bits_to_cvec", "tm_bits_to_cvec_ind",
-    "tm_predict_noalloc", "tm_int_peaks", "tm_debug_fail_alloc", "tm_set_autotune", "tm_force_variant", "tm_stats_enable", "tm_get_stats", "tm_reset_stats", "tm_serve_open", "tm_serve_submit", "tm_serve_poll",
+    "tm_predict_noalloc", "tm_int_peaks", "tm_debug_fail_alloc", "tm_set_autotune", "tm_force_variant", "tm_stats_enable", "tm_get_stats", "tm_predict_path", "tm_reset_stats", "tm_serve_open", "tm_serve_submit", "tm_serve_poll",
     "tm_serve_latency_us", "tm_serve_phases_us", "tm_serve_stats", "tm_serve_close",
 )
 
@@ -225,6 +228,7 @@ def lib():
     L.tm_bits_to_cvec_ind.argtypes = [vp, vp, vp, u32, u64, i32, i32, i32, vp, u64, vp]
     L.tm_stats_enable.argtypes = [vp, i32]
     L.tm_get_stats.argtypes = [vp, ctypes.POINTER(Stats)]
+    L.tm_predict_path.argtypes = [vp]
     L.tm_reset_stats.argtypes = [vp]
     L.tm_serve_open.argtypes = [ctypes.POINTER(_ServerConfig), ctypes.POINTER(vp), u32,
                                 ctypes.POINTER(vp)]
@@ -513,6 +517,12 @@ class Machine:
         st = Stats()
         _check(lib().tm_get_stats(self.handle, ctypes.byref(st)))
         return st.as_dict()
+
+    def predict_path(self):
+        """What evaluated the last predict: one of PREDICT_PATHS."""
+        path = lib().tm_predict_path(self.handle)
+        _check(path)
+        return PREDICT_PATHS[path]
 
     def reset_stats(self):
         _check(lib().tm_reset_stats(self.handle))
