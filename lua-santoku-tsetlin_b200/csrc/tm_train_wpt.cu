@@ -1291,6 +1291,11 @@ constexpr bool wpt_in_order() {
 }
 static_assert(wpt_in_order(), "a configuration's place is its id");
 
+// The configuration that a launch of rows of at most Wpmax words runs for `id`:
+// 7 serves rows of up to 64 words to callers that pin it, those above its own
+// slots in the 64-word ones of 6.
+static int wpt_slot(int id, uint32_t Wpmax) { return id == 7 && Wpmax > 56 ? 6 : id; }
+
 static uint32_t wpt_ovf_cap(uint32_t smax) { return smax / 4 > 0 ? smax / 4 : 1; }
 
 double wpt_overflow(uint32_t bits, uint32_t picks) {
@@ -1331,6 +1336,7 @@ static int config_occ(int id, size_t bytes) {
 // Wpmax words (0 when it cannot hold them), and its shared memory.
 int train_wpt_occupancy(int id, uint32_t Wpmax, uint32_t smax, bool many_ovf, size_t *smem_bytes) {
   if (id < 1 || id > kWptCount) return 0;
+  id = wpt_slot(id, Wpmax);
   const WptConfig &k = kWpt[id - 1];
   if (Wpmax > (uint32_t)k.sw) return 0;
   const size_t bytes = wpt_bytes(k, smax);
@@ -1403,7 +1409,9 @@ cudaError_t launch_train_wpt(int id, const TrainDev *machines, const WorkItem *w
                              uint32_t nwork, uint32_t *counter, uint32_t e_begin, uint32_t e_end,
                              uint32_t Wpmax, uint32_t smax, bool many_ovf, int grid, uint32_t *err,
                              cudaStream_t st) {
-  if (id < 1 || id > kWptCount || Wpmax > (uint32_t)kWpt[id - 1].sw) return cudaErrorInvalidValue;
+  if (id < 1 || id > kWptCount) return cudaErrorInvalidValue;
+  id = wpt_slot(id, Wpmax);
+  if (Wpmax > (uint32_t)kWpt[id - 1].sw) return cudaErrorInvalidValue;
   const size_t bytes = wpt_bytes(kWpt[id - 1], smax);
   (many_ovf ? config_launch<true> : config_launch<false>)(id, grid, bytes, st, machines, work, nwork,
                                                           counter, e_begin, e_end,

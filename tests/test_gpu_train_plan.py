@@ -6,6 +6,9 @@ all epochs at once."""
 import numpy as np
 import pytest
 
+import oracle as O
+from test_gpu_parity import ref_table, train_table
+
 pytestmark = pytest.mark.gpu
 
 SHAPES = [
@@ -90,3 +93,29 @@ def test_few_units_get_more_threads_where_that_is_faster(tm):
                  iterations=1))
     st = t.stats()
     assert (st["train_mode"], st["train_cpw"], st["train_autotuned"]) == (4, 4, 1)
+
+
+@pytest.mark.parametrize("features,config", [
+    (880, 7), (912, 7), (1024, 7), (1024, 6), (1024, 5), (4096, 4), (8192, 3), (4096, 2),
+    (16384, 1)])
+def test_pinned_configurations_hold_the_widest_rows_they_held(tm, features, config):
+    """Rows of 55 to 1,024 words under the configurations whose numbers callers may
+    have pinned: 7 holds 64 words, also since its own slots have 56."""
+    rng = np.random.default_rng(features)
+    n, classes = 80, 3
+    b = rng.random((n, features)) < 0.1
+    x = np.packbits(np.concatenate([b, ~b], axis=1), axis=1, bitorder="little").ravel()
+    y = rng.integers(0, classes, size=n).astype(np.int64)
+    cfg = dict(type="classifier", classes=classes, features=features, clauses=16,
+               clause_tolerance=12, clause_maximum=30, specificity=8.0, target=12)
+    m = O.Machine(**cfg)
+    m.train(x, n, 2, labels=y, seed=6)
+    kind, tbl = ref_table(cfg, seed=6)
+    t = tm.create(kind, tbl)
+    t.force_variant(4, config)
+    t.stats_enable(True)
+    t.train(train_table(kind, dict(n=n, x=x, labels=y), 2))
+    assert (t.stats()["train_mode"], t.stats()["train_cpw"]) == (4, config)
+    a, s = t.export_state()
+    assert np.array_equal(a, m.actions()) and np.array_equal(s, m.state())
+    t.destroy()
