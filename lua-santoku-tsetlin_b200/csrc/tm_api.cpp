@@ -192,6 +192,9 @@ struct tm_machine {
   // by the round's machines one after another, and the expanded holdout of
   // each distinct holdout row layout
   DevBuf search_act4;
+  // the same as bytes, for machines whose holdout runs as the library's GEMM
+  DevBuf search_act8;
+  std::vector<DevBuf> search_x8;
   // vote sums and CTA count of k_predict_few, zero between calls
   DevBuf few;
   int sms = 0;  // of the device, once asked
@@ -493,13 +496,14 @@ extern "C" void tm_destroy(tm_machine *m) {
   for (DevBuf *b : {&m->x, &m->tx, &m->raw, &m->labels, &m->codes, &m->perm, &m->perm_scratch, &m->sums,
                     &m->outc, &m->work, &m->tdev, &m->cls_job, &m->errf, &m->ckpt, &m->search,
                     &m->search_truth, &m->act8, &m->x8, &m->gemm_c, &m->gemm_ws,
-                    &m->search_act4, &m->tune_snap, &m->few})
+                    &m->search_act4, &m->search_act8, &m->tune_snap, &m->few})
     b->release();
   m->act4.release(m->st);
   m->lists.release(m->st);
   m->list_groups.release(m->st);
   m->x4.release(m->st);
   for (DevBuf &b : m->search_x4) b.release();
+  for (DevBuf &b : m->search_x8) b.release();
   if (m->ev0) cudaEventDestroy(m->ev0);
   if (m->ev1) cudaEventDestroy(m->ev1);
   if (m->pin_ev) cudaEventDestroy(m->pin_ev);
@@ -1475,6 +1479,7 @@ static int train_batch_impl(tm_machine *const *ms, const tm_train_args *args, ui
 // flag, so stopped machines drop out of the replays without a new graph.
 // ---------------------------------------------------------------------------
 static bool votes_path(tm_machine *m, uint64_t n);
+static bool gemm_wanted(tm_machine *m, uint64_t n);
 
 static int search_round(tm_machine *const *ms, const tm_train_args *args, uint32_t count,
                         const tm_search_args *sa) {
@@ -1586,6 +1591,78 @@ static int search_round(tm_machine *const *ms, const tm_train_args *args, uint32
     if (no_memory(e)) use_votes.assign(count, 0);
     else CK(e);
   }
+  // ---- or as the library's 8-bit GEMM ----------------------------------------
+  // where that is asked for, or k_votes' ranges do not hold: the same with bytes,
+  // in chunks of samples.  Each product width is tried once here, outside the
+  // capture: a machine whose shape the library cannot take keeps the bitwise
+  // predict, as one does whose copies find no memory.
+  const int gkind = gemm_kind_of(m0->device);
+  const size_t gws = 32u << 20;
+  std::vector<uint64_t> gchunk(count, 0);  // samples per product, 0: no GEMM
+  std::vector<const uint8_t *> gx8(count, nullptr);
+  auto holdout_products = [&](uint32_t i, uint64_t s0) {
+    const uint64_t M = (uint64_t)ms[i]->classes * ms[i]->clauses, K = (uint64_t)ms[i]->cls[0].W * 32;
+    return gemm_clause_products(m0->device, gkind, m0->search_act8.as<uint8_t>(),
+                                gx8[i] + s0 * K, m0->gemm_c.p, M,
+                                gemm_bucket(std::min(gchunk[i], nt - s0), gchunk[i]), K,
+                                m0->gemm_ws.p, gws, st);
+  };
+  {
+    uint64_t cmax = 0, amax = 0, pad = 0;
+    for (uint32_t i = 0; i < count; i++) {
+      tm_machine *m = ms[i];
+      const uint64_t M = (uint64_t)m->classes * m->clauses, W = m->cls[0].W;
+      if (use_votes[i] || !gemm_wanted(m, nt) || (votes_path(m, nt) && nt * W * 16 <= (2ull << 30)))
+        continue;
+      gchunk[i] = std::max<uint64_t>(64, ((512ull << 20) / (4 * M)) / 64 * 64);
+      const uint64_t cols = gemm_bucket(std::min<uint64_t>(gchunk[i], nt), gchunk[i]);
+      cmax = std::max<uint64_t>(cmax, cols * M * 4);
+      pad = std::max(pad, cols);
+      amax = std::max<uint64_t>(amax, M * W * 32);
+    }
+    if (cmax) {
+      cudaError_t e = m0->gemm_c.ensure(cmax);
+      if (e == cudaSuccess) e = m0->gemm_ws.ensure(gws);
+      if (e == cudaSuccess) e = m0->search_act8.ensure(amax);
+      if (no_memory(e)) gchunk.assign(count, 0);
+      else CK(e);
+    }
+    std::map<std::tuple<const void *, uint64_t, uint32_t, uint32_t>, size_t> x8_of;
+    for (uint32_t i = 0; i < count; i++) {
+      if (!gchunk[i]) continue;
+      tm_machine *m = ms[i];
+      const ClassDev &c0 = m->cls[0];
+      const void *src = sa->test_each && sa->test_each[i] ? (const void *)sa->test_each[i]
+                                                          : (const void *)sa->test_problems;
+      const auto key = std::make_tuple(src, (uint64_t)m->features, c0.Wp, c0.W);
+      auto it = x8_of.find(key);
+      if (it == x8_of.end()) {
+        const size_t at = x8_of.size();
+        if (m0->search_x8.size() <= at) m0->search_x8.resize(at + 1);
+        // rows past nt: the last product's bucket reads them (its columns there
+        // are not used)
+        const cudaError_t e = m0->search_x8[at].ensure((nt + pad) * c0.W * 32);
+        if (no_memory(e)) {
+          gchunk[i] = 0;
+          continue;
+        }
+        CK(e);
+        it = x8_of.emplace(key, at).first;
+        CK(launch_expand_bits(m->x.as<uint32_t>(), nt, c0.Wp, c0.W, 0xFFFFFFFFu, gkind,
+                              m0->search_x8[at].as<uint8_t>(), st));
+      }
+      gx8[i] = m0->search_x8[it->second].as<uint8_t>();
+      for (uint64_t s0 = 0; s0 < nt; s0 += gchunk[i]) {
+        const int g = holdout_products(i, s0);
+        if (g > 0) return fail(TM_ERR_CUDA, "search: cuBLASLt matmul failed (status %d)", g);
+        if (g < 0) {
+          gchunk[i] = 0;
+          break;
+        }
+      }
+    }
+    if (cmax) CK(cudaStreamSynchronize(st));
+  }
   // machine i's vote sums of the holdout, added to its (cleared) sums unless
   // *gate is 0
   auto holdout_votes = [&](uint32_t i, const uint32_t *gate, uint32_t *err) -> cudaError_t {
@@ -1645,7 +1722,7 @@ static int search_round(tm_machine *const *ms, const tm_train_args *args, uint32
     P.classes = m->classes;
     const uint32_t jt = predict_job_tiles((uint32_t)nt, m->classes, m->clauses, &P.stiles, &P.tpc);
     P.tile0 = tiles;
-    if (!use_votes[i]) tiles += jt;  // a job without tiles is never picked
+    if (!use_votes[i] && !gchunk[i]) tiles += jt;  // a job without tiles is never picked
     pjf[i] = P;
     pjf[i].tile0 = tiles_f;
     if (!use_votes[i]) tiles_f += jt;
@@ -1865,6 +1942,24 @@ static int search_round(tm_machine *const *ms, const tm_train_args *args, uint32
       if (!use_votes[i]) continue;
       ce = holdout_votes(i, &d_state[i].live, d_err);
       launches += 2;
+    }
+    for (uint32_t i = 0; i < count && ce == cudaSuccess; i++) {
+      if (!gchunk[i]) continue;
+      tm_machine *m = ms[i];
+      const ClassDev &c0 = m->cls[0];
+      ce = launch_expand_bits(m->d_act + c0.act_off, (uint64_t)m->classes * m->clauses, c0.Wp, c0.W,
+                              c0.emask, gkind, m0->search_act8.as<uint8_t>(), st);
+      launches++;
+      for (uint64_t s0 = 0; s0 < nt && ce == cudaSuccess; s0 += gchunk[i]) {
+        if (holdout_products(i, s0) != 0) {
+          ce = cudaErrorUnknown;
+          break;
+        }
+        ce = launch_gemm_votes(m0->gemm_c.p, gkind, m->d_lits, m->classes, m->clauses, m->tol,
+                               (uint32_t)std::min(gchunk[i], nt - s0),
+                               m->sums.as<int32_t>() + s0 * m->classes, st, &d_state[i].live);
+        launches++;  // the epilogue (the GEMM is the library's)
+      }
     }
     if (ce == cudaSuccess)
       ce = launch_search_score((const ScoreJob *)(base + o_sj), d_state, d_scores, Es, count,
