@@ -407,6 +407,8 @@ int tmb_fail(int code, const char *msg);
 // null when the device has no GEMM encoding or the machine is
 // individualized.  The bytes stay valid until the automata change.
 int tmb_machine_act8(tm_machine *m, tmb::MachineView *v);
+// samples that one launch of k_votes takes against `rows` clause rows (tm_votes.cu)
+extern "C" uint32_t tmb_votes_span(uint64_t rows);
 // whether the failure injection of tm_debug_fail_alloc fails this allocation
 bool tmb_alloc_fails();
 // gives the scratch pool's unused memory of the current device back (tm_util.cu)

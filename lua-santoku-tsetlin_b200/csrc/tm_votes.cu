@@ -29,6 +29,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <atomic>
 
 #include "tm_device.cuh"
@@ -447,11 +448,7 @@ cudaError_t launch_expand_fp4_bytes(const uint8_t *src, uint64_t rows, uint32_t 
 cudaError_t launch_votes(int dev, int sms, const uint8_t *act4, const uint8_t *x4, uint32_t classes,
                          uint32_t clauses, uint32_t W, uint32_t tol, const int32_t *lits, uint32_t n,
                          int32_t *sums, const uint32_t *gate, uint32_t *err, cudaStream_t st) {
-  if (!n) return cudaSuccess;
-  CUtensorMap xmap, amap;
   const uint64_t rows = (uint64_t)classes * clauses, bytes = 16ull * W;
-  if (!encode_rows(&xmap, x4, n, bytes, VT_M / 2) || !encode_rows(&amap, act4, rows, bytes, VT_N / 2))
-    return cudaErrorInvalidValue;
   static std::atomic<uint64_t> ready{0};  // devices whose shared-memory limit is raised
   if (!(ready.load() >> (dev & 63) & 1u)) {
     const cudaError_t e =
@@ -459,17 +456,35 @@ cudaError_t launch_votes(int dev, int sms, const uint8_t *act4, const uint8_t *x
     if (e != cudaSuccess) return e;
     ready.fetch_or(1ull << (dev & 63));
   }
-  VotesTiles T;
-  T.samples = n;
-  T.rows = (uint32_t)rows;
-  T.st = (n + VT_M - 1) / VT_M;
-  T.ct = (uint32_t)((rows + VT_N - 1) / VT_N);
-  T.steps = (uint32_t)((bytes + VT_KB - 1) / VT_KB);
-  const uint64_t tiles = (uint64_t)T.st * T.ct;
-  const uint64_t pairs = (uint64_t)sms / 2 < tiles ? (uint64_t)sms / 2 : tiles;
-  k_votes<<<(unsigned)(2 * pairs), 256, VT_SMEM, st>>>(xmap, amap, T, lits, clauses, classes, tol,
-                                                       sums, gate, err);
-  return cudaGetLastError();
+  const uint32_t span = tmb_votes_span(rows);
+  for (uint64_t s0 = 0; s0 < n; s0 += span) {
+    CUtensorMap xmap, amap;
+    VotesTiles T;
+    T.samples = (uint32_t)std::min<uint64_t>(span, n - s0);
+    if (!encode_rows(&xmap, x4 + s0 * bytes, T.samples, bytes, VT_M / 2) ||
+        !encode_rows(&amap, act4, rows, bytes, VT_N / 2))
+      return cudaErrorInvalidValue;
+    T.rows = (uint32_t)rows;
+    T.st = (uint32_t)(((uint64_t)T.samples + VT_M - 1) / VT_M);
+    T.ct = (uint32_t)((rows + VT_N - 1) / VT_N);
+    T.steps = (uint32_t)((bytes + VT_KB - 1) / VT_KB);
+    const uint64_t tiles = (uint64_t)T.st * T.ct;
+    const uint64_t pairs = (uint64_t)sms / 2 < tiles ? (uint64_t)sms / 2 : tiles;
+    k_votes<<<(unsigned)(2 * pairs), 256, VT_SMEM, st>>>(xmap, amap, T, lits, clauses, classes, tol,
+                                                         sums + s0 * classes, gate, err);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
 }  // namespace tmb
+
+// Samples per launch against `rows` clause rows: all of them, unless the launch
+// counts 2^31 tiles and more (the kernel's tile numbers, and their last step
+// past the end, have 32 bits); then whole tiles, at least one.
+uint32_t tmb_votes_span(uint64_t rows) {
+  const uint64_t ct = (rows + tmb::VT_N - 1) / tmb::VT_N, most = ((1ull << 31) - 1) / (ct ? ct : 1);
+  const uint64_t span = (most ? most : 1) * tmb::VT_M;
+  return span < (1ull << 31) ? (uint32_t)span : 1u << 31;
+}
