@@ -1137,6 +1137,10 @@ __global__ void __launch_bounds__(SP_NT, MINB)
                 const bool is1 = (t1 & jbit) != 0, incx = (incm & jbit) != 0;
                 const uint32_t slot = __popc(ibm & (jbit - 1u));
                 const uint32_t *xs = ring + ((b + w) % R) * SW + 2 * lane;
+                // nonzero if the clause's actions may move.  Those of a Type Ia clause
+                // without increments do not: other warps may be reading them for the
+                // next round, so they are not written
+                const uint32_t act_moves = ((ibm | incm | ~t1) & jbit) | (ib - 1u);
 #pragma unroll 1
                 for (int k = 0; k < NK; k++) {
                   uint32_t p[M7][2], ac[2], x[2], mv[2], ma[2];
@@ -1204,7 +1208,7 @@ __global__ void __launch_bounds__(SP_NT, MINB)
                   }
 #pragma unroll
                   for (int bb = 0; bb < M7; bb++) WVec<2>::st(own + bb * SW + 64 * k, p[bb]);
-                  WVec<2>::st(own + M7 * SW + 64 * k, ac);
+                  if (act_moves) WVec<2>::st(own + M7 * SW + 64 * k, ac);
                 }
               }
               if (ibm || incm || (fbm & ~t1) || ib > 1) {
