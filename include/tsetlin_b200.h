@@ -360,15 +360,19 @@ typedef struct tm_stats {
   uint64_t train_resident;    /* units resident at once in the last train launch */
 } tm_stats;
 /* Train-kernel variant choice.  All variants end in the same automaton
- * state; they differ in speed.  mode 0: heuristic (resident CTAs per SM);
- * 1 (default, or TSETLIN_B200_AUTOTUNE at create): the first train call of
- * a launch shape times every feasible variant on a short trial (up to 2,048
- * samples of epoch 0 on up to 32 units per SM taken evenly from the launch's
- * work list, from the initial automata), then the three fastest on a longer
- * one (8,192 samples, 64 units per SM: positions 8,192-16,383 of epoch 0
- * from the automata as the first 8,192 leave them, or the first 8,192 from
- * the initial state for shorter launches) -- the automata are reset to the
- * initial state afterwards -- and caches the fastest for
+ * state; they differ in speed.  mode 0: heuristic among modes 0-3 of
+ * train_mode (resident CTAs per SM); 1 (default, or TSETLIN_B200_AUTOTUNE at
+ * create): launches of 8-bit units with rows up to 1,024 words take mode 4 (of
+ * few units with rows above 256 words, mode 2 is tried too).  Where one
+ * configuration is worth trying it is taken, as is the first choice by later
+ * launches of a call whose shape was not tuned; where several are (few units),
+ * or for other units, the first train call of a launch shape times them on a
+ * short trial (up to 2,048 samples of epoch 0 on up to 32 units per SM taken
+ * evenly from the launch's work list, from the initial automata), then the three
+ * fastest on a longer one (8,192 samples, 64 units per SM: positions
+ * 8,192-16,383 of epoch 0 from the automata as the first 8,192 leave them, or
+ * the first 8,192 from the initial state for shorter launches) -- the automata
+ * are reset to the initial state afterwards -- and caches the fastest for
  * the process; 2: tune on every train call.  No counterpart in the
  * reference (it has one CPU code path). */
 int tm_set_autotune(tm_machine *m, int32_t mode);
@@ -376,7 +380,7 @@ int tm_set_autotune(tm_machine *m, int32_t mode);
 /* Pins the train-kernel variant (train_mode values of tm_stats; cpw, the
  * clauses evaluated per warp in a single-CTA variant with 8 state bits: 1,
  * 2 or 4 -- 256 / cpw threads per unit; for mode 3, 1 or 2: four units or
- * one per CTA; for mode 4, the configuration); mode -1 returns to the automatic
+ * one per CTA; for mode 4, the configuration, 1-8); mode -1 returns to the automatic
  * choice.  A train call that the pinned variant cannot run fails with
  * TM_ERR_ARG.  The environment variable TSETLIN_B200_VARIANT=mode:cpw, read
  * when a machine is created, pins the same way.  For tests and

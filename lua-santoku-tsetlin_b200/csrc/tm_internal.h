@@ -159,9 +159,10 @@ uint64_t gemm_bucket(uint64_t k, uint64_t cap);
 // The fused train kernels report through err[0] (status bits) and
 // err[2..3], a 64-bit count of active (unit, sample) steps -- the samples
 // each unit actually trained on after negative sampling.
-// The kernels of tm_train_wpt.cu: one CTA per unit, the automata of 8-bit
-// units on the SM while the unit trains; `cpw` of a plan with this mode is
-// the configuration id (1-based).  Callers may pin ids up to TM_WPT_PINNED.
+// The kernels of tm_train_wpt.cu: one CTA per 8-bit unit, its actions on the SM
+// while it trains, its count planes there or in global memory; `cpw` of a plan
+// with this mode is the configuration id (1-based).  Callers may pin ids up to
+// TM_WPT_PINNED; the others are row slots that only the choice by width uses.
 constexpr int TM_WPT_PINNED = 8;
 constexpr int TM_MODE_WPT = 4;
 int wpt_choices(uint32_t Wpmax, uint32_t smax, uint32_t units, int sms, int optin, int *ids,

@@ -1804,8 +1804,8 @@ __device__ __forceinline__ uint32_t xor3(uint32_t a, uint32_t b, uint32_t c) {
 constexpr int FEW_DEPTH = 8;  // copies in flight per lane
 
 // U: steps of the row loop unrolled, so that ring slots and the choice of
-// counting are fixed per step (4 for rows of more than 3 steps; rows are then
-// padded to whole groups of U steps), or 1.
+// counting are fixed per step (a whole ring of them, 4 or 8, for rows of more than
+// 3 steps, which are then padded to whole groups of U steps), or 1.
 template <int NS, int CR, int U>
 __global__ void __launch_bounds__(256, NS <= 2 ? 4 : (NS <= 5 ? 3 : 2))
     k_predict_few(const uint32_t *__restrict__ act, const int32_t *__restrict__ lits,
@@ -2049,7 +2049,7 @@ static cudaError_t few_launch_u(const PredictFew &f, uint32_t s0, uint32_t ns, c
 
 template <int NS, int CR>
 static cudaError_t few_launch(const PredictFew &f, uint32_t s0, uint32_t ns, cudaStream_t st) {
-  constexpr int U = 8 / (CR * 2) * 2;  // a whole ring of steps for CR 2, half of one for CR 1
+  constexpr int U = FEW_DEPTH / CR;  // a whole ring of steps
   return f.C.Wp > 3 * 128 ? few_launch_u<NS, CR, U>(f, s0, ns, st)
                           : few_launch_u<NS, CR, 1>(f, s0, ns, st);
 }

@@ -15,7 +15,7 @@
 //                   them from the clause's literal count and adds the votes in
 //                   bit-sliced sums, which are formed into numbers once per class
 //
-// Bound by LOP3 (59 % of the ALU pipe: 30 per 16 literals and sample word, 45
+// Bound by LOP3 (62 % of the ALU pipe: 30 per 16 literals and sample word, 45
 // per clause) and the shared-memory reads beside it (a literal is one read of
 // 4 TW bytes per lane, rows in random banks).  Tiles of TW x 32 samples, as
 // wide as shared memory allows: a wide read spends fewer clocks and fewer

@@ -1,6 +1,8 @@
 // The fused train kernels for units of 8-bit automata whose rows have at most
 // 1,024 words (capi.c:85-243 evaluation and feedback, automata.h:88-742
-// updates).  A unit's automata stay on its SM while it trains.
+// updates).  A unit's actions, and the count planes of rows up to 64 words (256
+// in k_train_spec), stay on its SM while it trains; the count planes of wider
+// rows stay in global memory, in L2 as far as the resident units' planes fit.
 //
 //   k_train_wpt   every thread owns WPT consecutive words of all eight clauses
 //   k_train_spec  few units: eight warps evaluate eight samples at once
@@ -831,7 +833,7 @@ __global__ void __launch_bounds__(NT, MINB)
 // valid unless it may move an action (Type II, Type Ib, Type Ia with
 // increments or several include bits): then the round ends after that sample
 // and the others are evaluated again.  Bit for bit the sequential rule.
-// Rows arrive in a ring of R slots, at least two rounds ahead.
+// Rows arrive in a ring of SP_RING slots.
 // ---------------------------------------------------------------------------
 namespace {
 
@@ -839,11 +841,12 @@ constexpr int SPW = 8;              // warps per unit: samples per round, clause
 constexpr uint32_t SP_NT = 32 * SPW;
 constexpr uint32_t SP_SC = 4;       // positions a thread examines per scan
 constexpr uint32_t SP_FILL = 128;
+constexpr uint32_t SP_RING = 32;    // sample rows held: at least two rounds ahead
 
 struct SpecLayout {
   uint32_t planes, ring, list, thr, lev, ovf, misc, total;
 };
-__host__ __device__ constexpr SpecLayout spec_layout(uint32_t SW, uint32_t R, uint32_t ovf_cap) {
+__host__ __device__ constexpr SpecLayout spec_layout(uint32_t SW, uint32_t ovf_cap) {
   SpecLayout L{};
   uint32_t at = 0;
   auto take = [&](uint32_t bytes) {
@@ -852,7 +855,7 @@ __host__ __device__ constexpr SpecLayout spec_layout(uint32_t SW, uint32_t R, ui
     return r;
   };
   L.planes = take(8 * 8 * SW * 4);
-  L.ring = take(R * SW * 4);
+  L.ring = take(SP_RING * SW * 4);
   L.list = take((SP_FILL + SP_SC * SP_NT) * 4);
   L.thr = take(SP_NT * 8 * 4);
   L.lev = take(4 * 2 * SW * 4);
@@ -866,7 +869,7 @@ __host__ __device__ constexpr SpecLayout spec_layout(uint32_t SW, uint32_t R, ui
 
 // misc: [0] unit, [8..39] live counts of a scan, [48..55] overflow counts
 // (2 parities x 4), [56..63] literal counts, [64..79] results (2 x 8)
-template <int SW, int R, int MINB, bool OV>
+template <int SW, int MINB, bool OV>
 __global__ void __launch_bounds__(SP_NT, MINB)
     k_train_spec(const TrainDev *__restrict__ machines, const WorkItem *__restrict__ work,
                  uint32_t nwork, uint32_t *__restrict__ counter, uint32_t e_begin, uint32_t e_end,
@@ -879,10 +882,11 @@ __global__ void __launch_bounds__(SP_NT, MINB)
   // the second exchange (333 units of 44 words 6.7 ms, 7.3 ms this way).
   constexpr bool ALONE = NK >= 4;
   constexpr uint32_t FULL = 0xFFFFFFFFu;
-  // rows a round may need were issued two rounds before it (R = 32) or one
-  constexpr int AHEAD = R >= 32 ? 1 : 0;
+  // rows a round may need were issued two rounds before it
+  constexpr uint32_t R = SP_RING;
+  constexpr int AHEAD = 1;
   extern __shared__ __align__(128) uint8_t smem[];
-  const SpecLayout o = spec_layout(SW, R, ovf_cap);
+  const SpecLayout o = spec_layout(SW, ovf_cap);
   uint32_t *planes = (uint32_t *)(smem + o.planes);  // [clause][count planes 0..6, action][SW]
   uint32_t *ring = (uint32_t *)(smem + o.ring);
   uint32_t *list = (uint32_t *)(smem + o.list);
@@ -1021,7 +1025,7 @@ __global__ void __launch_bounds__(SP_NT, MINB)
           }
           cp_commit();
         };
-        uint32_t fetched = cnt < (uint32_t)R ? cnt : (uint32_t)R;
+        uint32_t fetched = cnt < R ? cnt : R;
         fetch(0, fetched);
         for (uint32_t g0 = 0; g0 < cnt; g0 += SP_NT) {
           if (g0) __syncthreads();
@@ -1107,9 +1111,9 @@ __global__ void __launch_bounds__(SP_NT, MINB)
             // rows behind this round are done with: refill their slots, eight at
             // a time while the rounds are single samples (a round that grows from
             // one sample reaches at most 15 rows within the two rounds that its
-            // copies may take; a ring of 16 is refilled at once)
-            if (!alone || AHEAD == 0 || b + R - fetched >= 8) {
-              const uint32_t to = cnt - b < (uint32_t)R ? cnt : b + R;
+            // copies may take)
+            if (!alone || b + R - fetched >= 8) {
+              const uint32_t to = cnt - b < R ? cnt : b + R;
               fetch(fetched, to);
               fetched = to;
             } else {
@@ -1252,7 +1256,7 @@ __global__ void __launch_bounds__(SP_NT, MINB)
 // id (1-based).  k_train_wpt: W(threads per unit, words per thread, words
 // per row slot, count planes in registers, count planes in global memory,
 // Type Ib slots, CTAs per SM the registers are sized for); k_train_spec:
-// S(words per row slot, ring slots, CTAs per SM).
+// S(words per row slot, CTAs per SM).
 // Rows of up to 64 words keep every plane in shared memory (search rows: 26.2
 // ms; with three planes in L2 and 16 units per SM 30.7).  Wider rows leave
 // their count planes in L2, where the resident units' planes fit: the units
@@ -1263,26 +1267,27 @@ __global__ void __launch_bounds__(SP_NT, MINB)
 // three 105 ms).
 #define TM_WPT_CONFIGS(W, S)      \
   W(1, 256, 4, 1024, 1, 6, 4, 2)  \
-  S(2, 256, 32, 1)                \
+  S(2, 256, 1)                    \
   W(3, 128, 4, 512, 0, 7, 2, 5)   \
   W(4, 64, 4, 256, 0, 7, 2, 10)   \
-  S(5, 64, 32, 3)                 \
+  S(5, 64, 3)                     \
   W(6, 32, 2, 64, 0, 0, 4, 16)    \
   W(7, 32, 2, 56, 0, 0, 4, 16)    \
   W(8, 32, 1, 32, 0, 0, 4, 20)    \
-  S(9, 128, 32, 2)                \
+  S(9, 128, 2)                    \
   W(10, 32, 4, 128, 0, 7, 2, 20)  \
   W(11, 32, 2, 48, 0, 0, 4, 16)   \
   W(12, 32, 1, 24, 0, 0, 4, 20)
 
 struct WptConfig {
-  int id, ring;  // ring slots of k_train_spec, 0: k_train_wpt
+  int id;
+  bool spec;  // k_train_spec, else k_train_wpt
   int nt, sw, off;  // off: count planes not in shared memory
   int ibs;
 };
 static constexpr WptConfig kWpt[] = {
-#define TM_W(ID, NT, WPT, SW, RP, GP, IBS, MINB) {ID, 0, NT, SW, RP + GP, IBS},
-#define TM_S(ID, SW, R, MINB) {ID, R, (int)SP_NT, SW, 0, 4},
+#define TM_W(ID, NT, WPT, SW, RP, GP, IBS, MINB) {ID, false, NT, SW, RP + GP, IBS},
+#define TM_S(ID, SW, MINB) {ID, true, (int)SP_NT, SW, 0, 4},
     TM_WPT_CONFIGS(TM_W, TM_S)
 #undef TM_W
 #undef TM_S
@@ -1310,7 +1315,7 @@ double wpt_overflow(uint32_t bits, uint32_t picks) {
 
 static size_t wpt_bytes(const WptConfig &k, uint32_t smax) {
   const uint32_t oc = wpt_ovf_cap(smax);
-  return k.ring ? spec_layout(k.sw, k.ring, oc).total
+  return k.spec ? spec_layout(k.sw, oc).total
                 : wpt_layout(k.nt, k.sw, k.off, k.ibs, oc).total;
 }
 
@@ -1327,8 +1332,8 @@ static int config_occ(int id, size_t bytes) {
   switch (id) {
 #define TM_W(ID, NT, WPT, SW, RP, GP, IBS, MINB) \
   case ID: return wpt_occ(k_train_wpt<NT, WPT, SW, RP, GP, IBS, MINB, OV>, NT, bytes);
-#define TM_S(ID, SW, R, MINB) \
-  case ID: return wpt_occ(k_train_spec<SW, R, MINB, OV>, SP_NT, bytes);
+#define TM_S(ID, SW, MINB) \
+  case ID: return wpt_occ(k_train_spec<SW, MINB, OV>, SP_NT, bytes);
     TM_WPT_CONFIGS(TM_W, TM_S)
 #undef TM_W
 #undef TM_S
@@ -1369,7 +1374,7 @@ int wpt_choices(uint32_t Wpmax, uint32_t smax, uint32_t units, int sms, int opti
     int best = 0;
     for (int id = 1; id <= kWptCount; id++) {
       const WptConfig &k = kWpt[id - 1];
-      if ((k.ring != 0) != spec || k.nt < threads || Wpmax > (uint32_t)k.sw) continue;
+      if (k.spec != spec || k.nt < threads || Wpmax > (uint32_t)k.sw) continue;
       if (wpt_bytes(k, smax) > (size_t)optin) continue;
       if (best && kWpt[best - 1].sw <= k.sw) continue;
       best = id;
@@ -1398,9 +1403,9 @@ static void config_launch(int id, int grid, size_t bytes, cudaStream_t st,
     k_train_wpt<NT, WPT, SW, RP, GP, IBS, MINB, OV><<<grid, NT, bytes, st>>>(    \
         machines, work, nwork, counter, e_begin, e_end, ovf_cap, err);           \
     break;
-#define TM_S(ID, SW, R, MINB)                                                    \
+#define TM_S(ID, SW, MINB)                                                       \
   case ID:                                                                       \
-    k_train_spec<SW, R, MINB, OV><<<grid, SP_NT, bytes, st>>>(                   \
+    k_train_spec<SW, MINB, OV><<<grid, SP_NT, bytes, st>>>(                      \
         machines, work, nwork, counter, e_begin, e_end, ovf_cap, err);           \
     break;
     TM_WPT_CONFIGS(TM_W, TM_S)
