@@ -2176,14 +2176,14 @@ static int predict_gemm(tm_machine *m, uint64_t n) {
 }
 
 // A predict of at most TM_SMALL_N_MAX samples of a dense machine: one launch
-// per 16 samples from the byte rows to the outputs (k_predict_few).  Requests
+// per one or two groups of 16 samples from the byte rows to the outputs (k_predict_few).  Requests
 // from host memory of up to 3,840 bytes travel in the kernel's parameters,
 // larger ones through the machine's pinned buffer and a copy; the outputs come
 // back through the pinned buffer.
 static int predict_few(tm_machine *m, const uint8_t *problems, uint64_t n, int64_t *out_classes,
                        uint8_t *out_codes, int64_t *out_scores, bool on_device) {
   const ClassDev &c0 = m->cls[0];
-  const uint64_t sums_b = 16ull * m->classes * 4;
+  const uint64_t sums_b = 2 * 16ull * m->classes * 4;
   if (m->few.cap < sums_b + 16) {
     CK(m->few.ensure(sums_b + 16));
     CK(cudaMemsetAsync(m->few.p, 0, m->few.cap, m->st));
@@ -2238,9 +2238,7 @@ static int predict_few(tm_machine *m, const uint8_t *problems, uint64_t n, int64
     f.out_scores = out_scores;
   }
   if (m->timing) CK(cudaEventRecord(m->ev0, m->st));
-  CK(launch_predict_few(f, (uint32_t)n, m->st));
-  const uint32_t group = predict_few_group(c0.Wp);
-  note_launch(m, (n + group - 1) / group);
+  CK(launch_predict_few(f, (uint32_t)n, m->st, &m->stats.kernel_launches));
   if (m->timing) CK(cudaEventRecord(m->ev1, m->st));
   m->stats.predict_launches++;
   m->stats.predict_gemm = 0;

@@ -280,9 +280,9 @@ cudaError_t launch_serve_finalize(const ServeJob *jobs_dev, uint32_t njobs, cuda
 // warp per row (k_predict_small) instead of the 64 x 64 tiles.
 constexpr uint32_t TM_SMALL_N_MAX = 32;
 // A predict of at most TM_SMALL_N_MAX samples of a dense machine from byte
-// rows to outputs, one launch per group of samples (k_predict_few).  `in` and
+// rows to outputs, one launch per one or two groups of samples (k_predict_few).  `in` and
 // the outputs may be device memory or pinned host memory; without `in` the
-// rows are in `inl` (one launch).  sums (16 x classes) and done are zero
+// rows are in `inl` (one group).  sums (2 x 16 x classes) and done (2) are zero
 // between calls: the kernel leaves them so.
 struct FewRows {
   uint32_t w[960];
@@ -304,7 +304,8 @@ struct PredictFew {
   FewRows inl;
 };
 uint32_t predict_few_group(uint32_t Wp);
-cudaError_t launch_predict_few(const PredictFew &f, uint32_t n, cudaStream_t st);
+cudaError_t launch_predict_few(const PredictFew &f, uint32_t n, cudaStream_t st,
+                               uint64_t *launches);
 // k_lits with an optional gate (skipped while *gate == 0)
 cudaError_t launch_lits_gated(const uint32_t *act, const ClassDev *cls, uint32_t classes,
                               uint32_t clauses, int32_t *lits, const uint32_t *gate,

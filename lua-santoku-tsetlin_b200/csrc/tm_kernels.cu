@@ -1806,7 +1806,8 @@ constexpr int FEW_DEPTH = 8;  // copies in flight per lane
 // U: steps of the row loop unrolled, so that ring slots and the choice of
 // counting are fixed per step (a whole ring of them, 4 or 8, for rows of more than
 // 3 steps, which are then padded to whole groups of U steps), or 1.
-template <int NS, int CR, int U>
+// TWO: the blocks of blockIdx.y = 1 take the second half of the samples.
+template <int NS, int CR, int U, bool TWO = false>
 __global__ void __launch_bounds__(256, NS <= 2 ? 4 : (NS <= 5 ? 3 : 2))
     k_predict_few(const uint32_t *__restrict__ act, const int32_t *__restrict__ lits,
                   const ClassDev C, uint32_t classes, uint32_t clauses, uint32_t tol,
@@ -1817,6 +1818,20 @@ __global__ void __launch_bounds__(256, NS <= 2 ? 4 : (NS <= 5 ? 3 : 2))
   extern __shared__ __align__(16) uint32_t fsm[];
   __shared__ bool last;
   const uint32_t lane = threadIdx.x & 31;
+  if constexpr (TWO) {
+    const uint32_t half = (ns + 1) / 2;
+    if (blockIdx.y) {
+      in += (uint64_t)half * row_bytes;
+      sums += 16 * classes;
+      done += 1;
+      if (out_classes) out_classes += half;
+      if (out_codes) out_codes += half * ((classes + 7) >> 3);
+      if (out_scores) out_scores += (uint64_t)half * classes;
+      ns -= half;
+    } else {
+      ns = half;
+    }
+  }
   const uint32_t Wp = C.Wp, W = C.W, Q = Wp >> 2, KQ = ((Q + 31) / 32 + U - 1) / U * U;
   static_assert(U == 1 || (U * CR) % FEW_DEPTH == 0 || FEW_DEPTH % (U * CR) == 0, "ring slots");
   // [FEW_DEPTH][thread] 16-byte ring slots, then the samples' rows
@@ -2013,7 +2028,7 @@ __global__ void __launch_bounds__(256, NS <= 2 ? 4 : (NS <= 5 ? 3 : 2))
 
 // One launch of k_predict_few: one wave of resident CTAs, each warp with an
 // equal share of the machine's clauses.
-template <int NS, int CR, int U>
+template <int NS, int CR, int U, bool TWO>
 static cudaError_t few_launch_u(const PredictFew &f, uint32_t s0, uint32_t ns, cudaStream_t st) {
   // resident CTAs per SM at the last shared-memory size, per device (the
   // limit is raised to the most any call asks for when it is first used)
@@ -2023,35 +2038,36 @@ static cudaError_t few_launch_u(const PredictFew &f, uint32_t s0, uint32_t ns, c
   const uint64_t got = sc.load(std::memory_order_relaxed);
   int occ = (int)(got & 0xFF);
   if (got >> 8 != smem || !occ) {
-    cudaError_t e = cudaFuncSetAttribute(k_predict_few<NS, CR, U>,
+    cudaError_t e = cudaFuncSetAttribute(k_predict_few<NS, CR, U, TWO>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)TM_FEW_SMEM + FEW_DEPTH * 256 * 16);
     if (e == cudaSuccess)
-      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_predict_few<NS, CR, U>, 256, smem);
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_predict_few<NS, CR, U, TWO>, 256, smem);
     if (e != cudaSuccess) return e;
     if (occ <= 0) occ = 1;
     sc.store(smem << 8 | (uint64_t)occ, std::memory_order_relaxed);
   }
   const uint64_t total = (uint64_t)f.classes * f.clauses;
-  const uint64_t resident = (uint64_t)f.sms * occ * 8;
+  const uint64_t resident = (uint64_t)f.sms * occ * 8 / (TWO ? 2 : 1);
   uint64_t per = (total + resident - 1) / resident;
   if (per > 1) per = (per + CR - 1) / CR * CR;  // whole groups of CR rows
   const uint64_t used = (total + per - 1) / per;
   const uint32_t nb = (f.classes + 7) >> 3;
-  k_predict_few<NS, CR, U><<<(unsigned)((used + 7) / 8), 256, smem, st>>>(
+  k_predict_few<NS, CR, U, TWO><<<dim3((unsigned)((used + 7) / 8), TWO ? 2 : 1), 256, smem, st>>>(
       f.act, f.lits, f.C, f.classes, f.clauses, f.tol,
-      f.in ? f.in + (uint64_t)s0 * f.row_bytes : nullptr, f.row_bytes, ns, (uint32_t)per, f.sums, f.done, f.type,
+      f.in ? f.in + (uint64_t)s0 * f.row_bytes : nullptr, f.row_bytes, ns, (uint32_t)per,
+      f.sums, f.done, f.type,
       f.out_classes ? f.out_classes + s0 : nullptr,
       f.out_codes ? f.out_codes + (uint64_t)s0 * nb : nullptr,
       f.out_scores ? f.out_scores + (uint64_t)s0 * f.classes : nullptr, f.inl);
   return cudaGetLastError();
 }
 
-template <int NS, int CR>
+template <int NS, int CR, bool TWO = false>
 static cudaError_t few_launch(const PredictFew &f, uint32_t s0, uint32_t ns, cudaStream_t st) {
   constexpr int U = FEW_DEPTH / CR;  // a whole ring of steps
-  return f.C.Wp > 3 * 128 ? few_launch_u<NS, CR, U>(f, s0, ns, st)
-                          : few_launch_u<NS, CR, 1>(f, s0, ns, st);
+  return f.C.Wp > 3 * 128 ? few_launch_u<NS, CR, U, TWO>(f, s0, ns, st)
+                          : few_launch_u<NS, CR, 1, TWO>(f, s0, ns, st);
 }
 
 // Samples per launch for rows of Wp words (0: the rows do not fit): 16, or as
@@ -2063,11 +2079,20 @@ uint32_t predict_few_group(uint32_t Wp) {
   return 0;
 }
 
-cudaError_t launch_predict_few(const PredictFew &f, uint32_t n, cudaStream_t st) {
-  const uint32_t group = predict_few_group(f.C.Wp);
-  if (!group) return cudaErrorInvalidValue;
-  for (uint32_t s0 = 0; s0 < n; s0 += group) {
-    const uint32_t ns = n - s0 < group ? n - s0 : group;
+cudaError_t launch_predict_few(const PredictFew &f, uint32_t n, cudaStream_t st,
+                               uint64_t *launches) {
+  const uint32_t fit = predict_few_group(f.C.Wp);
+  if (!fit) return cudaErrorInvalidValue;
+  // Machines of up to 32 clauses per SM: both halves of more than 16 samples in
+  // one launch, since that of one leaves most of its time to latency (device rows,
+  // 32 samples: 2,560 clauses of 49 words 62 -> 43 us, 24 clauses of 1,024 words
+  // 68 -> 46 us).  Larger machines take the groups in turn.
+  if (n > 16 && fit == 16 && (uint64_t)f.classes * f.clauses <= 32ull * f.sms) {
+    *launches += 1;
+    return n <= 24 ? few_launch<12, 1, true>(f, 0, n, st) : few_launch<16, 1, true>(f, 0, n, st);
+  }
+  for (uint32_t s0 = 0; s0 < n; s0 += fit) {
+    const uint32_t ns = n - s0 < fit ? n - s0 : fit;
     cudaError_t e;
     if (ns <= 1) e = few_launch<1, 2>(f, s0, ns, st);
     else if (ns == 2) e = few_launch<2, 2>(f, s0, ns, st);
@@ -2080,6 +2105,7 @@ cudaError_t launch_predict_few(const PredictFew &f, uint32_t n, cudaStream_t st)
     else if (ns <= 12) e = few_launch<12, 1>(f, s0, ns, st);
     else e = few_launch<16, 1>(f, s0, ns, st);
     if (e != cudaSuccess) return e;
+    *launches += 1;
   }
   return cudaSuccess;
 }
