@@ -389,7 +389,8 @@ int tm_force_variant(tm_machine *m, int32_t mode, int32_t cpw);
 
 /* Failure injection for tests of the error paths: after `after` more
  * successful device allocations, the next one the library makes fails as if
- * the GPU were out of memory (the call reports TM_ERR_OOM); then the
+ * the GPU were out of memory (the call reports TM_ERR_OOM, or does the same
+ * work another way where the memory only makes it faster); then the
  * injection disarms itself.  after < 0 disarms it.  No counterpart in the
  * reference. */
 int tm_debug_fail_alloc(int64_t after);
